@@ -19,6 +19,9 @@
 //     mesh is finished there, every other site is listed (its cell stored as
 //     plane-id triples when it was built; the sites not done within the
 //     first kNN tier are listed again for their full neighbour rows);
+//   * (float predicates) k_cell_mesh over the cells that are finished but not
+//     inside the mesh: the part of each in the mesh from its edges and the
+//     mesh's open triangles (clip_mesh.cuh); k_clip_site then only builds;
 //   * k_clip_site over the listed sites (or over every site in the reference
 //     form), one warp per site, 2 slots per lane (64 vertices): the site's
 //     cell (stored, resumed, or built), its bound by the domain box when its
@@ -256,7 +259,10 @@ __device__ __forceinline__ void store_master(const WarpCell<SL>& c, SiteSmem<SL,
 // site goes on the completion list with the squared radius of its pieces,
 // and the completion pass (COMPLETE) clips its cell by every site within
 // twice that radius beyond its K nearest before it clips the tets again.
-template <bool CELL_TET, bool BATCHED, int SL, bool ROBUST, bool COMPLETE = false>
+//
+// MESH (exact form, float): a cell that is not inside the mesh goes to the
+// mesh pass (clip_mesh.cuh) instead of being clipped by each tet.
+template <bool CELL_TET, bool BATCHED, int SL, bool ROBUST, bool COMPLETE = false, bool MESH = false>
 __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : SL >= 4 ? 6 : VGB_CLIP_MIN_BLOCKS) k_clip_site(
     const float4* __restrict__ sites, int n, const unsigned* __restrict__ knn, const ProbDesc* __restrict__ probs,
     const int* __restrict__ site_prob, const ProbDesc lone, const float4* __restrict__ verts,
@@ -408,6 +414,8 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : SL >= 4 ? 6 :
         }
         c.nt = S.mnt;
         c.r2 = S.mr2;
+      } else if (MESH && !COMPLETE) {
+        break;  // (every cell of at most 64 vertices was handed on)
       } else {
         // refill the queue from the next chunk(s) of candidates
         while (qi >= nsurv) {
@@ -725,7 +733,10 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : SL >= 4 ? 6 :
                     const int src = __ffs(cm) - 1;
                     const float4 Q = make_float4(__shfl_sync(FULL, P.x, src), __shfl_sync(FULL, P.y, src),
                                                  __shfl_sync(FULL, P.z, src), __shfl_sync(FULL, P.w, src));
-                    if (lane == 0) S.plane[nxt] = Q;
+                    if (lane == 0) {
+                      S.plane[nxt] = Q;
+                      S.mtri[nxt] = (unsigned)(b0 + src);  // its site, for the mesh pass
+                    }
                     __syncwarp();
                     const int r = warp_clip<SL, ROBUST>(c, Q, (unsigned)nxt, S.plane, S.conf, S.bedge, lane, true,
                                                         S.cnt + WC_NEWV, S.cnt + WC_EXACT);
@@ -860,8 +871,47 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : SL >= 4 ? 6 :
           // With the pieces pass, the cell's record (face ids, radius,
           // outcome so far) goes to it and the site is done here; the
           // pieces pass clips each candidate tet by the faces crossing it.
-          emitted = CELL_TET && !COMPLETE && piece_list != nullptr && nfaces <= PIECE_FACES;
-          if (emitted) {
+          emitted = CELL_TET && !COMPLETE && !MESH && piece_list != nullptr && nfaces <= PIECE_FACES;
+          int nt_out = MESH ? c.nt : MESH_VERTS + 1;
+          if (MESH && COMPLETE) {
+            // the sites beyond the K nearest by rank among the cell's faces
+            // (S.faces is ascending): id -> 4 + K + 12 + rank, the site in
+            // the cell's record
+            const int first_free = 4 + K + 2 * BOX_PLANES;
+            unsigned char* const to = reinterpret_cast<unsigned char*>(S.conf);
+            int own = 0;
+            for (int f0 = 0; f0 < nfaces; f0 += WARP) {
+              const int id = f0 + lane < nfaces ? (int)S.faces[f0 + lane] : NPLANE;
+              own += __popc(__ballot_sync(FULL, id < first_free));
+            }
+            for (int f = lane; f < nfaces; f += WARP) {
+              const int id = S.faces[f];
+              to[id] = (unsigned char)(id < first_free ? id : first_free + f - own);
+              if (id >= first_free && f - own < MESH_EXT) store.faces[(size_t)s * PIECE_REC + f - own] = S.mtri[id];
+            }
+            __syncwarp();
+            if (nfaces - own > MESH_EXT || !cdone) nt_out = MESH_VERTS + 1;
+          }
+          if (MESH && nt_out <= MESH_VERTS) {
+            emitted = true;
+            int base = 0;
+#pragma unroll
+            for (int k = 0; k < SL; ++k) {
+              if (c.vm[k] & lane_bit) {
+                unsigned t = c.tri[k];
+                if (COMPLETE) {
+                  const unsigned char* const to = reinterpret_cast<const unsigned char*>(S.conf);
+                  t = pack_tri(to[tri_at(t, 0)], to[tri_at(t, 1)], to[tri_at(t, 2)]);
+                }
+                store.mtri[(size_t)s * MESH_VERTS + base + __popc(c.vm[k] & lt_mask)] = t;
+              }
+              base += __popc(c.vm[k]);
+            }
+            if (lane == 0) {
+              store.mnt[s] = c.nt | (int)(S.site_flags << 8);
+              piece_list[atomicAdd(piece_count, 1)] = s;
+            }
+          } else if (emitted) {
             unsigned* const rec = store.faces + (size_t)s * PIECE_REC;
             if (lane < PIECE_FACES / 4)
               rec[4 + lane] = (unsigned)S.faces[4 * lane] | ((unsigned)S.faces[4 * lane + 1] << 8) |
@@ -941,7 +991,9 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : SL >= 4 ? 6 :
     if (lane == 0) {
       unsigned f = S.site_flags;
       // a completion that failed keeps the earlier pass's moments
-      const bool keep_old = COMPLETE && ((f & (SITE_UNRESOLVED | SITE_DROPPED)) || S.unchanged);
+      // (in the mesh form those are good only where the K neighbours were
+      // enough: a failed completion leaves what it clipped)
+      const bool keep_old = COMPLETE && ((f & (MESH ? SITE_DROPPED : SITE_UNRESOLVED | SITE_DROPPED)) || S.unchanged);
       if (!keep_old)
         mom[s] = make_dmom4((double)S.acc[0] + (double)S.acc[4], (double)S.acc[1] + (double)S.acc[5],
                             (double)S.acc[2] + (double)S.acc[6], (double)S.acc[3] + (double)S.acc[7]);
@@ -1372,6 +1424,10 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, VGB_PIECE_MIN_BLOCKS) k_cli
   if (stats && lane < WC_N && S.cnt[lane]) atomicAdd(stats + stat_slot(lane), (unsigned long long)S.cnt[lane]);
 }
 
+}  // namespace vgb
+#include "clip_mesh.cuh"
+namespace vgb {
+
 // Shared state of one lane group of k_build: its clip scratch; the group's
 // planes (4+j bisector j, 4+K+b start-cube face b) are build_plane_stride(K)
 // float4 of the dynamic shared memory, sized by the largest K.
@@ -1400,7 +1456,7 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, BATCHED ? VGB_BUILD_MIN_BLO
     unsigned long long* __restrict__ stats, const unsigned char* __restrict__ field,
     const unsigned* __restrict__ field_sat, int* __restrict__ work, int* __restrict__ out_list,
     int* __restrict__ out_count, int kmax, const CellStore store, int k_tier, int* __restrict__ deep_list,
-    int* __restrict__ deep_count) {
+    int* __restrict__ deep_count, int* __restrict__ mesh_list, int* __restrict__ mesh_count) {
   constexpr int NG = WARP / G;
   __shared__ BuildSmem<G * SL> smem_all[CLIP_WARPS * NG];
   extern __shared__ float4 build_planes[];
@@ -1549,11 +1605,15 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, BATCHED ? VGB_BUILD_MIN_BLO
     // to resume from
     const bool keep = has && !interior && state == 0;
     const bool deep = has && !interior && K1 < K && !(state == 0 && !secmiss);
+    // (a cell that reached its radius goes straight to the mesh pass, when
+    // there is one)
+    const bool direct = keep && !secmiss && mesh_list != nullptr;
     if (store.tri) {
+      unsigned* const to = direct ? store.mtri + (size_t)s * MESH_VERTS : store.tri + (size_t)s * STORE_VERTS;
       int base = 0;
 #pragma unroll
       for (int k = 0; k < SL; ++k) {
-        if (keep && (c.vm[k] & lb)) store.tri[(size_t)s * STORE_VERTS + base + __popc(c.vm[k] & (lb - 1u))] = c.tri[k];
+        if (keep && (c.vm[k] & lb)) to[base + __popc(c.vm[k] & (lb - 1u))] = c.tri[k];
         base += __popc(c.vm[k]);
       }
     }
@@ -1562,7 +1622,10 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, BATCHED ? VGB_BUILD_MIN_BLO
       S.cnt[WC_CLIPS] += (seq_cnt >> 8) & 0xffu;
       S.cnt[WC_CONFLICT] += seq_cnt >> 16;
       if (store.flags) store.flags[s] = interior ? SITE_INTERIOR : SITE_HANDED;
-      if (!interior) {
+      if (direct) {
+        store.mnt[s] = c.nt;
+        mesh_list[atomicAdd(mesh_count, 1)] = s;
+      } else if (!interior) {
         if (store.nt) store.nt[s] = keep ? (c.nt | (secmiss ? 256 : 0) | (deep ? (4 + K1) << 16 : 0)) : 0;
         out_list[atomicAdd(out_count, 1)] = s;
         if (deep) deep_list[atomicAdd(deep_count, 1)] = s;
@@ -1612,9 +1675,11 @@ template <bool R>
 struct ClipPasses {
   // SMs x resident blocks per SM, per kernel variant: tet-cell, cell-tet lone
   // fast / redo, cell-tet batched fast / redo, completion lone / batched,
-  // the 96-vertex fast pass lone / batched, the pieces pass lone / batched
+  // the 96-vertex fast pass lone / batched, the pieces pass lone / batched,
+  // and of the float exact form the mesh pass, the one-warp pass and the
+  // completion pass that hand on to it, lone / batched each
   static int* resident() {
-    static int r[11] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    static int r[17] = {};
     return r;
   }
   static int prepare();
@@ -1646,6 +1711,13 @@ int ClipPasses<R>::prepare() {
       resident_blocks(k_clip_site<true, true, SLOTS_WIDE, R>, sms, r + 8) ||
       resident_blocks(k_clip_pieces<false, R>, sms, r + 9) || resident_blocks(k_clip_pieces<true, R>, sms, r + 10))
     return -2;
+  if constexpr (!R)
+    if (resident_blocks(k_cell_mesh<false>, sms, r + 11) || resident_blocks(k_cell_mesh<true>, sms, r + 12) ||
+        resident_blocks(k_clip_site<true, false, SLOTS_FAST, false, false, true>, sms, r + 13) ||
+        resident_blocks(k_clip_site<true, true, SLOTS_FAST, false, false, true>, sms, r + 14) ||
+        resident_blocks(k_clip_site<true, false, SLOTS_COMPLETE, false, true, true>, sms, r + 15) ||
+        resident_blocks(k_clip_site<true, true, SLOTS_COMPLETE, false, true, true>, sms, r + 16))
+      return -2;
   return 0;
 }
 
@@ -1714,7 +1786,9 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
   // completion pass's work counter; lists: [0, n) the hand-offs to the
   // 128-vertex pass, [n, 2n) the first pass's, [2n, 3n) the deep sites,
   // [3n, 4n) the sites to complete, [4n, 5n) their pieces' squared radius
-  // bounds (float) and [5n, 6n) the pieces pass's sites
+  // bounds (float) and [5n, 6n) the pieces pass's sites or the mesh pass's;
+  // [12] the mesh pass's sites, [13] its work counter, [14, 15] the same for
+  // its second launch, over completed cells (their list: [n, 2n) again)
   const bool exact = tet_order != nullptr;
   int* const redo = lists;
   int* const rest = lists + n;
@@ -1722,10 +1796,12 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
   int* const esc = exact ? lists + 3 * (size_t)n : nullptr;
   float* const esc_r2 = exact ? reinterpret_cast<float*>(lists + 4 * (size_t)n) : nullptr;
   // the pieces pass (cell-tet records needed)
-  const bool pieces = shape.pieces != 0 && store.faces != nullptr;
+  const bool mesh = !R && exact && store.rec != nullptr;
+  const bool pieces = !mesh && shape.pieces != 0 && store.faces != nullptr;
   int* const piece_list = pieces ? lists + 5 * (size_t)n : nullptr;
+  int* const mesh_list = mesh ? lists + 5 * (size_t)n : nullptr;
   const int kt = exact ? k_tier : 0;
-  VGB_CUDA_TRY(cudaMemsetAsync(counters, 0, 12 * sizeof(int), st));
+  VGB_CUDA_TRY(cudaMemsetAsync(counters, 0, CLIP_COUNTERS * sizeof(int), st));
   // every pass: one wave of resident blocks whose warps draw sites from a counter
   // the first pass's stored cells (exact form only)
   CellStore cs = store;
@@ -1757,7 +1833,7 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
     auto build = [&](auto kernel) {
       kernel<<<bb, CLIP_WARPS * WARP, dyn, st>>>(sites, n, knn, probs, site_prob, lone, mom, stats, field, field_sat,
                                                   counters + 2, rest, counters + 0, kmax, cs, kt, deep,
-                                                  counters + 8);
+                                                  counters + 8, mesh_list, counters + 12);
     };
     if (probs) {
       if (G == 16) build(k_build<true, 16, 2, R>);
@@ -1771,6 +1847,50 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
         knn_sites_listed(sites, n, cell_start, probs, site_prob, lone, kmax, pos_of_id, knn, deep, counters + 8,
                          counters + 9, st, shape.knn_warps))
       return -2;
+  }
+  if constexpr (!R) {
+    if (mesh) {
+      auto pass = [&](auto kernel, int variant, const int* in_list, int* in_count, int* out_list, int* out_count,
+                      int* work, int* to_list, int* to_count) {
+        kernel<<<g_clip_resident_blocks[variant], CLIP_WARPS * WARP, 0, st>>>(
+            sites, n, knn, probs, site_prob, lone, verts, tets, site_start, site_tets, mom, stats, field, field_sat,
+            tet_order, tet_cell_start, tet_sph, reach, reach_max_bits, prob_secmiss, in_list, in_count, out_list,
+            out_count, work, cs, kt, cell_start, esc, esc_r2, counters + 10, to_list, to_count);
+      };
+      auto mesh_pass = [&](const int* in_list, int* in_count, int* work, bool last) {
+        auto go = [&](auto kernel, int variant) {
+          kernel<<<g_clip_resident_blocks[variant], MESH_WARPS * WARP, 0, st>>>(
+              sites, knn, probs, site_prob, lone, cs.rec, tet_cell_start, tet_sph, reach, reach_max_bits, mom, stats,
+              prob_secmiss, in_list, in_count, work, last ? nullptr : redo, counters + 1, cs, last ? nullptr : esc,
+              esc_r2, counters + 10);
+        };
+        if (probs) go(k_cell_mesh<true>, 12);
+        else go(k_cell_mesh<false>, 11);
+      };
+      // the cells the first pass left, finished or taken whole; then what of
+      // each lies in the mesh; then the cells above 64 vertices, and those
+      // their K neighbours left unresolved
+      if (probs) {
+        pass(k_clip_site<true, true, SLOTS_FAST, false, false, true>, 14, rest, counters + 0, redo, counters + 1,
+             counters + 3, mesh_list, counters + 12);
+        mesh_pass(mesh_list, counters + 12, counters + 13, false);
+        pass(k_clip_site<true, true, SLOTS_REDO, false>, 4, redo, counters + 1, nullptr, nullptr, counters + 4,
+             nullptr, nullptr);
+        pass(k_clip_site<true, true, SLOTS_COMPLETE, false, true, true>, 16, esc, counters + 10, nullptr, nullptr,
+             counters + 11, rest, counters + 14);
+      } else {
+        pass(k_clip_site<true, false, SLOTS_FAST, false, false, true>, 13, rest, counters + 0, redo, counters + 1,
+             counters + 3, mesh_list, counters + 12);
+        mesh_pass(mesh_list, counters + 12, counters + 13, false);
+        pass(k_clip_site<true, false, SLOTS_REDO, false>, 2, redo, counters + 1, nullptr, nullptr, counters + 4,
+             nullptr, nullptr);
+        pass(k_clip_site<true, false, SLOTS_COMPLETE, false, true, true>, 15, esc, counters + 10, nullptr, nullptr,
+             counters + 11, rest, counters + 14);
+      }
+      mesh_pass(rest, counters + 14, counters + 15, true);
+      VGB_CUDA_TRY(cudaGetLastError());
+      return 0;
+    }
   }
   const int* in_list = exact ? rest : nullptr;
   const int* in_count = exact ? counters + 0 : nullptr;

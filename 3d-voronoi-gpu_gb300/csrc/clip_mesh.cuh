@@ -1,0 +1,684 @@
+// Mesh pass of the exact cell-tet form: the part of a finished cell that lies
+// in the mesh, without building the pieces cell ^ tet.
+//
+// The volume and first moment of cell ^ mesh are sums over its boundary: over
+// each face of the cell, the part inside the mesh; over each boundary
+// triangle of the mesh, the part inside the cell.  Split into signed tets
+// from an apex (the apex, the foot of the apex on a face, a piece of one of
+// the face's edges), only lines are left:
+//   * the cell's edges, each as far as it lies in the mesh.  A tet cuts a
+//     length off an edge (an interval of four plane tests); the lengths of
+//     all the tets add up on the lane that holds the edge.  Where two tets
+//     share a face, that face and its lines give opposite terms and drop out;
+//   * for each open triangle (a tet face that no other tet shares from its
+//     other side), the polygon triangle ^ cell: its edges on the cell's faces
+//     and on its own sides.
+// Summing det(F1 - F0, a, b) / 6 over the pieces [a, b] of every line of two
+// faces (feet F0, F1) gives the volume, and (F + a + b) / 4 of each signed tet
+// the moment.
+//
+// Consistency.  A tet face is one plane for both its tets: its three vertices
+// in mesh order make it, so an edge's interval ends where the next tet's
+// begins, bit for bit, also where the edge grazes the face or lies in it
+// within rounding.  Points that two lines share are made once: where an edge
+// of the cell meets a triangle (on the edge), where a side of a triangle meets
+// a face of the cell (on the side).  Lines are kept as their point nearest
+// the site and a unit direction, so that a long edge of an open cell is as
+// exact near the site as a short one.
+//
+// One warp per site: lanes take candidate tets, then (tet, edge) pairs, then
+// faces.  Bound by instruction issue and the latency of its short loops, like
+// the pass it replaces, but a boundary cell (at 1M torus sites 36 edges, 20
+// tets, 6 open triangles) needs no vertices of its pieces, whose inner faces
+// only cancel.  Measured per Lloyd iteration: 1M sites in 1.96M tets 15.0 ->
+// 6.6 ms from random sites and 4.6 -> 2.4 ms once relaxed (the one-warp pass
+// before, now that pass without its tets and this one); 131k sites in 1.57M
+// tets 6.9 -> 2.5 ms and 1.6 -> 0.6 ms (pieces from the tets before).
+#pragma once
+
+#include "clip_warp.cuh"
+
+namespace vgb {
+
+constexpr int MESH_WARPS = 4;
+// A cell of at most 64 vertices (three faces meet in each) has at most 34
+// faces and 96 edges.
+constexpr int MESH_FACES = 36, MESH_EDGES = 96;
+constexpr int MESH_IDS = 4 + MAX_SITE_K + 12 + MESH_EXT;  // plane ids a stored cell may use
+constexpr int MESH_ID_WORDS = (MESH_IDS + 31) / 32;
+// A cell whose terms from the site exceed this many times their sum is done
+// again from a point of what is left of it (sites outside the mesh).
+constexpr float MESH_APEX_RATIO = 32.f;
+#ifndef VGB_MESH_MIN_BLOCKS
+#define VGB_MESH_MIN_BLOCKS 5
+#endif
+
+struct MeshSmem {
+  float4 plane[MESH_FACES];  // the cell's faces, site-relative
+  union {
+    struct {
+      float4 vert[MESH_VERTS];    // the cell's vertices, while its edges are made
+      unsigned edge[MESH_EDGES];  // faces p, q and end vertices of each edge
+      unsigned char loc[MESH_ID_WORDS * 32];  // plane id -> face
+    };
+    float4 tp[WARP][4];  // the face planes of the tets in hand, in mesh order
+  };
+  union {
+    unsigned char twin[MESH_FACES * MESH_FACES];  // (p, q) -> vertex, while the edges are made
+    float4 slot[2][MESH_FACES];  // a triangle's plane across each face: first and second point
+  };
+  // the cell's edges: point nearest the site and direction, with the end
+  // parameters; the terms of a unit of its length (volume in w)
+  float4 epos[MESH_EDGES], edir[MESH_EDGES], eterm[MESH_EDGES];
+  unsigned short epq[MESH_EDGES];  // its faces, p | q << 8
+  int tidx[WARP];       // tets in hand: their record, and what is known of them
+  unsigned char tinf[WARP], thit[WARP];
+  int queue[2 * WARP];  // tets whose sphere meets the cell's
+  int rng[2][WARP];     // the rows in hand: first tet, tets of the rows before
+  unsigned cnt[WC_N];
+};
+
+// dot product ending in + c, the same rounding in every kernel
+__device__ __forceinline__ float fma3(float ax, float ay, float az, float bx, float by, float bz, float c) {
+  return __fmaf_rn(ax, bx, __fmaf_rn(ay, by, __fmaf_rn(az, bz, c)));
+}
+__device__ __forceinline__ float eval4(float4 P, float3 x) { return fma3(P.x, P.y, P.z, x.x, x.y, x.z, P.w); }
+__device__ __forceinline__ float3 cross_rn(float3 a, float3 b) {
+  return make_float3(cross_term(a.y, b.z, a.z, b.y), cross_term(a.z, b.x, a.x, b.z), cross_term(a.x, b.y, a.y, b.x));
+}
+__device__ __forceinline__ float dot_rn(float3 a, float3 b) { return dot3_rn(a.x, a.y, a.z, b.x, b.y, b.z); }
+__device__ __forceinline__ float3 sub_rn(float3 a, float3 b) {
+  return make_float3(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z));
+}
+__device__ __forceinline__ float3 along(float3 p, float t, float3 u) {
+  return make_float3(__fmaf_rn(t, u.x, p.x), __fmaf_rn(t, u.y, p.y), __fmaf_rn(t, u.z, p.z));
+}
+__device__ __forceinline__ float3 xyz(float4 v) { return make_float3(v.x, v.y, v.z); }
+
+// Where the line p + t u meets plane P, and whether the plane's positive side
+// lies ahead.  A line in the plane's direction meets it at -inf or +inf,
+// with "ahead": then every point of it is on the positive side (P >= 0) or
+// none is.  (The 1e-37 decides the line in the plane: positive side.)
+__device__ __forceinline__ float line_at(float4 P, float3 p, float3 u, bool& ahead) {
+  const float d = fma3(P.x, P.y, P.z, p.x, p.y, p.z, P.w);
+  const float du = fma3(P.x, P.y, P.z, u.x, u.y, u.z, 0.f);
+  ahead = du >= 0.f;
+  return __fdividef(__fsub_rn(-1e-37f, d), du);
+}
+
+// Signed tets of the piece [a, b] on the line of faces 0 and 1 (feet F0, F1;
+// all apex-relative; c = a x b, ab = a + b).
+struct MeshSum {
+  float v = 0.f, x = 0.f, y = 0.f, z = 0.f, mag = 0.f;
+  __device__ __forceinline__ void add(float k, float3 F, float3 ab) {
+    v = __fadd_rn(v, k);
+    mag = __fadd_rn(mag, fabsf(k));
+    x = __fmaf_rn(k, __fadd_rn(F.x, ab.x), x);
+    y = __fmaf_rn(k, __fadd_rn(F.y, ab.y), y);
+    z = __fmaf_rn(k, __fadd_rn(F.z, ab.z), z);
+  }
+};
+
+// Foot of the apex X on plane P, relative to X.
+__device__ __forceinline__ float3 foot_of(float4 P, float3 X) {
+  const float nn = dot3_rn(P.x, P.y, P.z, P.x, P.y, P.z);
+  const float l = __fdividef(-eval4(P, X), nn);
+  return make_float3(__fmul_rn(l, P.x), __fmul_rn(l, P.y), __fmul_rn(l, P.z));
+}
+
+// Largest / smallest of one float per lane (one instruction each).
+__device__ __forceinline__ float redux_max(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float redux_min(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+// The segment [P, Q] as a line (point nearest the origin, unit direction,
+// end parameters).
+struct Line {
+  float3 p, u;
+  float a, b;
+};
+__device__ __forceinline__ Line line_of(float3 P, float3 Q) {
+  Line L;
+  const float3 d = sub_rn(Q, P);
+  const float il = __frsqrt_rn(dot_rn(d, d));
+  L.u = make_float3(__fmul_rn(d.x, il), __fmul_rn(d.y, il), __fmul_rn(d.z, il));
+  L.a = dot_rn(P, L.u);
+  L.b = dot_rn(Q, L.u);
+  L.p = along(P, -L.a, L.u);
+  return L;
+}
+
+// info word of a tet record (its 13th float's bits): open faces 0-3 (by the
+// vertex they leave out, in mesh order), 4: mesh order is an even permutation
+// of a positively oriented tet, 5: not positively oriented (meets nothing)
+constexpr unsigned REC_EVEN = 16u, REC_SKIP = 32u;
+// the side of its canonical plane i the tet lies on (true: positive)
+__device__ __forceinline__ bool face_side(unsigned info, int i) { return ((info >> 4) & 1u) == (unsigned)(i & 1); }
+
+template <bool BATCHED>
+__global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell_mesh(
+    const float4* __restrict__ sites, const unsigned* __restrict__ knn, const ProbDesc* __restrict__ probs,
+    const int* __restrict__ site_prob, const ProbDesc lone, const float4* __restrict__ rec,
+    const int* __restrict__ tet_cell_start, const float4* __restrict__ tet_sph, const float* __restrict__ reach,
+    const unsigned* __restrict__ reach_max_bits, dmom4* __restrict__ mom, unsigned long long* __restrict__ stats,
+    unsigned* __restrict__ prob_secmiss, const int* __restrict__ in_list, const int* __restrict__ in_count,
+    int* __restrict__ work, int* __restrict__ out_list, int* __restrict__ out_count, const CellStore store,
+    int* __restrict__ esc_list, float* __restrict__ esc_r2, int* __restrict__ esc_count) {
+  __shared__ MeshSmem smem_all[MESH_WARPS];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  MeshSmem& S = smem_all[wib];
+  if (lane < WC_N) S.cnt[lane] = 0u;
+  __syncwarp();
+  const int n_items = *in_count;
+  for (;;) {
+    int it = 0;
+    if (lane == 0) it = atomicAdd(work, 1);
+    it = __shfl_sync(FULL, it, 0);
+    if (it >= n_items) break;
+    const int s = in_list[it];
+    const int pidx = BATCHED ? site_prob[s] : 0;
+#define PD(f) (BATCHED ? probs[pidx].f : lone.f)
+    const float4 seed = sites[s];
+    const int word = store.mnt[s];
+    const int nt = min(word & 255, MESH_VERTS);
+    unsigned flags = ((unsigned)word >> 8) & 255u;
+    const int K = PD(K);
+    const unsigned* const krow = knn + PD(knn_off) + (size_t)(s - PD(site_off)) * K;
+    const bool miss = (flags & SITE_SECMISS) && !(flags & SITE_COMPLETED);
+    const float dK2 = miss ? dist2(seed, sites[krow[K - 1]]) : FLT_MAX;
+
+    // -----------------------------------------------------------------
+    // the cell: its faces, vertices and edges
+    unsigned T[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int i = k * WARP + lane;
+      T[k] = i < nt ? store.mtri[(size_t)s * MESH_VERTS + i] : 0u;
+    }
+    for (int i = lane; i < MESH_ID_WORDS * 8; i += WARP) reinterpret_cast<unsigned*>(S.loc)[i] = 0u;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      if (k * WARP + lane < nt) {
+#pragma unroll
+        for (int e = 0; e < 3; ++e) S.loc[min(tri_at(T[k], e), (unsigned)(MESH_IDS - 1))] = 1;
+      }
+    __syncwarp();
+    int nf = 0;
+#pragma unroll
+    for (int w = 0; w < MESH_ID_WORDS; ++w) {
+      const int id = w * WARP + lane;
+      const bool has = S.loc[id] != 0;
+      const unsigned m = __ballot_sync(FULL, has);
+      const int f = min(nf + __popc(m & lt_mask), MESH_FACES - 1);
+      if (has) {
+        S.loc[id] = (unsigned char)f;
+        float4 P;
+        if (id < 4 + K) {
+          P = bisector_plane(seed, sites[krow[max(id - 4, 0)]]);
+        } else if (id < 4 + K + 2 * BOX_PLANES) {
+          P = start_plane(id - 4 - K, seed, cube_half_side(seed));
+        } else {
+          P = bisector_plane(seed, sites[store.faces[(size_t)s * PIECE_REC + min(id - (4 + K + 2 * BOX_PLANES), MESH_EXT - 1)]]);
+        }
+        S.plane[f] = P;
+      }
+      nf += __popc(m);
+    }
+    __syncwarp();
+    bool bad = nf > MESH_FACES || nt < 4;
+    nf = min(nf, MESH_FACES);
+    float lm = 0.f;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int i = k * WARP + lane;
+      if (i < nt) {
+        const unsigned a = S.loc[min(tri_at(T[k], 0), (unsigned)(MESH_IDS - 1))];
+        const unsigned b = S.loc[min(tri_at(T[k], 1), (unsigned)(MESH_IDS - 1))];
+        const unsigned c = S.loc[min(tri_at(T[k], 2), (unsigned)(MESH_IDS - 1))];
+        const float3 x = vertex_of(S.plane[a], S.plane[b], S.plane[c]);
+        const float r2 = norm2_rn(x);
+        S.vert[i] = make_float4(x.x, x.y, x.z, r2);
+        lm = fmaxf(lm, r2);
+        T[k] = pack_tri(a, b, c);
+        S.twin[a * MESH_FACES + b] = (unsigned char)i;
+        S.twin[b * MESH_FACES + c] = (unsigned char)i;
+        S.twin[c * MESH_FACES + a] = (unsigned char)i;
+      }
+    }
+    const float Rc = sqrtf(warp_max_nonneg(lm));
+    __syncwarp();
+    // an edge is the directed pair (p, q) of one vertex and (q, p) of another
+    int ne = 0;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (k * WARP >= nt) break;
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        const unsigned p = tri_at(T[k], e), q = tri_at(T[k], e == 2 ? 0 : e + 1);
+        const bool has = k * WARP + lane < nt && p < q;
+        const unsigned m = __ballot_sync(FULL, has);
+        const int pos = ne + __popc(m & lt_mask);
+        if (has && pos < MESH_EDGES)
+          S.edge[pos] = p | (q << 8) | ((unsigned)(k * WARP + lane) << 16) |
+                        ((unsigned)(S.twin[q * MESH_FACES + p] & (MESH_VERTS - 1)) << 24);
+        ne += __popc(m);
+      }
+    }
+    bad |= ne > MESH_EDGES || ne < 6;
+    ne = max(min(ne, MESH_EDGES), 1);
+    __syncwarp();
+    for (int i = lane; i < ne; i += WARP) {
+      const unsigned E = S.edge[i];
+      S.epq[i] = (unsigned short)(E & 0xffffu);
+      const float4 P = S.plane[E & 0xffu], Q = S.plane[(E >> 8) & 0xffu];
+      const float3 D = cross_rn(xyz(Q), xyz(P));  // from the end whose vertex holds (p, q)
+      const float dd = dot_rn(D, D);
+      const float3 a = cross_rn(xyz(P), D), b = cross_rn(D, xyz(Q));
+      const float i2 = __fdividef(-1.f, dd), i1 = rsqrtf(dd);
+      const float3 u = make_float3(__fmul_rn(D.x, i1), __fmul_rn(D.y, i1), __fmul_rn(D.z, i1));
+      S.epos[i] = make_float4(__fmul_rn(i2, __fmaf_rn(Q.w, a.x, __fmul_rn(P.w, b.x))),
+                              __fmul_rn(i2, __fmaf_rn(Q.w, a.y, __fmul_rn(P.w, b.y))),
+                              __fmul_rn(i2, __fmaf_rn(Q.w, a.z, __fmul_rn(P.w, b.z))),
+                              dot_rn(xyz(S.vert[(E >> 16) & 0xffu]), u));
+      S.edir[i] = make_float4(u.x, u.y, u.z, dot_rn(xyz(S.vert[E >> 24]), u));
+    }
+    __syncwarp();
+
+    // -----------------------------------------------------------------
+    // the tets.  When the first apex (the site) turns out far from what is left
+    // of the cell: again for the mean point of its edges there (their lengths
+    // and moments in place of their terms, no triangles), and from that point
+    float3 X = make_float3(0.f, 0.f, 0.f);
+    float pr2 = 0.f, vol = 0.f, mx = 0.f, my = 0.f, mz = 0.f;
+    const int dim = PD(dim), cbase = PD(cell_off);
+    const float R = __fadd_rn(fminf(__fmaf_rn(PD(rt_max), 1.001f, Rc), __uint_as_float(reach_max_bits[pidx])), 0.01f);
+    const float h = 1000.f / (float)dim;
+    const int j0 = grid_axis(seed.y - R, dim), k0 = grid_axis(seed.z - R, dim);
+    const int nj = grid_axis(seed.y + R, dim) - j0 + 1;
+    const int nrow = nj * (grid_axis(seed.z + R, dim) - k0 + 1);
+    for (int round = 0; round < 3 && !bad; ++round) {
+      MeshSum sum;
+      float far2 = 0.f;
+      // a piece [a, b] of an edge: k = det(F1 - F0, p, u) (b - a), and the
+      // moment k1 (F1 + a + b) - k0 (F0 + a + b)
+      for (int i = lane; i < ne; i += WARP) {
+        const unsigned pq = S.epq[i];
+        const float3 F0 = foot_of(S.plane[pq & 0xffu], X), F1 = foot_of(S.plane[pq >> 8], X);
+        const float3 p = sub_rn(xyz(S.epos[i]), X), cr = cross_rn(p, xyz(S.edir[i]));
+        const float k0 = dot_rn(F0, cr), k1 = dot_rn(F1, cr), k = __fsub_rn(k1, k0), k2 = 2.f * k;
+        S.eterm[i] = round == 1 ? make_float4(2.f * p.x, 2.f * p.y, 2.f * p.z, 1.f)
+                                : make_float4(__fmaf_rn(k2, p.x, cross_term(k1, F1.x, k0, F0.x)),
+                                              __fmaf_rn(k2, p.y, cross_term(k1, F1.y, k0, F0.y)),
+                                              __fmaf_rn(k2, p.z, cross_term(k1, F1.z, k0, F0.z)), k);
+      }
+      __syncwarp();
+      int nq = 0, row0 = 0, f0 = 0, total = 0, incl = 0;
+      bool more = true;
+      while (more || nq > 0) {
+        // candidates to the queue: rows of centroid cells, 32 rows at a time,
+        // each cut to the ball of radius R, then 32 tets at a time
+        while (more && nq < WARP) {
+          if (f0 >= total) {
+            if (row0 >= nrow) {
+              more = false;
+              break;
+            }
+            const int r = row0 + lane;
+            int len = 0, rb = 0;
+            if (r < nrow) {
+              const int j = j0 + r % nj, k = k0 + r / nj;
+              // (the cells at the ends of the grid also hold what lies beyond)
+              const float m = 0.01f;
+              float lo = j == 0 ? -FLT_MAX : __fmaf_rn((float)j, h, -m);
+              float hi = j == dim - 1 ? FLT_MAX : __fmaf_rn((float)(j + 1), h, m);
+              const float dy = fmaxf(fmaxf(lo - seed.y, seed.y - hi), 0.f);
+              lo = k == 0 ? -FLT_MAX : __fmaf_rn((float)k, h, -m);
+              hi = k == dim - 1 ? FLT_MAX : __fmaf_rn((float)(k + 1), h, m);
+              const float dz = fmaxf(fmaxf(lo - seed.z, seed.z - hi), 0.f);
+              const float left = __fmaf_rn(__fmul_rn(R, R), 1.0001f, -__fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
+              if (left >= 0.f) {
+                const float w = __fadd_rn(sqrtf(left), m);
+                const int row = cbase + dim * (j + dim * k);
+                rb = tet_cell_start[row + grid_axis(seed.x - w, dim)];
+                len = tet_cell_start[row + grid_axis(seed.x + w, dim) + 1] - rb;
+              }
+            }
+            row0 += WARP;
+            incl = len;
+#pragma unroll
+            for (int o = 1; o < WARP; o <<= 1) {
+              const int y = __shfl_up_sync(FULL, incl, o);
+              if (lane >= o) incl += y;
+            }
+            total = __shfl_sync(FULL, incl, WARP - 1);
+            f0 = 0;
+            __syncwarp();
+            S.rng[0][lane] = rb;
+            S.rng[1][lane] = incl - len;
+            __syncwarp();
+            continue;
+          }
+          const int f = f0 + lane;
+          int lo = 0;  // the row holding f
+#pragma unroll
+          for (int step = 16; step > 0; step >>= 1) {
+            const int v = __shfl_sync(FULL, incl, lo + step - 1);
+            if (v <= f) lo += step;
+          }
+          const int idx = S.rng[0][lo] + f - S.rng[1][lo];
+          bool meets = false;
+          if (f < total) {
+            // bounding spheres (the cell lies within Rc of its site), and the
+            // tet's reach: beyond it every point of the tet has a nearer site
+            const float4 sp = tet_sph[idx];
+            const float ex = sp.x - seed.x, ey = sp.y - seed.y, ez = sp.z - seed.z;
+            const float dm = sqrtf(dot3_rn(ex, ey, ez, ex, ey, ez));
+            meets = dm <= __fmaf_rn(__fadd_rn(Rc, sp.w), 1.0001f, 1e-3f) && dm <= __fmaf_rn(reach[idx], 1.0001f, 1e-2f);
+          }
+          const unsigned m = __ballot_sync(FULL, meets);
+          if (meets) S.queue[nq + __popc(m & lt_mask)] = idx;
+          nq += __popc(m);
+          if (lane == 0) S.cnt[WC_CAND] += (unsigned)min(WARP, total - f0);
+          f0 += WARP;
+        }
+        if (nq == 0) break;
+        __syncwarp();
+        // 32 of them (the rest of the queue at the end), one per lane: a tet
+        // with all four corners strictly outside one face cannot meet the cell
+        const int take = min(nq, WARP);
+        const int idx = lane < take ? S.queue[lane] : 0;
+        bool alive = lane < take;
+        float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0, r2 = r0;
+        unsigned info = 0u;
+        if (alive) {
+          const float4* q = rec + 4 * (size_t)idx;
+          r0 = q[0];
+          r1 = q[1];
+          r2 = q[2];
+          info = __float_as_uint(q[3].x);
+          alive = !(info & REC_SKIP);
+        }
+        const float3 A0 = make_float3(r0.x, r0.y, r0.z), A1 = make_float3(r0.w, r1.x, r1.y),
+                     A2 = make_float3(r1.z, r1.w, r2.x), A3 = make_float3(r2.y, r2.z, r2.w);
+        const float3 sd = make_float3(seed.x, seed.y, seed.z);
+        const float3 c0 = sub_rn(A0, sd), c1 = sub_rn(A1, sd), c2 = sub_rn(A2, sd), c3 = sub_rn(A3, sd);
+        for (int f = 0; f < nf; ++f) {
+          if (!__any_sync(FULL, alive)) break;
+          const float4 P = S.plane[f];
+          const float e = fmaxf(fmaxf(eval4(P, c0), eval4(P, c1)), fmaxf(eval4(P, c2), eval4(P, c3)));
+          alive &= !(e < 0.f);
+        }
+        const unsigned am = __ballot_sync(FULL, alive);
+        const int nb = __popc(am);
+        // the rest of the queue to its front
+        const int rest = nq - take;
+        const int move = lane < rest ? S.queue[take + lane] : 0;
+        __syncwarp();
+        if (lane < rest) S.queue[lane] = move;
+        nq = rest;
+        if (lane == 0) {
+          S.cnt[WC_CULLED] += (unsigned)(take - nb);
+          S.cnt[WC_CLIPPED] += (unsigned)nb;
+          S.cnt[WC_CULLTESTS] += (unsigned)(take * nf);
+          S.cnt[WC_CONFLICT] += (unsigned)(8 * ne * nb);
+        }
+        if (alive) {
+          const int pos = __popc(am & lt_mask);
+          auto face = [&](int i, float3 a, float3 b, float3 c, float3 ca) {
+            const float3 n = cross_rn(sub_rn(b, a), sub_rn(c, a));
+            S.tp[pos][i] = make_float4(n.x, n.y, n.z, -dot_rn(n, ca));
+          };
+          face(0, A1, A2, A3, c1);
+          face(1, A0, A2, A3, c0);
+          face(2, A0, A1, A3, c0);
+          face(3, A0, A1, A2, c0);
+          unsigned far = 0u;
+          if (miss) {
+            const float m2 = fmaxf(fmaxf(dot_rn(c0, c0), dot_rn(c1, c1)), fmaxf(dot_rn(c2, c2), dot_rn(c3, c3)));
+            far = !(dK2 > __fmaf_rn(4.f * m2, 1.0001f, 1e-4f)) ? 64u : 0u;
+          }
+          S.tidx[pos] = idx;
+          S.tinf[pos] = (unsigned char)((info & 31u) | far);
+          S.thit[pos] = 0;
+        }
+        __syncwarp();
+
+        // what each tet holds of each edge, a pair per lane
+        {
+          int b = lane / ne, e = lane - b * ne;
+          const int db = WARP / ne, de = WARP - db * ne;
+          for (int w = lane; w < nb * ne; w += WARP) {
+            const float4 ep = S.epos[e], eu = S.edir[e];
+            const float3 p = xyz(ep), u = xyz(eu);
+            const bool even = (S.tinf[b] & REC_EVEN) != 0u;  // sides: -, +, -, + of an even tet
+            float lo = ep.w, hi = eu.w;
+            bool up;
+            float t = line_at(S.tp[b][0], p, u, up);
+            if (up != even) lo = fmaxf(lo, t); else hi = fminf(hi, t);
+            t = line_at(S.tp[b][1], p, u, up);
+            if (up == even) lo = fmaxf(lo, t); else hi = fminf(hi, t);
+            t = line_at(S.tp[b][2], p, u, up);
+            if (up != even) lo = fmaxf(lo, t); else hi = fminf(hi, t);
+            t = line_at(S.tp[b][3], p, u, up);
+            if (up == even) lo = fmaxf(lo, t); else hi = fminf(hi, t);
+            if (hi > lo) {
+              const float4 T4 = S.eterm[e];
+              const float d = __fsub_rn(hi, lo), m = __fadd_rn(hi, lo), k = __fmul_rn(T4.w, d), km = __fmul_rn(k, m);
+              sum.v = __fadd_rn(sum.v, k);
+              sum.mag = __fadd_rn(sum.mag, fabsf(k));
+              sum.x = __fadd_rn(sum.x, __fmaf_rn(km, u.x, __fmul_rn(d, T4.x)));
+              sum.y = __fadd_rn(sum.y, __fmaf_rn(km, u.y, __fmul_rn(d, T4.y)));
+              sum.z = __fadd_rn(sum.z, __fmaf_rn(km, u.z, __fmul_rn(d, T4.z)));
+              far2 = fmaxf(far2, __fadd_rn(dot_rn(p, p), fmaxf(lo * lo, hi * hi)));
+              S.thit[b] = 1;
+            }
+            b += db;
+            e += de;
+            if (e >= ne) {
+              e -= ne;
+              ++b;
+            }
+          }
+        }
+        __syncwarp();
+        const unsigned hits = __ballot_sync(FULL, lane < nb && S.thit[lane] != 0);
+        const unsigned farm = __ballot_sync(FULL, lane < nb && (S.tinf[lane] & 64u) != 0u);
+        unsigned open = __ballot_sync(FULL, lane < nb && round != 1 && (S.tinf[lane] & 15u) != 0u);
+        if (lane == 0) {
+          S.cnt[WC_CONTRIB] += (unsigned)__popc(hits);
+          S.cnt[WC_EMPTY] += (unsigned)(nb - __popc(hits));
+        }
+        const float3 site = make_float3(seed.x, seed.y, seed.z);
+        // the tets reaching beyond half the K-th neighbour's distance, of a
+        // cell its K neighbours left open: how far their pieces reach (the
+        // tets' edges, one per lane; the cell's edges are in far2)
+        if ((farm >> lane) & 1u) S.thit[__popc(farm & lt_mask)] = (unsigned char)lane;
+        __syncwarp();
+        for (int w = lane; w < 6 * __popc(farm); w += WARP) {
+          const int e = w % 6;
+          const float4* q = rec + 4 * (size_t)S.tidx[S.thit[w / 6]];
+          const float4 r0 = q[0], r1 = q[1], r2 = q[2];
+          const float3 c0 = make_float3(r0.x, r0.y, r0.z), c1 = make_float3(r0.w, r1.x, r1.y),
+                       c2 = make_float3(r1.z, r1.w, r2.x), c3 = make_float3(r2.y, r2.z, r2.w);
+          const float3 P = e < 3 ? c0 : e < 5 ? c1 : c2, Q = e == 0 ? c1 : (e == 1 || e == 3) ? c2 : c3;
+          const Line L = line_of(sub_rn(P, site), sub_rn(Q, site));
+          float lo = L.a, hi = L.b;
+          for (int f = 0; f < nf; ++f) {
+            bool up;
+            const float t = line_at(S.plane[f], L.p, L.u, up);
+            if (up) lo = fmaxf(lo, t); else hi = fminf(hi, t);
+          }
+          if (hi > lo) far2 = fmaxf(far2, __fadd_rn(dot_rn(L.p, L.p), fmaxf(lo * lo, hi * hi)));
+        }
+
+        for (; open != 0u; open &= open - 1u) {
+          const int b = __ffs(open) - 1;
+          const unsigned inf = S.tinf[b];
+          // its corners in mesh order, for its open faces
+          const float4* q = rec + 4 * (size_t)S.tidx[b];
+          const float4 r0 = q[0], r1 = q[1], r2 = q[2];
+          const float3 c[4] = {sub_rn(make_float3(r0.x, r0.y, r0.z), site), sub_rn(make_float3(r0.w, r1.x, r1.y), site),
+                               sub_rn(make_float3(r1.z, r1.w, r2.x), site), sub_rn(make_float3(r2.y, r2.z, r2.w), site)};
+#pragma unroll 1
+          for (int i = 0; i < 4; ++i) {
+            if (!((inf >> i) & 1u)) continue;
+            // triangle (t0, t1, t2): face i, in mesh order
+            const float3 t0 = i == 0 ? c[1] : c[0], t1 = i <= 1 ? c[2] : c[1], t2 = i <= 2 ? c[3] : c[2];
+            bool out = false;
+            for (int f = lane; f < nf; f += WARP) {
+              const float4 P = S.plane[f];
+              out |= fmaxf(fmaxf(eval4(P, t0), eval4(P, t1)), eval4(P, t2)) < 0.f;
+              S.slot[0][f].w = 0.f;
+              S.slot[1][f].w = 0.f;
+            }
+            if (__any_sync(FULL, out)) continue;
+            __syncwarp();
+            const float4 PT = S.tp[b][i];
+            const bool side = face_side(inf, i);
+            // the cell's edges across its plane: where each face's line with
+            // it begins and ends
+            for (int e = lane; e < ne; e += WARP) {
+              const float4 ep = S.epos[e], eu = S.edir[e];
+              bool up;
+              const float t = line_at(PT, xyz(ep), xyz(eu), up);
+              if (t > ep.w && t < eu.w) {
+                const float3 x = along(xyz(ep), t, xyz(eu));
+                const int in = up == side ? 0 : 1;
+                const unsigned pq = S.epq[e];
+                S.slot[in][pq & 0xffu] = make_float4(x.x, x.y, x.z, 1.f);
+                S.slot[1 - in][pq >> 8] = make_float4(x.x, x.y, x.z, 1.f);
+              }
+            }
+            // its sides: 0 (t1, t2), 1 (t0, t2), 2 (t0, t1)
+            const Line L0 = line_of(t1, t2), L1 = line_of(t0, t2), L2 = line_of(t0, t1);
+            const float3 FT = foot_of(PT, X);
+            __syncwarp();
+            float l0 = L0.a, h0 = L0.b, l1 = L1.a, h1 = L1.b, l2 = L2.a, h2 = L2.b;
+            for (int f = lane; f < nf; f += WARP) {
+              const float4 P = S.plane[f];
+              bool up0, up1, up2;
+              const float w0 = line_at(P, L0.p, L0.u, up0), w1 = line_at(P, L1.p, L1.u, up1),
+                          w2 = line_at(P, L2.p, L2.u, up2);
+              if (up0) l0 = fmaxf(l0, w0); else h0 = fminf(h0, w0);
+              if (up1) l1 = fmaxf(l1, w1); else h1 = fminf(h1, w1);
+              if (up2) l2 = fmaxf(l2, w2); else h2 = fminf(h2, w2);
+              const float4 a4 = S.slot[0][f], b4 = S.slot[1][f];
+              if (a4.w != 0.f && b4.w != 0.f) {
+                float3 a = xyz(a4), bb = xyz(b4);
+                bool keep = true;
+                // the side planes: the tet's faces that leave out t0, t1, t2
+                auto cut = [&](int o, const Line& L, float w) {
+                  const float4 PS = S.tp[b][o];
+                  const bool pos = face_side(inf, o);
+                  const float va = eval4(PS, a), vb = eval4(PS, bb);
+                  const bool oa = pos ? va < 0.f : va > 0.f, ob = pos ? vb < 0.f : vb > 0.f;
+                  keep &= !(oa && ob);
+                  if (oa != ob) {
+                    const float3 y = along(L.p, w, L.u);
+                    if (oa) a = y; else bb = y;
+                  }
+                };
+                cut(i == 0 ? 1 : 0, L0, w0);
+                cut(i <= 1 ? 2 : 1, L1, w1);
+                cut(i <= 2 ? 3 : 2, L2, w2);
+                if (keep) {
+                  const float3 aX = sub_rn(a, X), bX = sub_rn(bb, X);
+                  const float3 cr = cross_rn(aX, bX), ab = make_float3(__fadd_rn(aX.x, bX.x), __fadd_rn(aX.y, bX.y), __fadd_rn(aX.z, bX.z));
+                  const float3 F = foot_of(P, X);
+                  sum.add(dot_rn(F, cr), F, ab);
+                  sum.add(-dot_rn(FT, cr), FT, ab);
+                }
+              }
+            }
+            // the sides inside the cell (lanes 0-2), walked around the inward
+            // normal
+            l0 = redux_max(l0);
+            l1 = redux_max(l1);
+            l2 = redux_max(l2);
+            h0 = redux_min(h0);
+            h1 = redux_min(h1);
+            h2 = redux_min(h2);
+            const float lo = lane == 0 ? l0 : lane == 1 ? l1 : l2, hi = lane == 0 ? h0 : lane == 1 ? h1 : h2;
+            if (lane < 3 && hi > lo) {
+              const float3 p = lane == 0 ? L0.p : lane == 1 ? L1.p : L2.p, u = lane == 0 ? L0.u : lane == 1 ? L1.u : L2.u;
+              const float3 a = along(p, lo, u), bb = along(p, hi, u);
+              const float3 aX = sub_rn(a, X), bX = sub_rn(bb, X);
+              const float3 cr = cross_rn(aX, bX), ab = make_float3(__fadd_rn(aX.x, bX.x), __fadd_rn(aX.y, bX.y), __fadd_rn(aX.z, bX.z));
+              const float k6 = dot_rn(FT, cr);
+              sum.add((side == (lane != 1)) ? -k6 : k6, FT, ab);
+            }
+            __syncwarp();
+          }
+        }
+        __syncwarp();
+      }
+      const float v6 = warp_sum(sum.v), x24 = warp_sum(sum.x), y24 = warp_sum(sum.y), z24 = warp_sum(sum.z);
+      const float mag = warp_sum(sum.mag);
+      pr2 = fmaxf(pr2, warp_max_nonneg(far2));
+      if (round == 1) {
+        if (!(v6 > 0.f)) break;
+        const float w = __fdividef(0.5f, v6);
+        X = make_float3(__fmul_rn(x24, w), __fmul_rn(y24, w), __fmul_rn(z24, w));
+        continue;
+      }
+      vol = __fmul_rn(v6, 1.f / 6.f);
+      mx = __fmaf_rn(x24, 1.f / 24.f, __fmul_rn(vol, X.x));
+      my = __fmaf_rn(y24, 1.f / 24.f, __fmul_rn(vol, X.y));
+      mz = __fmaf_rn(z24, 1.f / 24.f, __fmul_rn(vol, X.z));
+      // large terms for a small sum: the apex is far from what is left
+      if (mag <= MESH_APEX_RATIO * v6 || mag == 0.f) break;
+    }
+    bad |= !(isfinite(vol) && isfinite(mx) && isfinite(my) && isfinite(mz));
+    if (bad) {
+      // degenerate: the 128-vertex pass clips a copy of the cell by each tet
+      // (a completed cell keeps its earlier moments)
+      if (lane == 0) {
+        if (out_list) {
+          out_list[atomicAdd(out_count, 1)] = s;
+          S.cnt[WC_REDO]++;
+          store.nt[s] = 0;
+          if (store.flags) store.flags[s] = (unsigned char)(flags | SITE_HANDED | SITE_REDO);
+        } else {
+          S.cnt[WC_UNRESOLVED]++;
+          if (store.flags) store.flags[s] = (unsigned char)(flags | SITE_UNRESOLVED);
+        }
+      }
+      __syncwarp();
+      continue;
+    }
+    if (lane == 0) {
+      unsigned f = flags | SITE_HANDED;
+      mom[s] = make_dmom4((double)vol, (double)mx, (double)my, (double)mz);
+      if (esc_list && miss) {
+        // exact where it meets the mesh when that lies within half the K-th
+        // neighbour's distance; else completed by the completion pass
+        if (!(dK2 > __fmaf_rn(4.f * pr2, 1.0001f, 1e-4f))) {
+          const int pos = atomicAdd(esc_count, 1);
+          esc_list[pos] = s;
+          esc_r2[pos] = pr2;
+          f |= SITE_UNRESOLVED;
+        }
+      }
+      if (miss) {
+        S.cnt[WC_SECMISS]++;
+        if (prob_secmiss) atomicAdd(prob_secmiss + pidx, 1u);
+      }
+      if (flags & SITE_COMPLETED) S.cnt[WC_COMPLETED]++;
+      if (store.flags) store.flags[s] = (unsigned char)f;
+    }
+    __syncwarp();
+#undef PD
+  }
+  if (stats && lane < WC_N && S.cnt[lane]) atomicAdd(stats + stat_slot(lane), (unsigned long long)S.cnt[lane]);
+}
+
+}  // namespace vgb

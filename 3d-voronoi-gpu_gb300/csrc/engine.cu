@@ -21,6 +21,7 @@
 #include <cstring>
 #include <algorithm>
 #include <new>
+#include <thread>
 #include <vector>
 
 #include "../../include/voronoi_gb300.h"
@@ -61,7 +62,8 @@ struct vgb_engine {
   float4* tet_sph = nullptr;       // exact form: tet bounding spheres (centroid-cell order)
   unsigned* reach_max = nullptr;   // exact form: float bits of the largest reach
   int* redo_list = nullptr;        // cell-tet: the clip passes' site lists (6n)
-  int* redo_count = nullptr;       // clip hand-off and work counters, kNN work counters (12)
+  int* redo_count = nullptr;       // clip hand-off and work counters, kNN work counters
+  float4* rec = nullptr;           // exact form, float: tet records of the mesh pass
   vgb::CellStore store{};          // cells the first clip pass built and handed on, cell records (by site)
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // [update]
   cudaEvent_t ev[VGB_PHASES + 1] = {};
@@ -176,7 +178,8 @@ void free_engine(vgb_engine* e) {
   void* bufs[] = {e->verts, e->tets, e->sites, e->sites_tmp, e->cell_start, e->cell_fill, e->site_cell,
                   e->scan_tmp, e->pos_of_id, e->tet_order, e->tet_cell_start, e->knn, e->cand, e->site_start, e->site_fill, e->site_tets, e->mom, e->mom_f,
                   e->io_stage, e->stats, e->field, e->field_sat, e->reach, e->reach_max, e->tet_sph,
-                  e->redo_list, e->redo_count, e->store.tri, e->store.nt, e->store.flags, e->store.faces};
+                  e->redo_list, e->redo_count, e->store.tri, e->store.nt, e->store.flags, e->store.faces, e->store.mtri,
+                  e->store.mnt, e->rec};
   for (void* b : bufs)
     if (b) cudaFree(b);
   if (e->st) cudaStreamDestroy(e->st);
@@ -245,6 +248,8 @@ int run_pass(vgb_engine* e, int update) {
 // (first-pass lane groups of 8 or 16, one-warp pass of 64 or 96 vertices)
 // with 8-warp kNN blocks, then the fastest of them with 4-warp kNN blocks,
 // then with the other clip form (copies of the cell or pieces from the tets).
+// With the mesh pass there is no clip by each tet: no 96-vertex shapes and no
+// other form.
 int tune_shapes(vgb_engine* e) {
   static const int shapes[4][2] = {{8, 2}, {16, 2}, {8, 3}, {16, 3}};
   auto timed = [&](const KernelShape& s, float* ms) {
@@ -266,6 +271,7 @@ int tune_shapes(vgb_engine* e) {
   float best_ms = 1e30f;
   int rc = VGB_OK;
   for (auto& sh : shapes) {
+    if (e->store.rec && sh[1] != 2) continue;
     KernelShape s{};
     s.pieces = best.pieces;
     s.build_g = sh[0];
@@ -280,7 +286,7 @@ int tune_shapes(vgb_engine* e) {
     float ms = 0.f;
     if (!(rc = timed(s, &ms)) && ms < best_ms) best = s, best_ms = ms;
   }
-  if (!rc) {
+  if (!rc && !e->store.rec) {
     // the other clip form
     KernelShape s = best;
     s.pieces = 1 - best.pieces;
@@ -410,6 +416,8 @@ int vgb_engine_create(vgb_engine** out, const vgb_config* cfg_in, const float* v
   int rc = VGB_OK;
   size_t pairs = (size_t)n_tet * e->tk;
   const bool exact_form = cfg.method == VGB_METHOD_CELL_TET && cfg.exact;
+  const bool mesh_form = 
+      exact_form && runs_mesh_pass(cfg.robust_predicates != 0, cfg.tet_pieces != 0, n_tet, n_site);
   size_t scan_n = std::max((size_t)e->ncell + 1, (size_t)n_site + 1);
   if ((rc = dalloc(&e->verts, n_vert)) || (rc = dalloc(&e->tets, n_tet)) || (rc = dalloc(&e->sites, n_site)) ||
       (rc = dalloc(&e->sites_tmp, n_site)) || (rc = dalloc(&e->cell_start, e->ncell + 1)) ||
@@ -419,13 +427,15 @@ int vgb_engine_create(vgb_engine** out, const vgb_config* cfg_in, const float* v
       (rc = dalloc(&e->knn, (size_t)n_site * e->K)) || (rc = dalloc(&e->cand, exact_form ? 1 : pairs)) ||
       (rc = dalloc(&e->site_start, (size_t)n_site + 1)) || (rc = dalloc(&e->site_fill, n_site)) ||
       (rc = dalloc(&e->site_tets, cfg.method != VGB_METHOD_PLAIN && !exact_form ? pairs : 1)) ||
-      (rc = dalloc(&e->mom, n_site)) || (rc = dalloc(&e->redo_list, 6 * (size_t)n_site)) || (rc = dalloc(&e->redo_count, 12)) || (rc = dalloc(&e->mom_f, cfg.method == VGB_METHOD_PLAIN ? n_site : 1)) ||
+      (rc = dalloc(&e->mom, n_site)) || (rc = dalloc(&e->redo_list, 6 * (size_t)n_site)) || (rc = dalloc(&e->redo_count, CLIP_COUNTERS)) || (rc = dalloc(&e->mom_f, cfg.method == VGB_METHOD_PLAIN ? n_site : 1)) ||
       (rc = dalloc(&e->io_stage, 3 * (size_t)std::max(n_site, n_vert))) ||
       (rc = dalloc(&e->stats, VGB_STAT_COUNT)) ||
       (rc = dalloc(&e->store.tri, exact_form ? (size_t)n_site * STORE_VERTS : 1)) ||
       (rc = dalloc(&e->store.nt, exact_form ? (size_t)n_site : 1)) ||
       (rc = dalloc(&e->store.flags, cfg.method == VGB_METHOD_CELL_TET ? (size_t)n_site : 1)) ||
-      (rc = dalloc(&e->store.faces, cfg.method == VGB_METHOD_CELL_TET ? (size_t)n_site * PIECE_REC : 1))) {
+      (rc = dalloc(&e->store.faces, cfg.method == VGB_METHOD_CELL_TET ? (size_t)n_site * PIECE_REC : 1)) ||
+      (rc = dalloc(&e->store.mtri, mesh_form ? (size_t)n_site * MESH_VERTS : 1)) ||
+      (rc = dalloc(&e->store.mnt, mesh_form ? (size_t)n_site : 1))) {
     free_engine(e);
     return rc;
   }
@@ -497,7 +507,9 @@ int vgb_engine_create(vgb_engine** out, const vgb_config* cfg_in, const float* v
     e->fdim = (int)std::min(512.0, std::max(8.0, std::ceil(3000.0 / spacing)));
     std::vector<unsigned char> field;
     std::vector<unsigned> field_sat;
-    build_inside_field(verts, n_vert, tets, n_tet, e->fdim, field, field_sat);
+    std::vector<unsigned char> open_faces;
+    build_inside_field(verts, n_vert, tets, n_tet, e->fdim, field, field_sat, open_faces,
+                       std::max(1, std::min(8, (int)std::thread::hardware_concurrency())));
     e->prob.fdim = e->fdim;
     if ((rc = dalloc(&e->field, field.size())) || (rc = dalloc(&e->field_sat, field_sat.size())) ||
         (rc = dalloc(&e->reach, n_tet)) ||
@@ -506,6 +518,21 @@ int vgb_engine_create(vgb_engine** out, const vgb_config* cfg_in, const float* v
       return rc;
     }
     if (tet_spheres(e->verts, e->tets, e->tet_order, n_tet, e->tet_sph, e->st)) { free_engine(e); return VGB_ERR_CUDA; }
+    if (mesh_form) {
+      unsigned char* d_open = nullptr;
+      if ((rc = dalloc(&d_open, n_tet)) || (rc = dalloc(&e->rec, 4 * (size_t)n_tet))) {
+        if (d_open) cudaFree(d_open);
+        free_engine(e);
+        return rc;
+      }
+      ce = cudaMemcpyAsync(d_open, open_faces.data(), (size_t)n_tet, cudaMemcpyHostToDevice, e->st);
+      if (ce == cudaSuccess && tet_records(e->verts, e->tets, e->tet_order, d_open, n_tet, e->rec, e->st))
+        ce = cudaErrorUnknown;
+      if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->st);
+      cudaFree(d_open);
+      if (ce != cudaSuccess) { set_error("tet records: %s", cudaGetErrorString(ce)); free_engine(e); return VGB_ERR_CUDA; }
+      e->store.rec = e->rec;
+    }
     ce = cudaMemcpy(e->field, field.data(), field.size(), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess)
       ce = cudaMemcpy(e->field_sat, field_sat.data(), sizeof(unsigned) * field_sat.size(), cudaMemcpyHostToDevice);

@@ -886,6 +886,41 @@ int tet_spheres(const float4* verts, const int4* tets, const int* tet_order, int
   return 0;
 }
 
+// The mesh pass's tets (once per mesh and grid): corners by vertex index.
+__global__ void k_tet_records(const float4* __restrict__ verts, const int4* __restrict__ tets,
+                              const int* __restrict__ tet_order, const unsigned char* __restrict__ open_faces,
+                              int n_tet, float4* __restrict__ rec) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n_tet) return;
+  const int t = tet_order[q];
+  const int4 v = tets[t];
+  int i0 = v.x, i1 = v.y, i2 = v.z, i3 = v.w;
+  auto order = [](int& a, int& b) {
+    const int lo = min(a, b), hi = max(a, b);
+    a = lo;
+    b = hi;
+  };
+  order(i0, i1);
+  order(i2, i3);
+  order(i0, i2);
+  order(i1, i3);
+  order(i1, i2);
+  const float4 a = verts[i0], b = verts[i1], c = verts[i2], d = verts[i3];
+  float4* out = rec + 4 * (size_t)q;
+  out[0] = make_float4(a.x, a.y, a.z, b.x);
+  out[1] = make_float4(b.y, b.z, c.x, c.y);
+  out[2] = make_float4(c.z, d.x, d.y, d.z);
+  out[3] = make_float4(__uint_as_float((unsigned)open_faces[t]), 0.f, 0.f, 0.f);
+}
+
+int tet_records(const float4* verts, const int4* tets, const int* tet_order, const unsigned char* open_faces, int n_tet,
+                float4* rec, cudaStream_t st) {
+  if (n_tet <= 0) return 0;
+  k_tet_records<<<(n_tet + 255) / 256, 256, 0, st>>>(verts, tets, tet_order, open_faces, n_tet, rec);
+  VGB_CUDA_TRY(cudaGetLastError());
+  return 0;
+}
+
 int tets_by_cell(const float4* verts, const int4* tets, int n_tet, long long ncell, const ProbDesc* probs,
                  const int* tet_prob, const ProbDesc& lone, int* tet_cell_start, int* cell_fill, int* tcell,
                  int* tet_order, int* scan_tmp, cudaStream_t st) {

@@ -210,6 +210,13 @@ int tet_reach(const float4* sites, const int* cell_start, const ProbDesc* probs,
               unsigned* reach_max_bits, cudaStream_t st);
 // Bounding spheres (centroid, radius) of the tets in centroid-cell order.
 int tet_spheres(const float4* verts, const int4* tets, const int* tet_order, int n_tet, float4* sph, cudaStream_t st);
+// The tets for the mesh pass, in centroid-cell order: corners by ascending
+// vertex index (12 floats), an info word (bits 0-3: the face that leaves out
+// the i-th corner is open; 4: that corner order is an even permutation of a
+// positively oriented tet; 5: not positively oriented), 3 spare words.
+// open_faces: bits 0-5 per tet in input order, from build_inside_field.
+int tet_records(const float4* verts, const int4* tets, const int* tet_order, const unsigned char* open_faces, int n_tet,
+                float4* rec, cudaStream_t st);
 // Tets sorted by the grid cell of their float32 centroid in their problem's
 // grid (once per mesh): tet_cell_start ncell + 1 ints, cell_fill ncell
 // scratch, tcell n_tet scratch, tet_order n_tet ints.
@@ -253,12 +260,38 @@ struct CellStore {
   int* nt;               // [n]
   unsigned char* flags;  // [n] SITE_* bits of the last pass (cell-tet method), may be null
   unsigned* faces;       // [n][PIECE_REC] cell records for the pieces pass (cell-tet method), may be null
+  // The mesh pass (exact form, float): the finished cells handed to it -- at
+  // most MESH_VERTS plane-id triples, their count | outcome bits << 8 -- and
+  // the tets it reads, 64 bytes each in centroid-cell order (null: the passes
+  // that clip by every tet run instead).
+  unsigned* mtri;        // [n][MESH_VERTS]
+  int* mnt;              // [n]
+  const float4* rec;     // [n_tet][4], from tet_records
 };
 // A cell record of the one-warp pass for the pieces pass: its face count,
 // radius (float bits) and outcome bits so far, a spare word, then its face
 // plane ids (8 bits each, at most PIECE_FACES).
 constexpr int PIECE_FACES = 64;
 constexpr int PIECE_REC = 4 + PIECE_FACES / 4;
+// The mesh pass takes cells of at most this many vertices; a cell of the
+// completion pass names the sites beyond its K nearest (at most MESH_EXT) in
+// its record.
+constexpr int MESH_VERTS = 64;
+constexpr int MESH_EXT = PIECE_REC;
+
+// Whether the exact cell-tet form of a problem (or batch) runs the mesh pass
+// (clip_mesh.cuh): with float predicates, it does.  It is faster than clipping by each tet
+// at every size and mesh measured (Lloyd iteration, us: 20k sites in 48k tets
+// 610 -> 290, 100k in 6 tets 1,955 -> 1,020, 1M in 1.96M 10,100 -> 7,400); the
+// pieces pass is left to callers who ask for it on a mesh of fewer than a tet
+// per 256 sites, where its pieces outgrow their lane groups and the counters
+// say so (3,000 sites in 6 tets: 350 us, with the mesh pass 280).
+inline bool runs_mesh_pass(bool robust, bool tet_pieces, long long n_tet, long long n_site) {
+  return !robust && !(tet_pieces && n_tet * 256 < n_site);
+}
+
+// Counters of the clip passes (clip_kernels.cuh lists them).
+constexpr int CLIP_COUNTERS = 16;
 
 int clip_site_major(bool cell_tet, const float4* sites, int n, unsigned* knn, const ProbDesc* probs,
                     const int* site_prob, const ProbDesc& lone, const float4* verts, const int4* tets,
@@ -280,8 +313,8 @@ int clip_site_major(bool cell_tet, const float4* sites, int n, unsigned* knn, co
 // kNN ran with that tier); the first pass builds from them, and the rows of
 // the sites it leaves unfinished are completed (knn_sites_listed, from
 // cell_start and pos_of_id) before the one-warp pass.  lists: 6n ints,
-// counters: at least 12 (the exact form's completion list, the pieces pass's
-// list and their counters among them).
+// counters: CLIP_COUNTERS (the exact form's completion list, the pieces and
+// mesh passes' lists and their counters among them).
 
 // Inside field of one problem: turn the inside flags (fdim^3 bytes) into
 // 1 + the clear radius in cells, from the summed table of touched cells.
@@ -312,6 +345,7 @@ double mesh_volume(const float* verts, const int* tets, int nt);
 // vgb_grid_dim, the reference's heuristic over the whole box).
 int site_grid_dim(int n_site, double mesh_vol, float density);
 // Inside field of a mesh on a dim^3 grid over [0,1000]^3 (mesh_field.cpp).
+// open_faces: per tet, the info bits of tet_records.  On `threads` host threads.
 int build_inside_field(const float* verts, int nv, const int* tets, int nt, int dim, std::vector<unsigned char>& inside,
-                       std::vector<unsigned>& sat);
+                       std::vector<unsigned>& sat, std::vector<unsigned char>& open_faces, int threads);
 }  // namespace vgb
