@@ -57,8 +57,6 @@ struct MeshSmem {
   float4 plane[MESH_FACES];  // the cell's faces, site-relative
   union {
     struct {
-      float4 vert[MESH_VERTS];    // the cell's vertices, while its edges are made
-      unsigned edge[MESH_EDGES];  // faces p, q and end vertices of each edge
       unsigned char loc[MESH_ID_WORDS * 32];  // plane id -> face
     };
     float4 tp[WARP][4];  // the face planes of the tets in hand, in mesh order
@@ -70,7 +68,8 @@ struct MeshSmem {
   // the cell's edges: point nearest the site and direction, with the end
   // parameters; the terms of a unit of its length (volume in w)
   float4 epos[MESH_EDGES], edir[MESH_EDGES], eterm[MESH_EDGES];
-  unsigned short epq[MESH_EDGES];  // its faces, p | q << 8
+  unsigned edge[MESH_EDGES];  // faces p, q and end vertices of each
+  float3 vert[MESH_VERTS];    // the cell's vertices
   int tidx[WARP];       // tets in hand: their record, and what is known of them
   unsigned char tinf[WARP], thit[WARP];
   int queue[2 * WARP];  // tets whose sphere meets the cell's
@@ -246,7 +245,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
         const unsigned c = S.loc[min(tri_at(T[k], 2), (unsigned)(MESH_IDS - 1))];
         const float3 x = vertex_of(S.plane[a], S.plane[b], S.plane[c]);
         const float r2 = norm2_rn(x);
-        S.vert[i] = make_float4(x.x, x.y, x.z, r2);
+        S.vert[i] = x;
         lm = fmaxf(lm, r2);
         T[k] = pack_tri(a, b, c);
         S.twin[a * MESH_FACES + b] = (unsigned char)i;
@@ -278,7 +277,6 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
     __syncwarp();
     for (int i = lane; i < ne; i += WARP) {
       const unsigned E = S.edge[i];
-      S.epq[i] = (unsigned short)(E & 0xffffu);
       const float4 P = S.plane[E & 0xffu], Q = S.plane[(E >> 8) & 0xffu];
       const float3 D = cross_rn(xyz(Q), xyz(P));  // from the end whose vertex holds (p, q)
       const float dd = dot_rn(D, D);
@@ -288,8 +286,8 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
       S.epos[i] = make_float4(__fmul_rn(i2, __fmaf_rn(Q.w, a.x, __fmul_rn(P.w, b.x))),
                               __fmul_rn(i2, __fmaf_rn(Q.w, a.y, __fmul_rn(P.w, b.y))),
                               __fmul_rn(i2, __fmaf_rn(Q.w, a.z, __fmul_rn(P.w, b.z))),
-                              dot_rn(xyz(S.vert[(E >> 16) & 0xffu]), u));
-      S.edir[i] = make_float4(u.x, u.y, u.z, dot_rn(xyz(S.vert[E >> 24]), u));
+                              dot_rn(S.vert[(E >> 16) & 0xffu], u));
+      S.edir[i] = make_float4(u.x, u.y, u.z, dot_rn(S.vert[E >> 24], u));
     }
     __syncwarp();
 
@@ -311,8 +309,8 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
       // a piece [a, b] of an edge: k = det(F1 - F0, p, u) (b - a), and the
       // moment k1 (F1 + a + b) - k0 (F0 + a + b)
       for (int i = lane; i < ne; i += WARP) {
-        const unsigned pq = S.epq[i];
-        const float3 F0 = foot_of(S.plane[pq & 0xffu], X), F1 = foot_of(S.plane[pq >> 8], X);
+        const unsigned E = S.edge[i];
+        const float3 F0 = foot_of(S.plane[E & 0xffu], X), F1 = foot_of(S.plane[(E >> 8) & 0xffu], X);
         const float3 p = sub_rn(xyz(S.epos[i]), X), cr = cross_rn(p, xyz(S.edir[i]));
         const float k0 = dot_rn(F0, cr), k1 = dot_rn(F1, cr), k = __fsub_rn(k1, k0), k2 = 2.f * k;
         S.eterm[i] = round == 1 ? make_float4(2.f * p.x, 2.f * p.y, 2.f * p.z, 1.f)
@@ -545,17 +543,23 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
             const float4 PT = S.tp[b][i];
             const bool side = face_side(inf, i);
             // the cell's edges across its plane: where each face's line with
-            // it begins and ends
+            // it begins and ends.  The side of each vertex is decided once for
+            // all its edges, so that every face has its two ends or none (the
+            // box that bounds an open cell has edges that lie in mesh planes)
+            const unsigned up0 = __ballot_sync(FULL, lane < nt && eval4(PT, S.vert[lane]) >= 0.f);
+            const unsigned up1 = __ballot_sync(FULL, lane + WARP < nt && eval4(PT, S.vert[lane + WARP]) >= 0.f);
+            auto above = [&](unsigned v) { return ((v < WARP ? up0 : up1) >> (v & 31u)) & 1u; };
             for (int e = lane; e < ne; e += WARP) {
-              const float4 ep = S.epos[e], eu = S.edir[e];
-              bool up;
-              const float t = line_at(PT, xyz(ep), xyz(eu), up);
-              if (t > ep.w && t < eu.w) {
-                const float3 x = along(xyz(ep), t, xyz(eu));
-                const int in = up == side ? 0 : 1;
-                const unsigned pq = S.epq[e];
-                S.slot[in][pq & 0xffu] = make_float4(x.x, x.y, x.z, 1.f);
-                S.slot[1 - in][pq >> 8] = make_float4(x.x, x.y, x.z, 1.f);
+              const unsigned E = S.edge[e];
+              const bool end = above(E >> 24) != 0u;
+              if (end != (above((E >> 16) & 0xffu) != 0u)) {
+                const float4 ep = S.epos[e], eu = S.edir[e];
+                bool up;
+                const float t = line_at(PT, xyz(ep), xyz(eu), up);
+                const float3 x = along(xyz(ep), fminf(fmaxf(t, ep.w), eu.w), xyz(eu));
+                const int in = end == side ? 0 : 1;
+                S.slot[in][E & 0xffu] = make_float4(x.x, x.y, x.z, 1.f);
+                S.slot[1 - in][(E >> 8) & 0xffu] = make_float4(x.x, x.y, x.z, 1.f);
               }
             }
             // its sides: 0 (t1, t2), 1 (t0, t2), 2 (t0, t1)
