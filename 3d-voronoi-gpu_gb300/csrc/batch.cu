@@ -73,7 +73,7 @@ struct vgb_batch {
   int* redo_list = nullptr;
   int* redo_count = nullptr;       // clip hand-off and work counters, kNN work counters
   float4* rec = nullptr;           // float form: tet records of the mesh pass
-  unsigned char* open_faces = nullptr;  // their info bits, tets in input order
+  unsigned* face_info = nullptr;   // their info words, tets in input order
   vgb::CellStore store{};          // cells the first clip pass built and handed on (by site)
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   cudaEvent_t tev[2] = {};
@@ -106,7 +106,7 @@ void free_batch(vgb_batch* b) {
                   b->cell_start, b->cell_fill, b->site_cell, b->scan_tmp, b->pos_of_id, b->tet_order,
                   b->tet_cell_start, b->tcell, b->knn, b->mom, b->stats, b->field, b->field_sat, b->reach,
                   b->tet_sph, b->reach_max, b->secmiss, b->redo_list, b->redo_count, b->store.tri, b->store.nt,
-                  b->store.faces, b->store.mtri, b->store.mnt, b->rec, b->open_faces};
+                  b->store.faces, b->store.mtri, b->store.mnt, b->rec, b->face_info};
   for (void* p : bufs)
     if (p) cudaFree(p);
   if (b->st) cudaStreamDestroy(b->st);
@@ -151,7 +151,7 @@ int layout(vgb_batch* b) {
                    b->cell_fill, b->tcell, b->tet_order, b->scan_tmp, b->st))
     return VGB_ERR_CUDA;
   if (tet_spheres(b->verts, b->tets, b->tet_order, b->n_tet, b->tet_sph, b->st)) return VGB_ERR_CUDA;
-  if (b->rec && tet_records(b->verts, b->tets, b->tet_order, b->open_faces, b->n_tet, b->rec, b->st))
+  if (b->rec && tet_records(b->verts, b->tets, b->tet_order, b->face_info, b->n_tet, b->rec, b->st))
     return VGB_ERR_CUDA;
   VGB_CUDA_TRY(cudaStreamSynchronize(b->st));
   return VGB_OK;
@@ -214,7 +214,6 @@ int ensure_graph(vgb_batch* b, int update) {
 struct HostProblem {
   std::vector<unsigned char> inside;
   std::vector<unsigned> sat;
-  std::vector<unsigned char> open_faces;
   float rt_max = 0.f;
   int fdim = 8;
   double vol = 0.0;
@@ -248,7 +247,7 @@ void prepare_problem(const float* verts, int nv, const int* tets, int nt, int n_
   // field cells about a third of the site spacing, at most 256 per side
   const double spacing = std::cbrt(std::max(vol, 1.0) / std::max(n_site, 1));
   h.fdim = (int)std::min(256.0, std::max(8.0, std::ceil(3000.0 / spacing)));
-  build_inside_field(verts, nv, tets, nt, h.fdim, h.inside, h.sat, h.open_faces, 1);
+  build_inside_field(verts, nv, tets, nt, h.fdim, h.inside, h.sat, 1);
 }
 
 }  // namespace
@@ -360,7 +359,7 @@ int vgb_batch_create(vgb_batch** out, const vgb_config* cfg_in, int n_prob, cons
       (rc = balloc(&b->store.faces, (size_t)b->n * vgb::PIECE_REC)) ||
       (runs_mesh_pass(cfg.robust_predicates != 0, cfg.tet_pieces != 0, nt_tot, ns_tot) &&
        ((rc = balloc(&b->store.mtri, (size_t)b->n * vgb::MESH_VERTS)) || (rc = balloc(&b->store.mnt, b->n)) ||
-        (rc = balloc(&b->rec, 4 * (size_t)b->n_tet)) || (rc = balloc(&b->open_faces, b->n_tet))))) {
+        (rc = balloc(&b->rec, 4 * (size_t)b->n_tet)) || (rc = balloc(&b->face_info, b->n_tet))))) {
     free_batch(b);
     return rc;
   }
@@ -381,7 +380,6 @@ int vgb_batch_create(vgb_batch** out, const vgb_config* cfg_in, int n_prob, cons
     std::vector<int> sp((size_t)b->n), tp((size_t)b->n_tet);
     std::vector<unsigned char> fld((size_t)f_off);
     std::vector<unsigned> sat((size_t)q_off);
-    std::vector<unsigned char> open_faces((size_t)b->n_tet);
     long long vo = 0;
     for (int p = 0; p < n_prob; ++p) {
       const ProbDesc& P = b->probs[p];
@@ -402,7 +400,6 @@ int vgb_batch_create(vgb_batch** out, const vgb_config* cfg_in, int n_prob, cons
       }
       std::copy(hp[p].inside.begin(), hp[p].inside.end(), fld.begin() + P.field_off);
       std::copy(hp[p].sat.begin(), hp[p].sat.end(), sat.begin() + P.sat_off);
-      std::copy(hp[p].open_faces.begin(), hp[p].open_faces.end(), open_faces.begin() + P.tet_off);
       vo += n_vert[p];
       HostProblem().inside.swap(hp[p].inside);
       HostProblem().sat.swap(hp[p].sat);
@@ -414,8 +411,6 @@ int vgb_batch_create(vgb_batch** out, const vgb_config* cfg_in, int n_prob, cons
     if (ce == cudaSuccess) ce = cudaMemcpy(b->tet_prob, tp.data(), sizeof(int) * tp.size(), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess) ce = cudaMemcpy(b->field, fld.data(), fld.size(), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess) ce = cudaMemcpy(b->field_sat, sat.data(), sizeof(unsigned) * sat.size(), cudaMemcpyHostToDevice);
-    if (ce == cudaSuccess && b->open_faces)
-      ce = cudaMemcpy(b->open_faces, open_faces.data(), open_faces.size(), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess) ce = cudaMemset(b->mom, 0, sizeof(dmom4) * (size_t)b->n);
     if (ce != cudaSuccess) { set_error("batch upload: %s", cudaGetErrorString(ce)); free_batch(b); return VGB_ERR_CUDA; }
     for (int p = 0; p < n_prob; ++p)
@@ -424,6 +419,10 @@ int vgb_batch_create(vgb_batch** out, const vgb_config* cfg_in, int n_prob, cons
         free_batch(b);
         return VGB_ERR_CUDA;
       }
+  }
+  if (b->rec && face_info(b->verts, b->tets, b->n_vert, b->n_tet, b->face_info, nullptr, b->st)) {
+    free_batch(b);
+    return VGB_ERR_CUDA;
   }
   if ((rc = layout(b))) { free_batch(b); return rc; }
 // two passes timed after one untimed, on the current layout

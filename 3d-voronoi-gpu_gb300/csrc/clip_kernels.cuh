@@ -1677,9 +1677,10 @@ struct ClipPasses {
   // fast / redo, cell-tet batched fast / redo, completion lone / batched,
   // the 96-vertex fast pass lone / batched, the pieces pass lone / batched,
   // and of the float exact form the mesh pass, the one-warp pass and the
-  // completion pass that hand on to it, lone / batched each
+  // completion pass that hand on to it, lone / batched each, then the mesh
+  // pass of the reference form
   static int* resident() {
-    static int r[17] = {};
+    static int r[18] = {};
     return r;
   }
   static int prepare();
@@ -1712,7 +1713,9 @@ int ClipPasses<R>::prepare() {
       resident_blocks(k_clip_pieces<false, R>, sms, r + 9) || resident_blocks(k_clip_pieces<true, R>, sms, r + 10))
     return -2;
   if constexpr (!R)
-    if (resident_blocks(k_cell_mesh<false>, sms, r + 11) || resident_blocks(k_cell_mesh<true>, sms, r + 12) ||
+    if (resident_blocks(k_cell_mesh<false, false>, sms, r + 11) ||
+        resident_blocks(k_cell_mesh<true, false>, sms, r + 12) ||
+        resident_blocks(k_cell_mesh<false, true>, sms, r + 17) ||
         resident_blocks(k_clip_site<true, false, SLOTS_FAST, false, false, true>, sms, r + 13) ||
         resident_blocks(k_clip_site<true, true, SLOTS_FAST, false, false, true>, sms, r + 14) ||
         resident_blocks(k_clip_site<true, false, SLOTS_COMPLETE, false, true, true>, sms, r + 15) ||
@@ -1758,17 +1761,18 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
     set_error("clip: shape (%d lanes, %d slots) not built", shape.build_g, shape.fast_sl);
     return -1;
   }
+  const bool ref_mesh = !R && store.rec != nullptr && store.last != nullptr;
   int* const g_clip_resident_blocks = resident();
   if (g_clip_resident_blocks[0] == 0 && prepare()) return -2;
   if (!cell_tet && probs) {
     set_error("the tet-cell method runs one problem at a time");
     return -1;
   }
-  if (cell_tet && (!lists || !counters)) {
+  if ((cell_tet || ref_mesh) && (!lists || !counters)) {
     set_error("the cell-tet clip needs its site lists and counters");
     return -1;
   }
-  if (!cell_tet) {
+  if (!cell_tet && !ref_mesh) {
     // a few waves of resident blocks, sites dealt round-robin
     const long long want = (long long)g_clip_resident_blocks[0] * 4, need = (n + CLIP_WARPS - 1) / CLIP_WARPS;
     k_clip_site<false, false, SLOTS_TET_CELL, R><<<(int)(want < need ? want : need), CLIP_WARPS * WARP, 0, st>>>(
@@ -1796,16 +1800,19 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
   int* const esc = exact ? lists + 3 * (size_t)n : nullptr;
   float* const esc_r2 = exact ? reinterpret_cast<float*>(lists + 4 * (size_t)n) : nullptr;
   // the pieces pass (cell-tet records needed)
-  const bool mesh = !R && exact && store.rec != nullptr;
+  const bool mesh = !R && store.rec != nullptr && (exact || ref_mesh);
   const bool pieces = !mesh && shape.pieces != 0 && store.faces != nullptr;
   int* const piece_list = pieces ? lists + 5 * (size_t)n : nullptr;
   int* const mesh_list = mesh ? lists + 5 * (size_t)n : nullptr;
-  const int kt = exact ? k_tier : 0;
+  // (the reference form's rows are whole; its first pass reads as many as a
+  // relaxed cell needs)
+  const int kt = exact ? k_tier : (mesh && kmax > KNN_TIER) ? KNN_TIER : 0;
   VGB_CUDA_TRY(cudaMemsetAsync(counters, 0, CLIP_COUNTERS * sizeof(int), st));
   // every pass: one wave of resident blocks whose warps draw sites from a counter
   // the first pass's stored cells (exact form only)
   CellStore cs = store;
-  if (!exact) cs.tri = nullptr, cs.nt = nullptr;  // stored cells: exact form only
+  if (!exact && !mesh) cs.tri = nullptr, cs.nt = nullptr;  // stored cells: only after the first pass
+  if (!cell_tet) cs.flags = nullptr;
   auto launch = [&](auto kernel, int variant, const int* in_list, const int* in_count, int* out_list, int* out_count,
                     int* work, bool emit = false) {
     kernel<<<g_clip_resident_blocks[variant], CLIP_WARPS * WARP, 0, st>>>(
@@ -1821,7 +1828,7 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
         tet_cell_start, tet_sph, reach, reach_max_bits, prob_secmiss, piece_list, counters + 6, counters + 7,
         redo, counters + 1, cs, esc, esc_r2, exact ? counters + 10 : nullptr);
   };
-  if (exact) {
+  if (exact || mesh) {
     if (kmax < 1 || kmax > MAX_SITE_K) {
       set_error("clip: largest K %d outside [1, %d]", kmax, MAX_SITE_K);
       return -1;
@@ -1843,7 +1850,7 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
       else build(k_build<false, BUILD_G, BUILD_SL, R>);
     }
     // the full rows of the deep sites, before the one-warp pass reads them
-    if (kt > 0 && kt < kmax &&
+    if (exact && kt > 0 && kt < kmax &&
         knn_sites_listed(sites, n, cell_start, probs, site_prob, lone, kmax, pos_of_id, knn, deep, counters + 8,
                          counters + 9, st, shape.knn_warps))
       return -2;
@@ -1855,17 +1862,18 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
         kernel<<<g_clip_resident_blocks[variant], CLIP_WARPS * WARP, 0, st>>>(
             sites, n, knn, probs, site_prob, lone, verts, tets, site_start, site_tets, mom, stats, field, field_sat,
             tet_order, tet_cell_start, tet_sph, reach, reach_max_bits, prob_secmiss, in_list, in_count, out_list,
-            out_count, work, cs, kt, cell_start, esc, esc_r2, counters + 10, to_list, to_count);
+            out_count, work, cs, kt, cell_start, esc, esc_r2, exact ? counters + 10 : nullptr, to_list, to_count);
       };
       auto mesh_pass = [&](const int* in_list, int* in_count, int* work, bool last) {
         auto go = [&](auto kernel, int variant) {
           kernel<<<g_clip_resident_blocks[variant], MESH_WARPS * WARP, 0, st>>>(
               sites, knn, probs, site_prob, lone, cs.rec, tet_cell_start, tet_sph, reach, reach_max_bits, mom, stats,
               prob_secmiss, in_list, in_count, work, last ? nullptr : redo, counters + 1, cs, last ? nullptr : esc,
-              esc_r2, counters + 10);
+              esc_r2, counters + 10, site_start);
         };
-        if (probs) go(k_cell_mesh<true>, 12);
-        else go(k_cell_mesh<false>, 11);
+        if (ref_mesh) go(k_cell_mesh<false, true>, 17);
+        else if (probs) go(k_cell_mesh<true, false>, 12);
+        else go(k_cell_mesh<false, false>, 11);
       };
       // the cells the first pass left, finished or taken whole; then what of
       // each lies in the mesh; then the cells above 64 vertices, and those
@@ -1884,6 +1892,10 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
         mesh_pass(mesh_list, counters + 12, counters + 13, false);
         pass(k_clip_site<true, false, SLOTS_REDO, false>, 2, redo, counters + 1, nullptr, nullptr, counters + 4,
              nullptr, nullptr);
+        if (!exact) {
+          VGB_CUDA_TRY(cudaGetLastError());
+          return 0;
+        }
         pass(k_clip_site<true, false, SLOTS_COMPLETE, false, true, true>, 15, esc, counters + 10, nullptr, nullptr,
              counters + 11, rest, counters + 14);
       }

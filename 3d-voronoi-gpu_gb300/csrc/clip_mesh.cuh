@@ -49,6 +49,9 @@ constexpr int MESH_ID_WORDS = (MESH_IDS + 31) / 32;
 // A cell whose terms from the site exceed this many times their sum is done
 // again from a point of what is left of it (sites outside the mesh).
 constexpr float MESH_APEX_RATIO = 32.f;
+// A sum below this fraction of its terms (rounded to 1e-7 of them each) is
+// rounding: the cell only touches the mesh, and its site stays where it is.
+constexpr float MESH_NOISE = 1e-6f;
 #ifndef VGB_MESH_MIN_BLOCKS
 #define VGB_MESH_MIN_BLOCKS 5
 #endif
@@ -161,7 +164,10 @@ constexpr unsigned REC_EVEN = 16u, REC_SKIP = 32u;
 // the side of its canonical plane i the tet lies on (true: positive)
 __device__ __forceinline__ bool face_side(unsigned info, int i) { return ((info >> 4) & 1u) == (unsigned)(i & 1); }
 
-template <bool BATCHED>
+// REF (reference form): a site's sum is over the tets it is a candidate of
+// (one of the tet_k nearest sites of their centroid), and the face between
+// such a tet and one it is no candidate of is open.
+template <bool BATCHED, bool REF>
 __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell_mesh(
     const float4* __restrict__ sites, const unsigned* __restrict__ knn, const ProbDesc* __restrict__ probs,
     const int* __restrict__ site_prob, const ProbDesc lone, const float4* __restrict__ rec,
@@ -169,7 +175,8 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
     const unsigned* __restrict__ reach_max_bits, dmom4* __restrict__ mom, unsigned long long* __restrict__ stats,
     unsigned* __restrict__ prob_secmiss, const int* __restrict__ in_list, const int* __restrict__ in_count,
     int* __restrict__ work, int* __restrict__ out_list, int* __restrict__ out_count, const CellStore store,
-    int* __restrict__ esc_list, float* __restrict__ esc_r2, int* __restrict__ esc_count) {
+    int* __restrict__ esc_list, float* __restrict__ esc_r2, int* __restrict__ esc_count,
+    const int* __restrict__ site_start) {
   __shared__ MeshSmem smem_all[MESH_WARPS];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const unsigned lt_mask = (1u << lane) - 1u;
@@ -192,7 +199,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
     const int K = PD(K);
     const unsigned* const krow = knn + PD(knn_off) + (size_t)(s - PD(site_off)) * K;
     const bool miss = (flags & SITE_SECMISS) && !(flags & SITE_COMPLETED);
-    const float dK2 = miss ? dist2(seed, sites[krow[K - 1]]) : FLT_MAX;
+    const float dK2 = miss && !REF ? dist2(seed, sites[krow[K - 1]]) : FLT_MAX;
 
     // -----------------------------------------------------------------
     // the cell: its faces, vertices and edges
@@ -293,12 +300,20 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
 
     // -----------------------------------------------------------------
     // the tets.  When the first apex (the site) turns out far from what is left
-    // of the cell: again for the mean point of its edges there (their lengths
-    // and moments in place of their terms, no triangles), and from that point
+    // of the cell: again for a mean of its points (lengths of its edges and
+    // moments of them in place of their terms), and then from that point
     float3 X = make_float3(0.f, 0.f, 0.f);
-    float pr2 = 0.f, vol = 0.f, mx = 0.f, my = 0.f, mz = 0.f;
+    float pr2 = 0.f, vol = 0.f, mx = 0.f, my = 0.f, mz = 0.f, v6 = 0.f, mag = 0.f;
     const int dim = PD(dim), cbase = PD(cell_off);
-    const float R = __fadd_rn(fminf(__fmaf_rn(PD(rt_max), 1.001f, Rc), __uint_as_float(reach_max_bits[pidx])), 0.01f);
+    const float rt = REF ? __uint_as_float(reach_max_bits[1]) : PD(rt_max);
+    const float R = __fadd_rn(fminf(__fmaf_rn(rt, 1.001f, Rc), __uint_as_float(reach_max_bits[pidx])), 0.01f);
+    // is the site a candidate of the tet? (the search's order: distance, then id)
+    auto candidate = [&](int q) {
+      const float2 z = store.last[q];
+      const float d2 = dist2(tet_sph[q], seed);
+      return d2 < z.x || (d2 == z.x && site_id(seed) <= __float_as_int(z.y));
+    };
+    int nclip = 0;
     const float h = 1000.f / (float)dim;
     const int j0 = grid_axis(seed.y - R, dim), k0 = grid_axis(seed.z - R, dim);
     const int nj = grid_axis(seed.y + R, dim) - j0 + 1;
@@ -380,12 +395,13 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
             const float4 sp = tet_sph[idx];
             const float ex = sp.x - seed.x, ey = sp.y - seed.y, ez = sp.z - seed.z;
             const float dm = sqrtf(dot3_rn(ex, ey, ez, ex, ey, ez));
-            meets = dm <= __fmaf_rn(__fadd_rn(Rc, sp.w), 1.0001f, 1e-3f) && dm <= __fmaf_rn(reach[idx], 1.0001f, 1e-2f);
+            meets = dm <= __fmaf_rn(__fadd_rn(Rc, sp.w), 1.0001f, 1e-3f);
+            if (meets) meets = REF ? candidate(idx) : dm <= __fmaf_rn(reach[idx], 1.0001f, 1e-2f);
           }
           const unsigned m = __ballot_sync(FULL, meets);
           if (meets) S.queue[nq + __popc(m & lt_mask)] = idx;
           nq += __popc(m);
-          if (lane == 0) S.cnt[WC_CAND] += (unsigned)min(WARP, total - f0);
+          if (!REF && lane == 0) S.cnt[WC_CAND] += (unsigned)min(WARP, total - f0);
           f0 += WARP;
         }
         if (nq == 0) break;
@@ -424,8 +440,8 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
         if (lane < rest) S.queue[lane] = move;
         nq = rest;
         if (lane == 0) {
-          S.cnt[WC_CULLED] += (unsigned)(take - nb);
-          S.cnt[WC_CLIPPED] += (unsigned)nb;
+          if (!REF) S.cnt[WC_CULLED] += (unsigned)(take - nb);
+          if (!REF) S.cnt[WC_CLIPPED] += (unsigned)nb;
           S.cnt[WC_CULLTESTS] += (unsigned)(take * nf);
           S.cnt[WC_CONFLICT] += (unsigned)(8 * ne * nb);
         }
@@ -440,11 +456,18 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
           face(2, A0, A1, A3, c0);
           face(3, A0, A1, A2, c0);
           unsigned far = 0u;
-          if (miss) {
+          if (miss && !REF) {
             const float m2 = fmaxf(fmaxf(dot_rn(c0, c0), dot_rn(c1, c1)), fmaxf(dot_rn(c2, c2), dot_rn(c3, c3)));
             far = !(dK2 > __fmaf_rn(4.f * m2, 1.0001f, 1e-4f)) ? 64u : 0u;
           }
           S.tidx[pos] = idx;
+          if (REF) {
+            const int4 nb4 = store.beside[idx];
+            if (nb4.x >= 0 && !candidate(nb4.x)) info |= 1u;
+            if (nb4.y >= 0 && !candidate(nb4.y)) info |= 2u;
+            if (nb4.z >= 0 && !candidate(nb4.z)) info |= 4u;
+            if (nb4.w >= 0 && !candidate(nb4.w)) info |= 8u;
+          }
           S.tinf[pos] = (unsigned char)((info & 31u) | far);
           S.thit[pos] = 0;
         }
@@ -490,7 +513,8 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
         __syncwarp();
         const unsigned hits = __ballot_sync(FULL, lane < nb && S.thit[lane] != 0);
         const unsigned farm = __ballot_sync(FULL, lane < nb && (S.tinf[lane] & 64u) != 0u);
-        unsigned open = __ballot_sync(FULL, lane < nb && round != 1 && (S.tinf[lane] & 15u) != 0u);
+        unsigned open = __ballot_sync(FULL, lane < nb && (S.tinf[lane] & 15u) != 0u);
+        nclip += nb;
         if (lane == 0) {
           S.cnt[WC_CONTRIB] += (unsigned)__popc(hits);
           S.cnt[WC_EMPTY] += (unsigned)(nb - __popc(hits));
@@ -598,8 +622,12 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
                   const float3 aX = sub_rn(a, X), bX = sub_rn(bb, X);
                   const float3 cr = cross_rn(aX, bX), ab = make_float3(__fadd_rn(aX.x, bX.x), __fadd_rn(aX.y, bX.y), __fadd_rn(aX.z, bX.z));
                   const float3 F = foot_of(P, X);
-                  sum.add(dot_rn(F, cr), F, ab);
-                  sum.add(-dot_rn(FT, cr), FT, ab);
+                  if (round == 1) {
+                    sum.add(1.f, make_float3(0.f, 0.f, 0.f), ab);
+                  } else {
+                    sum.add(dot_rn(F, cr), F, ab);
+                    sum.add(-dot_rn(FT, cr), FT, ab);
+                  }
                 }
               }
             }
@@ -618,15 +646,17 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
               const float3 aX = sub_rn(a, X), bX = sub_rn(bb, X);
               const float3 cr = cross_rn(aX, bX), ab = make_float3(__fadd_rn(aX.x, bX.x), __fadd_rn(aX.y, bX.y), __fadd_rn(aX.z, bX.z));
               const float k6 = dot_rn(FT, cr);
-              sum.add((side == (lane != 1)) ? -k6 : k6, FT, ab);
+              sum.add(round == 1 ? 1.f : (side == (lane != 1)) ? -k6 : k6,
+                      round == 1 ? make_float3(0.f, 0.f, 0.f) : FT, ab);
             }
             __syncwarp();
           }
         }
         __syncwarp();
       }
-      const float v6 = warp_sum(sum.v), x24 = warp_sum(sum.x), y24 = warp_sum(sum.y), z24 = warp_sum(sum.z);
-      const float mag = warp_sum(sum.mag);
+      v6 = warp_sum(sum.v);
+      mag = warp_sum(sum.mag);
+      const float x24 = warp_sum(sum.x), y24 = warp_sum(sum.y), z24 = warp_sum(sum.z);
       pr2 = fmaxf(pr2, warp_max_nonneg(far2));
       if (round == 1) {
         if (!(v6 > 0.f)) break;
@@ -640,6 +670,14 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
       mz = __fmaf_rn(z24, 1.f / 24.f, __fmul_rn(vol, X.z));
       // large terms for a small sum: the apex is far from what is left
       if (mag <= MESH_APEX_RATIO * v6 || mag == 0.f) break;
+    }
+    // a sum within its terms' rounding is none (a tet that only touches)
+    if (!(v6 > MESH_NOISE * mag)) vol = mx = my = mz = v6 == v6 ? 0.f : v6;
+    if (REF && lane == 0) {
+      const unsigned nc = (unsigned)(site_start[s + 1] - site_start[s]);
+      S.cnt[WC_CAND] += nc;
+      S.cnt[WC_CLIPPED] += min((unsigned)nclip, nc);
+      S.cnt[WC_CULLED] += nc - min((unsigned)nclip, nc);
     }
     bad |= !(isfinite(vol) && isfinite(mx) && isfinite(my) && isfinite(mz));
     if (bad) {

@@ -63,7 +63,9 @@ struct vgb_engine {
   unsigned* reach_max = nullptr;   // exact form: float bits of the largest reach
   int* redo_list = nullptr;        // cell-tet: the clip passes' site lists (6n)
   int* redo_count = nullptr;       // clip hand-off and work counters, kNN work counters
-  float4* rec = nullptr;           // exact form, float: tet records of the mesh pass
+  float4* rec = nullptr;           // float predicates: tet records of the mesh pass
+  float2* last = nullptr;          // reference form: each tet's last candidate,
+  int4* beside = nullptr;          // and the tets across its faces
   vgb::CellStore store{};          // cells the first clip pass built and handed on, cell records (by site)
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // [update]
   cudaEvent_t ev[VGB_PHASES + 1] = {};
@@ -179,7 +181,7 @@ void free_engine(vgb_engine* e) {
                   e->scan_tmp, e->pos_of_id, e->tet_order, e->tet_cell_start, e->knn, e->cand, e->site_start, e->site_fill, e->site_tets, e->mom, e->mom_f,
                   e->io_stage, e->stats, e->field, e->field_sat, e->reach, e->reach_max, e->tet_sph,
                   e->redo_list, e->redo_count, e->store.tri, e->store.nt, e->store.flags, e->store.faces, e->store.mtri,
-                  e->store.mnt, e->rec};
+                  e->store.mnt, e->rec, e->last, e->beside};
   for (void* b : bufs)
     if (b) cudaFree(b);
   if (e->st) cudaStreamDestroy(e->st);
@@ -211,6 +213,9 @@ int run_pass(vgb_engine* e, int update) {
       knn_tet_centroids(e->sites, e->n, e->dim, e->cell_start, e->pos_of_id, e->verts, e->tets, e->tet_order,
                         e->tet_cell_start, e->n_tet, e->tk, e->cand, e->redo_count + 5, st))
     return VGB_ERR_CUDA;
+  if (e->store.last && last_candidates(e->sites, e->tet_sph, e->tet_order, e->cand, e->n_tet, e->tk, e->last,
+                                       e->reach_max, st))
+    return VGB_ERR_CUDA;
   MARK(3);
   if (!exact && e->cfg.method != VGB_METHOD_PLAIN) {
     if (candidates_by_site(e->cand, e->n_tet, e->tk, e->n, e->site_start, e->site_fill, e->site_tets,
@@ -223,7 +228,8 @@ int run_pass(vgb_engine* e, int update) {
   if (e->cfg.method != VGB_METHOD_PLAIN) {
     if (clip_site_major(e->cfg.method == VGB_METHOD_CELL_TET, e->sites, e->n, e->knn, nullptr, nullptr, e->prob,
                         e->verts, e->tets, e->site_start, e->site_tets, e->mom, e->stats, e->field, e->field_sat,
-                        exact ? e->tet_order : nullptr, exact ? e->tet_cell_start : nullptr, e->tet_sph, e->reach,
+                        exact ? e->tet_order : nullptr, exact || e->store.last ? e->tet_cell_start : nullptr, e->tet_sph,
+                        e->reach,
                         e->reach_max, nullptr, e->redo_list, e->redo_count, e->K, e->store, tier, e->cell_start,
                         e->pos_of_id, e->cfg.robust_predicates != 0, e->shape, st))
       return VGB_ERR_CUDA;
@@ -416,8 +422,8 @@ int vgb_engine_create(vgb_engine** out, const vgb_config* cfg_in, const float* v
   int rc = VGB_OK;
   size_t pairs = (size_t)n_tet * e->tk;
   const bool exact_form = cfg.method == VGB_METHOD_CELL_TET && cfg.exact;
-  const bool mesh_form = 
-      exact_form && runs_mesh_pass(cfg.robust_predicates != 0, cfg.tet_pieces != 0, n_tet, n_site);
+  const bool mesh_form = cfg.method != VGB_METHOD_PLAIN &&
+                         runs_mesh_pass(cfg.robust_predicates != 0, cfg.tet_pieces != 0, n_tet, n_site);
   size_t scan_n = std::max((size_t)e->ncell + 1, (size_t)n_site + 1);
   if ((rc = dalloc(&e->verts, n_vert)) || (rc = dalloc(&e->tets, n_tet)) || (rc = dalloc(&e->sites, n_site)) ||
       (rc = dalloc(&e->sites_tmp, n_site)) || (rc = dalloc(&e->cell_start, e->ncell + 1)) ||
@@ -430,8 +436,8 @@ int vgb_engine_create(vgb_engine** out, const vgb_config* cfg_in, const float* v
       (rc = dalloc(&e->mom, n_site)) || (rc = dalloc(&e->redo_list, 6 * (size_t)n_site)) || (rc = dalloc(&e->redo_count, CLIP_COUNTERS)) || (rc = dalloc(&e->mom_f, cfg.method == VGB_METHOD_PLAIN ? n_site : 1)) ||
       (rc = dalloc(&e->io_stage, 3 * (size_t)std::max(n_site, n_vert))) ||
       (rc = dalloc(&e->stats, VGB_STAT_COUNT)) ||
-      (rc = dalloc(&e->store.tri, exact_form ? (size_t)n_site * STORE_VERTS : 1)) ||
-      (rc = dalloc(&e->store.nt, exact_form ? (size_t)n_site : 1)) ||
+      (rc = dalloc(&e->store.tri, exact_form || mesh_form ? (size_t)n_site * STORE_VERTS : 1)) ||
+      (rc = dalloc(&e->store.nt, exact_form || mesh_form ? (size_t)n_site : 1)) ||
       (rc = dalloc(&e->store.flags, cfg.method == VGB_METHOD_CELL_TET ? (size_t)n_site : 1)) ||
       (rc = dalloc(&e->store.faces, cfg.method == VGB_METHOD_CELL_TET ? (size_t)n_site * PIECE_REC : 1)) ||
       (rc = dalloc(&e->store.mtri, mesh_form ? (size_t)n_site * MESH_VERTS : 1)) ||
@@ -476,6 +482,37 @@ int vgb_engine_create(vgb_engine** out, const vgb_config* cfg_in, const float* v
   if (ce == cudaSuccess) ce = cudaMemsetAsync(e->mom, 0, sizeof(dmom4) * n_site, e->st);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->st);
   if (ce != cudaSuccess) { set_error("mesh upload: %s", cudaGetErrorString(ce)); free_engine(e); return VGB_ERR_CUDA; }
+  if (mesh_form) {
+    // the mesh pass's tets: open faces, corners, bounding spheres
+    // (the reference form: also the tets across their faces)
+    unsigned* info = nullptr;
+    int4* across = nullptr;
+    if ((rc = dalloc(&info, 2 * (size_t)n_tet)) || (!exact_form && (rc = dalloc(&across, n_tet))) ||
+        (!exact_form && (rc = dalloc(&e->beside, n_tet))) || (rc = dalloc(&e->rec, 4 * (size_t)n_tet)) ||
+        (rc = dalloc(&e->reach_max, 2)) || (rc = dalloc(&e->tet_sph, n_tet)) ||
+        (rc = dalloc(&e->last, exact_form ? 1 : n_tet))) {
+      if (info) cudaFree(info);
+      if (across) cudaFree(across);
+      free_engine(e);
+      return rc;
+    }
+    if (face_info(e->verts, e->tets, n_vert, n_tet, info, across, e->st) ||
+        (across && tets_beside(e->tet_order, across, n_tet, (int*)info + n_tet, e->beside, e->st)) ||
+        tet_records(e->verts, e->tets, e->tet_order, info, n_tet, e->rec, e->st) ||
+        tet_spheres(e->verts, e->tets, e->tet_order, n_tet, e->tet_sph, e->st)) {
+      cudaFree(info);
+      if (across) cudaFree(across);
+      free_engine(e);
+      return VGB_ERR_CUDA;
+    }
+    ce = cudaStreamSynchronize(e->st);
+    cudaFree(info);
+    if (across) cudaFree(across);
+    if (ce != cudaSuccess) { set_error("tet records: %s", cudaGetErrorString(ce)); free_engine(e); return VGB_ERR_CUDA; }
+    e->store.rec = e->rec;
+    e->store.last = exact_form ? nullptr : e->last;
+    e->store.beside = e->beside;
+  }
   if (cfg.method == VGB_METHOD_CELL_TET && cfg.exact) {
     float rt = 0.f;
     double mesh_vol = 0.0;
@@ -507,31 +544,18 @@ int vgb_engine_create(vgb_engine** out, const vgb_config* cfg_in, const float* v
     e->fdim = (int)std::min(512.0, std::max(8.0, std::ceil(3000.0 / spacing)));
     std::vector<unsigned char> field;
     std::vector<unsigned> field_sat;
-    std::vector<unsigned char> open_faces;
-    build_inside_field(verts, n_vert, tets, n_tet, e->fdim, field, field_sat, open_faces,
+    build_inside_field(verts, n_vert, tets, n_tet, e->fdim, field, field_sat,
                        std::max(1, std::min(8, (int)std::thread::hardware_concurrency())));
     e->prob.fdim = e->fdim;
     if ((rc = dalloc(&e->field, field.size())) || (rc = dalloc(&e->field_sat, field_sat.size())) ||
         (rc = dalloc(&e->reach, n_tet)) ||
-        (rc = dalloc(&e->reach_max, 1)) || (rc = dalloc(&e->tet_sph, n_tet))) {
+        (!mesh_form && ((rc = dalloc(&e->reach_max, 1)) || (rc = dalloc(&e->tet_sph, n_tet))))) {
       free_engine(e);
       return rc;
     }
-    if (tet_spheres(e->verts, e->tets, e->tet_order, n_tet, e->tet_sph, e->st)) { free_engine(e); return VGB_ERR_CUDA; }
-    if (mesh_form) {
-      unsigned char* d_open = nullptr;
-      if ((rc = dalloc(&d_open, n_tet)) || (rc = dalloc(&e->rec, 4 * (size_t)n_tet))) {
-        if (d_open) cudaFree(d_open);
-        free_engine(e);
-        return rc;
-      }
-      ce = cudaMemcpyAsync(d_open, open_faces.data(), (size_t)n_tet, cudaMemcpyHostToDevice, e->st);
-      if (ce == cudaSuccess && tet_records(e->verts, e->tets, e->tet_order, d_open, n_tet, e->rec, e->st))
-        ce = cudaErrorUnknown;
-      if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->st);
-      cudaFree(d_open);
-      if (ce != cudaSuccess) { set_error("tet records: %s", cudaGetErrorString(ce)); free_engine(e); return VGB_ERR_CUDA; }
-      e->store.rec = e->rec;
+    if (!mesh_form && tet_spheres(e->verts, e->tets, e->tet_order, n_tet, e->tet_sph, e->st)) {
+      free_engine(e);
+      return VGB_ERR_CUDA;
     }
     ce = cudaMemcpy(e->field, field.data(), field.size(), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess)

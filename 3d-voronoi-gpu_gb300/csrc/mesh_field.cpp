@@ -78,35 +78,14 @@ int site_grid_dim(int n_site, double mesh_vol, float density) {
 }
 
 int build_inside_field(const float* verts, int nv, const int* tets, int nt, int dim,
-                       std::vector<unsigned char>& inside, std::vector<unsigned>& sat,
-                       std::vector<unsigned char>& open_faces, int threads) {
+                       std::vector<unsigned char>& inside, std::vector<unsigned>& sat, int threads) {
   const long long nc = (long long)dim * dim * dim;
   const size_t W = (size_t)dim + 1;
   // (a thread costs about 20 us: one for small fields)
   if (nc < (1LL << 20)) threads = 1;
   inside.assign((size_t)nc, 0);
   sat.assign(W * W * W, 0u);
-  open_faces.assign((size_t)std::max(nt, 0), 0);
   if (nt <= 0 || nv <= 0) return 0;
-  // 0. each tet's corner order and orientation: bit 4 when ascending vertex
-  //    order is an even permutation of a positively oriented tet, bit 5 when
-  //    it is not positively oriented
-  parallel_ranges((size_t)nt, threads, [&](size_t t0, size_t t1) {
-  for (size_t t = t0; t < t1; ++t) {
-    const int* q = tets + 4 * t;
-    int inversions = 0;
-    for (int i = 0; i < 4; ++i)
-      for (int j = i + 1; j < 4; ++j) inversions += q[i] > q[j];
-    double e[3][3];
-    for (int i = 0; i < 3; ++i)
-      for (int d = 0; d < 3; ++d)
-        e[i][d] = (double)verts[3 * (size_t)q[i + 1] + d] - (double)verts[3 * (size_t)q[0] + d];
-    const double det = e[0][0] * (e[1][1] * e[2][2] - e[1][2] * e[2][1]) +
-                       e[0][1] * (e[1][2] * e[2][0] - e[1][0] * e[2][2]) +
-                       e[0][2] * (e[1][0] * e[2][1] - e[1][1] * e[2][0]);
-    open_faces[t] = (unsigned char)((inversions & 1 ? 0 : 16) | (det > 0.0 ? 0 : 32));
-  }
-  });
   // 1. boundary faces
   std::vector<int> count((size_t)nv + 1, 0);
   static const int fv[4][3] = {{1, 2, 3}, {0, 2, 3}, {0, 1, 3}, {0, 1, 2}};
@@ -119,42 +98,25 @@ int build_inside_field(const float* verts, int nv, const int* tets, int nt, int 
   for (int t = 0; t < nt; ++t)
     for (int f = 0; f < 4; ++f) count[(size_t)face(t, f)[0] + 1]++;
   for (int v = 0; v < nv; ++v) count[(size_t)v + 1] += count[v];
-  // (the face's other two vertices, then its tet and the place of the corner
-  // it leaves out in the tet's vertex order)
-  struct Entry {
-    int b, c, tet, at;
-  };
-  std::vector<Entry> bucket((size_t)nt * 4);
+  std::vector<std::array<int, 2>> bucket((size_t)nt * 4);
   {
     std::vector<int> fill(count.begin(), count.end() - 1);
     for (int t = 0; t < nt; ++t)
       for (int f = 0; f < 4; ++f) {
         auto k = face(t, f);
-        const int* q = tets + 4 * (size_t)t;
-        const int at = (q[0] < q[f]) + (q[1] < q[f]) + (q[2] < q[f]) + (q[3] < q[f]);
-        bucket[(size_t)fill[k[0]]++] = {k[1], k[2], t, at};
+        bucket[(size_t)fill[k[0]]++] = {k[1], k[2]};
       }
   }
   std::vector<unsigned char> touch((size_t)nc, 0);
   const float margin = 1e-3f * 1000.f / dim + 1e-3f;
   for (int a = 0; a < nv; ++a) {
     auto b0 = bucket.begin() + count[a], b1 = bucket.begin() + count[(size_t)a + 1];
-    std::sort(b0, b1, [](const Entry& x, const Entry& y) { return x.b != y.b ? x.b < y.b : x.c < y.c; });
+    std::sort(b0, b1);
     for (auto it = b0; it != b1;) {
       auto jt = it + 1;
-      while (jt != b1 && jt->b == it->b && jt->c == it->c) ++jt;
-      // a face of two tets on opposite sides of it is inner; any other is open
-      // on the side of each of its tets
-      int sides[2] = {0, 0}, real = 0;
-      for (auto f = it; f != jt; ++f)
-        if (!(open_faces[f->tet] & 32)) {
-          ++real;
-          ++sides[((open_faces[f->tet] >> 4) ^ f->at) & 1];
-        }
-      if (!(real == 2 && sides[0] == 1))
-        for (auto f = it; f != jt; ++f) open_faces[f->tet] |= (unsigned char)(1 << f->at);
+      while (jt != b1 && *jt == *it) ++jt;
       if (jt - it == 1) {  // a face of one tet only
-        const float* p[3] = {verts + 3 * (size_t)a, verts + 3 * (size_t)it->b, verts + 3 * (size_t)it->c};
+        const float* p[3] = {verts + 3 * (size_t)a, verts + 3 * (size_t)(*it)[0], verts + 3 * (size_t)(*it)[1]};
         int lo[3], hi[3];
         for (int d = 0; d < 3; ++d) {
           float mn = std::min(std::min(p[0][d], p[1][d]), p[2][d]) - margin;

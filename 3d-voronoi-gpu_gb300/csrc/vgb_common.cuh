@@ -214,9 +214,22 @@ int tet_spheres(const float4* verts, const int4* tets, const int* tet_order, int
 // vertex index (12 floats), an info word (bits 0-3: the face that leaves out
 // the i-th corner is open; 4: that corner order is an even permutation of a
 // positively oriented tet; 5: not positively oriented), 3 spare words.
-// open_faces: bits 0-5 per tet in input order, from build_inside_field.
-int tet_records(const float4* verts, const int4* tets, const int* tet_order, const unsigned char* open_faces, int n_tet,
+// info: bits 0-5 per tet in input order, from face_info.
+int tet_records(const float4* verts, const int4* tets, const int* tet_order, const unsigned* info, int n_tet,
                 float4* rec, cudaStream_t st);
+// Which faces of each tet are open (no other tet shares them from the other
+// side) and the tets' orientations: the info words of tet_records, input
+// order.  Allocates its scratch; synchronises.
+// beside (may be null): the tet across each face, input order, -1 where open.
+int face_info(const float4* verts, const int4* tets, int n_vert, int n_tet, unsigned* info, int4* beside,
+              cudaStream_t st);
+// The same in centroid-cell order; where: n_tet ints scratch.
+int tets_beside(const int* tet_order, const int4* beside, int n_tet, int* where, int4* out, cudaStream_t st);
+// Reference form: last[q] = (squared distance from its centroid, id) of the
+// last candidate of the q-th tet in centroid-cell order; reach_max_bits[0] =
+// float bits of the largest such distance, [1] of the largest tet's radius.
+int last_candidates(const float4* sites, const float4* tet_sph, const int* tet_order, const unsigned* cand, int n_tet,
+                    int tk, float2* last, unsigned* reach_max_bits, cudaStream_t st);
 // Tets sorted by the grid cell of their float32 centroid in their problem's
 // grid (once per mesh): tet_cell_start ncell + 1 ints, cell_fill ncell
 // scratch, tcell n_tet scratch, tet_order n_tet ints.
@@ -267,6 +280,8 @@ struct CellStore {
   unsigned* mtri;        // [n][MESH_VERTS]
   int* mnt;              // [n]
   const float4* rec;     // [n_tet][4], from tet_records
+  const float2* last;    // reference form: last candidate of each tet, from last_candidates (else null)
+  const int4* beside;    // and the tets (centroid-cell order) its inner faces lead to, from tets_beside
 };
 // A cell record of the one-warp pass for the pieces pass: its face count,
 // radius (float bits) and outcome bits so far, a spare word, then its face
@@ -279,8 +294,8 @@ constexpr int PIECE_REC = 4 + PIECE_FACES / 4;
 constexpr int MESH_VERTS = 64;
 constexpr int MESH_EXT = PIECE_REC;
 
-// Whether the exact cell-tet form of a problem (or batch) runs the mesh pass
-// (clip_mesh.cuh): with float predicates, it does.  It is faster than clipping by each tet
+// Whether a problem (or batch) runs the mesh pass (clip_mesh.cuh): the exact
+// form and the reference forms do, with float predicates.  It is faster than clipping by each tet
 // at every size and mesh measured (Lloyd iteration, us: 20k sites in 48k tets
 // 610 -> 290, 100k in 6 tets 1,955 -> 1,020, 1M in 1.96M 10,100 -> 7,400); the
 // pieces pass is left to callers who ask for it on a mesh of fewer than a tet
@@ -345,7 +360,7 @@ double mesh_volume(const float* verts, const int* tets, int nt);
 // vgb_grid_dim, the reference's heuristic over the whole box).
 int site_grid_dim(int n_site, double mesh_vol, float density);
 // Inside field of a mesh on a dim^3 grid over [0,1000]^3 (mesh_field.cpp).
-// open_faces: per tet, the info bits of tet_records.  On `threads` host threads.
+// On `threads` host threads.
 int build_inside_field(const float* verts, int nv, const int* tets, int nt, int dim, std::vector<unsigned char>& inside,
-                       std::vector<unsigned>& sat, std::vector<unsigned char>& open_faces, int threads);
+                       std::vector<unsigned>& sat, int threads);
 }  // namespace vgb

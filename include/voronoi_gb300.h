@@ -50,7 +50,9 @@ enum vgb_stat {
   VGB_STAT_CLIPPED = 2,         /* run through the full clip                          */
   VGB_STAT_EMPTY = 3,           /* clipped to nothing (mesh pass: no edge of the cell in it) */
   VGB_STAT_CONTRIB = 4,         /* contributed volume (mesh pass: an edge of the cell in it) */
-  VGB_STAT_SECURITY_MISS = 5,   /* contributed without reaching the security radius   */
+  VGB_STAT_SECURITY_MISS = 5,   /* contributed without reaching the security radius
+                                   (mesh pass: cells, otherwise pairs in the tet-cell
+                                   method)                                            */
   VGB_STAT_TRI_OVERFLOW = 6,    /* dropped: more cell vertices than the capacity      */
   VGB_STAT_BOUNDARY_FAIL = 7,   /* dropped: cavity boundary not one loop              */
   VGB_STAT_PLANES = 8,          /* bisector planes applied                            */
@@ -141,10 +143,10 @@ typedef struct vgb_config {
                    on the sites after two Lloyd steps (the initial sites are put
                    back).  0: the defaults (8, 8, 64, the configured clip form).  The
                    batched form tunes them with the grid density (grid_dim 0).      */
-  int tet_pieces; /* cell-tet method, where cells are clipped by each tet (the exact
-                   form with float predicates sums a cell's edges and the mesh's
-                   open triangles instead, whatever this says, on meshes of at
-                   least a tet per 256 sites).  0 (default): a copy of the cell is clipped by
+  int tet_pieces; /* cell-tet method, where cells are clipped by each tet (with
+                   float predicates a cell's edges and the mesh's open triangles are
+                   summed instead, unless this is 1 and the mesh has fewer than a
+                   tet per 256 sites).  0 (default): a copy of the cell is clipped by
                    each candidate tet's four faces, one warp per site.  1: each piece
                    (cell ^ tet) of a cell the first pass does not finish is built
                    from its tet, clipped by the cell faces that cross the tet, four
