@@ -1432,8 +1432,8 @@ namespace vgb {
 // planes (4+j bisector j, 4+K+b start-cube face b) are build_plane_stride(K)
 // float4 of the dynamic shared memory, sized by the largest K.
 template <int CAP>
-struct BuildSmem {
-  unsigned conf[CAP];
+struct alignas(16) BuildSmem {
+  unsigned conf[CAP];  // (16-byte aligned: build_cells keeps new vertices here)
   unsigned bedge[CAP];
   unsigned cnt[WC_N];
   float4 seed;  // the group's site (read after the build rather than held in registers)
@@ -1512,6 +1512,10 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, BATCHED ? VGB_BUILD_MIN_BLO
     int pi = 4, state = 0;
     const int pend = 4 + K1;
     unsigned seq_cnt = 0u;  // planes (bits 0-7), cuts (8-15), vertex-vs-plane tests (16-31)
+    if constexpr (G == 8 && SL == 4 && !ROBUST) {
+      build_cells(c, plane, S.conf, S.bedge, (int)(sizeof(BuildSmem<G * SL>) / sizeof(unsigned)), gl, gbase, gid, pend,
+                  building, secmiss, state, seq_cnt, S.cnt + WC_NEWV);
+    } else {
     while (__any_sync(FULL, building)) {
       const float4 P = building ? plane[pi] : make_float4(0.f, 0.f, 0.f, 1.f);
       if (building) seq_cnt += 1u + ((unsigned)c.nt << 16);
@@ -1537,6 +1541,7 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, BATCHED ? VGB_BUILD_MIN_BLO
           }
         }
       }
+    }
     }
 
     // inside the mesh: the site cell's clear radius against the ball of
