@@ -153,6 +153,11 @@ struct SiteSmem {
   // completion pass: no site beyond the K nearest cut the cell, so the
   // earlier pass's moments are exact and stand
   int unchanged;
+  // completion pass: the site of each plane slot it fills, where mtri (free
+  // until the cell is stored) has not room for them
+  static constexpr bool OWN_SRC = NPLANE == COMPLETE_PLANES && WARP * SL < NPLANE;
+  unsigned own_src[OWN_SRC ? NPLANE : 1];
+  __device__ __forceinline__ unsigned* src() { return OWN_SRC ? own_src : mtri; }
 };
 
 // Compensated add (TwoSum) of x into the pair (hi, lo) in shared memory.
@@ -263,7 +268,7 @@ __device__ __forceinline__ void store_master(const WarpCell<SL>& c, SiteSmem<SL,
 // MESH (exact form, float): a cell that is not inside the mesh goes to the
 // mesh pass (clip_mesh.cuh) instead of being clipped by each tet.
 template <bool CELL_TET, bool BATCHED, int SL, bool ROBUST, bool COMPLETE = false, bool MESH = false>
-__global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : SL >= 4 ? 6 : VGB_CLIP_MIN_BLOCKS) k_clip_site(
+__global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : SL >= 4 || COMPLETE ? 6 : VGB_CLIP_MIN_BLOCKS) k_clip_site(
     const float4* __restrict__ sites, int n, const unsigned* __restrict__ knn, const ProbDesc* __restrict__ probs,
     const int* __restrict__ site_prob, const ProbDesc lone, const float4* __restrict__ verts,
     const int4* __restrict__ tets, const int* __restrict__ site_start, const int* __restrict__ site_tets,
@@ -274,7 +279,8 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : SL >= 4 ? 6 :
     const int* __restrict__ in_list, const int* __restrict__ in_count, int* __restrict__ out_list,
     int* __restrict__ out_count, int* __restrict__ work, const CellStore store, int k_tier,
     const int* __restrict__ cell_start, int* __restrict__ esc_list, float* __restrict__ esc_r2,
-    int* __restrict__ esc_count, int* __restrict__ piece_list, int* __restrict__ piece_count) {
+    int* __restrict__ esc_count, int* __restrict__ piece_list, int* __restrict__ piece_count,
+    float* __restrict__ out_r2) {
   constexpr int NPLANE = COMPLETE ? COMPLETE_PLANES : SITE_PLANES;
   constexpr int PWORDS = (NPLANE + 31) / 32;
   __shared__ SiteSmem<SL, NPLANE> smem_all[CLIP_WARPS];
@@ -735,7 +741,7 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : SL >= 4 ? 6 :
                                                  __shfl_sync(FULL, P.z, src), __shfl_sync(FULL, P.w, src));
                     if (lane == 0) {
                       S.plane[nxt] = Q;
-                      S.mtri[nxt] = (unsigned)(b0 + src);  // its site, for the mesh pass
+                      S.src()[nxt] = (unsigned)(b0 + src);  // its site, for the mesh pass
                     }
                     __syncwarp();
                     const int r = warp_clip<SL, ROBUST>(c, Q, (unsigned)nxt, S.plane, S.conf, S.bedge, lane, true,
@@ -766,6 +772,8 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : SL >= 4 ? 6 :
                       fail = nxt >= NPLANE;
                       // the rest of this chunk's candidates are tested again below
                       nfar = gather_far();
+                    } else if (r == CLIP_OVERFLOW && out_list) {
+                      abandon = fail = true;  // (the larger pass completes it)
                     } else if (r != CLIP_NONE) {
                       fail = true;
                       if (lane == 0 && (r == CLIP_OVERFLOW || r == CLIP_BOUNDARY))
@@ -774,6 +782,7 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : SL >= 4 ? 6 :
                   }
                 }
               }
+          if (abandon) break;
           cdone = !fail;
           if (cdone && ncut == 0) {
             // nothing beyond the K nearest cuts the cell: the earlier pass's
@@ -887,7 +896,7 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : SL >= 4 ? 6 :
             for (int f = lane; f < nfaces; f += WARP) {
               const int id = S.faces[f];
               to[id] = (unsigned char)(id < first_free ? id : first_free + f - own);
-              if (id >= first_free && f - own < MESH_EXT) store.faces[(size_t)s * PIECE_REC + f - own] = S.mtri[id];
+              if (id >= first_free && f - own < MESH_EXT) store.faces[(size_t)s * PIECE_REC + f - own] = S.src()[id];
             }
             __syncwarp();
             if (nfaces - own > MESH_EXT || !cdone) nt_out = MESH_VERTS + 1;
@@ -979,7 +988,13 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : SL >= 4 ? 6 :
     }
     if (abandon) {
       // the larger-capacity pass redoes this site from scratch
-      if (lane == 0) {
+      if (COMPLETE) {
+        if (lane == 0) {
+          const int pos = atomicAdd(out_count, 1);
+          out_list[pos] = s;
+          out_r2[pos] = esc_r2[it];
+        }
+      } else if (lane == 0) {
         out_list[atomicAdd(out_count, 1)] = s;
         S.cnt[WC_REDO]++;
         if (CELL_TET && store.flags) store.flags[s] = (unsigned char)(S.site_flags | SITE_REDO);
@@ -1683,9 +1698,10 @@ struct ClipPasses {
   // the 96-vertex fast pass lone / batched, the pieces pass lone / batched,
   // and of the float exact form the mesh pass, the one-warp pass and the
   // completion pass that hand on to it, lone / batched each, then the mesh
-  // pass of the reference form
+  // pass of the reference form, and the completion pass of 64 vertices, lone
+  // / batched
   static int* resident() {
-    static int r[18] = {};
+    static int r[20] = {};
     return r;
   }
   static int prepare();
@@ -1723,6 +1739,8 @@ int ClipPasses<R>::prepare() {
         resident_blocks(k_cell_mesh<false, true>, sms, r + 17) ||
         resident_blocks(k_clip_site<true, false, SLOTS_FAST, false, false, true>, sms, r + 13) ||
         resident_blocks(k_clip_site<true, true, SLOTS_FAST, false, false, true>, sms, r + 14) ||
+        resident_blocks(k_clip_site<true, false, SLOTS_FAST, false, true, true>, sms, r + 18) ||
+        resident_blocks(k_clip_site<true, true, SLOTS_FAST, false, true, true>, sms, r + 19) ||
         resident_blocks(k_clip_site<true, false, SLOTS_COMPLETE, false, true, true>, sms, r + 15) ||
         resident_blocks(k_clip_site<true, true, SLOTS_COMPLETE, false, true, true>, sms, r + 16))
       return -2;
@@ -1783,7 +1801,7 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
     k_clip_site<false, false, SLOTS_TET_CELL, R><<<(int)(want < need ? want : need), CLIP_WARPS * WARP, 0, st>>>(
         sites, n, knn, probs, site_prob, lone, verts, tets, site_start, site_tets, mom, stats, nullptr, nullptr,
         nullptr, nullptr, nullptr, nullptr, nullptr, prob_secmiss, nullptr, nullptr, nullptr, nullptr, nullptr,
-        CellStore{}, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+        CellStore{}, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
     VGB_CUDA_TRY(cudaGetLastError());
     return 0;
   }
@@ -1797,7 +1815,9 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
   // [3n, 4n) the sites to complete, [4n, 5n) their pieces' squared radius
   // bounds (float) and [5n, 6n) the pieces pass's sites or the mesh pass's;
   // [12] the mesh pass's sites, [13] its work counter, [14, 15] the same for
-  // its second launch, over completed cells (their list: [n, 2n) again)
+  // its second launch, over completed cells (their list: [n, 2n) again),
+  // [16] the cells the completion pass finds above 64 vertices (in [0, n), the
+  // bounds in [2n, 3n)), [17] the work counter of the pass that takes them
   const bool exact = tet_order != nullptr;
   int* const redo = lists;
   int* const rest = lists + n;
@@ -1824,7 +1844,7 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
         sites, n, knn, probs, site_prob, lone, verts, tets, site_start, site_tets, mom, stats, field, field_sat,
         tet_order, tet_cell_start, tet_sph, reach, reach_max_bits, prob_secmiss, in_list, in_count, out_list,
         out_count, work, cs, kt, cell_start, esc, esc_r2, exact ? counters + 10 : nullptr,
-        emit ? piece_list : nullptr, emit ? counters + 6 : nullptr);
+        emit ? piece_list : nullptr, emit ? counters + 6 : nullptr, nullptr);
   };
   // the pieces pass over the sites the one-warp pass handed on
   auto launch_pieces = [&](auto kernel, int variant) {
@@ -1863,11 +1883,12 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
   if constexpr (!R) {
     if (mesh) {
       auto pass = [&](auto kernel, int variant, const int* in_list, int* in_count, int* out_list, int* out_count,
-                      int* work, int* to_list, int* to_count) {
+                      int* work, int* to_list, int* to_count, float* r2 = nullptr, float* out_r2 = nullptr) {
         kernel<<<g_clip_resident_blocks[variant], CLIP_WARPS * WARP, 0, st>>>(
             sites, n, knn, probs, site_prob, lone, verts, tets, site_start, site_tets, mom, stats, field, field_sat,
             tet_order, tet_cell_start, tet_sph, reach, reach_max_bits, prob_secmiss, in_list, in_count, out_list,
-            out_count, work, cs, kt, cell_start, esc, esc_r2, exact ? counters + 10 : nullptr, to_list, to_count);
+            out_count, work, cs, kt, cell_start, esc, r2 ? r2 : esc_r2, exact ? counters + 10 : nullptr, to_list,
+            to_count, out_r2);
       };
       auto mesh_pass = [&](const int* in_list, int* in_count, int* work, bool last) {
         auto go = [&](auto kernel, int variant) {
@@ -1880,6 +1901,9 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
         else if (probs) go(k_cell_mesh<true, false>, 12);
         else go(k_cell_mesh<false, false>, 11);
       };
+      // (cells the completion pass finds above 64 vertices: their bounds, in
+      // the deep sites' place)
+      float* const large_r2 = reinterpret_cast<float*>(deep);
       // the cells the first pass left, finished or taken whole; then what of
       // each lies in the mesh; then the cells above 64 vertices, and those
       // their K neighbours left unresolved
@@ -1889,8 +1913,10 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
         mesh_pass(mesh_list, counters + 12, counters + 13, false);
         pass(k_clip_site<true, true, SLOTS_REDO, false>, 4, redo, counters + 1, nullptr, nullptr, counters + 4,
              nullptr, nullptr);
-        pass(k_clip_site<true, true, SLOTS_COMPLETE, false, true, true>, 16, esc, counters + 10, nullptr, nullptr,
-             counters + 11, rest, counters + 14);
+        pass(k_clip_site<true, true, SLOTS_FAST, false, true, true>, 19, esc, counters + 10, redo, counters + 16,
+             counters + 11, rest, counters + 14, nullptr, large_r2);
+        pass(k_clip_site<true, true, SLOTS_COMPLETE, false, true, true>, 16, redo, counters + 16, nullptr, nullptr,
+             counters + 17, rest, counters + 14, large_r2);
       } else {
         pass(k_clip_site<true, false, SLOTS_FAST, false, false, true>, 13, rest, counters + 0, redo, counters + 1,
              counters + 3, mesh_list, counters + 12);
@@ -1901,8 +1927,10 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
           VGB_CUDA_TRY(cudaGetLastError());
           return 0;
         }
-        pass(k_clip_site<true, false, SLOTS_COMPLETE, false, true, true>, 15, esc, counters + 10, nullptr, nullptr,
-             counters + 11, rest, counters + 14);
+        pass(k_clip_site<true, false, SLOTS_FAST, false, true, true>, 18, esc, counters + 10, redo, counters + 16,
+             counters + 11, rest, counters + 14, nullptr, large_r2);
+        pass(k_clip_site<true, false, SLOTS_COMPLETE, false, true, true>, 15, redo, counters + 16, nullptr, nullptr,
+             counters + 17, rest, counters + 14, large_r2);
       }
       mesh_pass(rest, counters + 14, counters + 15, true);
       VGB_CUDA_TRY(cudaGetLastError());

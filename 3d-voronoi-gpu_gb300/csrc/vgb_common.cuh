@@ -306,7 +306,7 @@ inline bool runs_mesh_pass(bool robust, bool tet_pieces, long long n_tet, long l
 }
 
 // Counters of the clip passes (clip_kernels.cuh lists them).
-constexpr int CLIP_COUNTERS = 16;
+constexpr int CLIP_COUNTERS = 18;
 
 int clip_site_major(bool cell_tet, const float4* sites, int n, unsigned* knn, const ProbDesc* probs,
                     const int* site_prob, const ProbDesc& lone, const float4* verts, const int4* tets,
