@@ -161,10 +161,9 @@ int layout(vgb_batch* b) {
 int batch_pass(vgb_batch* b, int update, bool count_secmiss) {
   cudaStream_t st = b->st;
   const ProbDesc none{};
-  if (grid_sort(b->sites, b->sites_tmp, b->n, b->ncell, b->d_probs, b->site_prob, none, b->cell_start, b->site_cell,
-                st))
+  if (grid_sort_in_place(b->sites, b->sites_tmp, b->n, b->ncell, b->d_probs, b->site_prob, none, b->cell_start,
+                         b->site_cell, st))
     return VGB_ERR_CUDA;
-  VGB_CUDA_TRY(cudaMemcpyAsync(b->sites, b->sites_tmp, sizeof(float4) * b->n, cudaMemcpyDeviceToDevice, st));
   // KNN_TIER neighbours first; the rest for the sites that need them (clip phase)
   const int tier = b->kmax > KNN_TIER ? KNN_TIER : 0;
   if (knn_sites(b->sites, b->n, b->cell_start, b->d_probs, b->site_prob, none, b->kmax, b->pos_of_id, b->knn,

@@ -194,9 +194,9 @@ int run_pass(vgb_engine* e, int update) {
 #define MARK(i) \
   if (e->timed) VGB_CUDA_TRY(cudaEventRecord(e->ev[i], st))
   MARK(0);
-  if (grid_sort(e->sites, e->sites_tmp, e->n, e->ncell, nullptr, nullptr, e->prob, e->cell_start, e->site_cell, st))
+  if (grid_sort_in_place(e->sites, e->sites_tmp, e->n, e->ncell, nullptr, nullptr, e->prob, e->cell_start,
+                         e->site_cell, st))
     return VGB_ERR_CUDA;
-  VGB_CUDA_TRY(cudaMemcpyAsync(e->sites, e->sites_tmp, sizeof(float4) * e->n, cudaMemcpyDeviceToDevice, st));
   MARK(1);
   const bool exact = e->field != nullptr;
   // the exact cell-tet form computes KNN_TIER neighbours first (the rest for

@@ -2,7 +2,12 @@
 // deterministic: the sites are gathered into id order with their cell keys,
 // then stably radix-sorted by cell (8-bit digits, as many passes as the cell
 // count needs: 3 at 1M sites); cell starts come from an atomic count and a
-// device exclusive scan.  Replaces kn_firstbuild's count / reserve / store
+// device exclusive scan.  Up to 65,536 sites are placed by counting instead:
+// the gather's atomic gives each site a slot of its cell, and a site's place
+// is its rank by id among its cell's (launch-bound sizes: 20k sites 160 -> 25
+// us, 500 sites 45 -> 20; above that the radix passes, whose cost does not
+// depend on how many sites share a cell, with tiles small enough to fill the
+// chip: 125k sites 46 -> 11 us a pass).  Replaces kn_firstbuild's count / reserve / store
 // (knearests.cu:29-57, 149-198), whose `reserve` hands out cell ranges in
 // atomic order and whose `store` leaves the order inside a cell to the
 // scheduler.  The cost per site does not depend on how many sites share a
@@ -115,8 +120,51 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(const int* in, int*
   }
 }
 
+// Up to SCAN_ONE_MAX ints in one block: each thread sums a run of its own,
+// the runs are scanned, and each thread writes its run out.  One launch (5 us
+// at 20,000 ints) instead of three of 3 us and their gaps.
+constexpr int SCAN_ONE_MAX = 32768;
+__global__ void __launch_bounds__(1024) k_scan_one(const int* in, int* out, int n) {
+  __shared__ int ws[32];
+  __shared__ int buf[SCAN_ONE_MAX / 4];
+  // a quarter of the largest size at a time, read and written coalesced
+  int carry = 0;
+  for (int b = 0; b < n; b += SCAN_ONE_MAX / 4) {
+    const int m = min(n - b, SCAN_ONE_MAX / 4);
+    for (int i = threadIdx.x; i < m; i += 1024) buf[i] = in[b + i];
+    __syncthreads();
+    constexpr int RUN = SCAN_ONE_MAX / 4 / 1024;
+    int s = 0;
+#pragma unroll
+    for (int i = 0; i < RUN; ++i) {
+      const int j = (int)threadIdx.x * RUN + i;
+      s += j < m ? buf[j] : 0;
+    }
+    int total;
+    int ex = block_exclusive_scan(s, ws, total) + carry;
+#pragma unroll
+    for (int i = 0; i < RUN; ++i) {
+      const int j = (int)threadIdx.x * RUN + i;
+      if (j < m) {
+        const int v = buf[j];
+        buf[j] = ex;
+        ex += v;
+      }
+    }
+    carry += total;
+    __syncthreads();
+    for (int i = threadIdx.x; i < m; i += 1024) out[b + i] = buf[i];
+    __syncthreads();
+  }
+}
+
 int scan_exclusive(const int* in, int* out, long long n, int* tmp, cudaStream_t st) {
   if (n <= 0) return 0;
+  if (n <= SCAN_ONE_MAX) {
+    k_scan_one<<<1, 1024, 0, st>>>(in, out, (int)n);
+    VGB_CUDA_TRY(cudaGetLastError());
+    return 0;
+  }
   int ntiles = (int)((n + SCAN_TILE - 1) / SCAN_TILE);
   k_scan_tile_sums<<<ntiles, SCAN_THREADS, 0, st>>>(in, n, tmp);
   k_scan_sums<<<1, 1024, 0, st>>>(tmp, ntiles);
@@ -132,7 +180,7 @@ int scan_exclusive(const int* in, int* out, long long n, int* tmp, cudaStream_t 
 // global cell keys; cell populations counted.
 __global__ void k_grid_gather(const float4* __restrict__ in, int n, const ProbDesc* __restrict__ probs,
                               const int* __restrict__ site_prob, ProbDesc lone, int* __restrict__ count,
-                              unsigned* __restrict__ key, float4* __restrict__ val) {
+                              unsigned* __restrict__ key, float4* __restrict__ val, int* __restrict__ arrived) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int pb;
@@ -142,23 +190,46 @@ __global__ void k_grid_gather(const float4* __restrict__ in, int n, const ProbDe
   const int dst = P.site_off + site_id(p);
   key[dst] = c;
   val[dst] = p;
-  atomicAdd(count + c, 1);
+  const int a = atomicAdd(count + c, 1);
+  if (arrived) arrived[dst] = a;
 }
 
-// Digit histogram of one tile of RADIX_TILE keys per warp, written bucket-major
+// Counting placement: the sites (id order) of each cell in order of arrival,
+// then each by its rank among them.
+__global__ void k_grid_place(const unsigned* __restrict__ key, const int* __restrict__ arrived, int n,
+                             const int* __restrict__ cell_start, int* __restrict__ member) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) member[cell_start[key[i]] + arrived[i]] = i;
+}
+
+__global__ void k_grid_rank(const unsigned* __restrict__ key, const int* __restrict__ member, int n,
+                            const int* __restrict__ cell_start, const float4* __restrict__ val,
+                            float4* __restrict__ out) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  const int i = member[p];
+  const unsigned c = key[i];
+  const int b = cell_start[c], e = cell_start[c + 1];
+  int r = 0;
+  for (int q = b; q < e; ++q) r += member[q] < i;
+  out[b + r] = val[i];
+}
+
+// Digit histogram of one tile of keys per warp, written bucket-major
 // (counts[digit * ntiles + tile]) so one exclusive scan gives every tile's
 // output offset per digit.
 constexpr int RADIX_WARPS = 8;
 
 __global__ void __launch_bounds__(RADIX_WARPS * 32) k_radix_hist(const unsigned* __restrict__ key, int n, int shift,
-                                                                 int ntiles, int* __restrict__ counts) {
+                                                                 int tile_keys, int ntiles,
+                                                                 int* __restrict__ counts) {
   __shared__ int hist[RADIX_WARPS][RADIX_BUCKETS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int tile = blockIdx.x * RADIX_WARPS + w;
   for (int d = lane; d < RADIX_BUCKETS; d += 32) hist[w][d] = 0;
   __syncwarp();
   if (tile < ntiles) {
-    const int b = tile * RADIX_TILE, e = min(n, b + RADIX_TILE);
+    const int b = tile * tile_keys, e = min(n, b + tile_keys);
     for (int i = b + lane; i < e; i += 32) atomicAdd(&hist[w][(key[i] >> shift) & (RADIX_BUCKETS - 1)], 1);
     __syncwarp();
     for (int d = lane; d < RADIX_BUCKETS; d += 32) counts[(size_t)d * ntiles + tile] = hist[w][d];
@@ -170,7 +241,7 @@ __global__ void __launch_bounds__(RADIX_WARPS * 32) k_radix_hist(const unsigned*
 // per-digit running offset carries the order across steps.
 __global__ void __launch_bounds__(RADIX_WARPS * 32) k_radix_scatter(const unsigned* __restrict__ key_in,
                                                                     const float4* __restrict__ val_in, int n,
-                                                                    int shift, int ntiles,
+                                                                    int shift, int tile_keys, int ntiles,
                                                                     const int* __restrict__ offsets,
                                                                     unsigned* __restrict__ key_out,
                                                                     float4* __restrict__ val_out) {
@@ -181,7 +252,7 @@ __global__ void __launch_bounds__(RADIX_WARPS * 32) k_radix_scatter(const unsign
   for (int d = lane; d < RADIX_BUCKETS; d += 32) next[w][d] = offsets[(size_t)d * ntiles + tile];
   __syncwarp();
   const unsigned lt = (1u << lane) - 1u;
-  const int b = tile * RADIX_TILE, e = min(n, b + RADIX_TILE);
+  const int b = tile * tile_keys, e = min(n, b + tile_keys);
   for (int i0 = b; i0 < e; i0 += 32) {
     const int i = i0 + lane;
     const bool valid = i < e;
@@ -199,42 +270,68 @@ __global__ void __launch_bounds__(RADIX_WARPS * 32) k_radix_scatter(const unsign
   }
 }
 
-int grid_sort(const float4* in, float4* out, int n, long long ncell, const ProbDesc* probs, const int* site_prob,
-              const ProbDesc& lone, int* cell_start, int* work, cudaStream_t st) {
+// Sites sorted from `sites` by way of `tmp`; the result is left in either,
+// *at of them.
+static int sort_sites(float4* sites, float4* tmp, int n, long long ncell, const ProbDesc* probs, const int* site_prob,
+                      const ProbDesc& lone, int* cell_start, int* work, cudaStream_t st, float4** at) {
   VGB_CUDA_TRY(cudaMemsetAsync(cell_start, 0, sizeof(int) * (ncell + 1), st));
+  const bool counting = n <= GRID_COUNT_MAX;
   const long long ntiles = grid_sort_tiles(n);
   unsigned* key_a = reinterpret_cast<unsigned*>(work);
   unsigned* key_b = key_a + n;
-  int* counts = reinterpret_cast<int*>(key_b + n);
+  int* const arrived = reinterpret_cast<int*>(key_b);
+  int* const member = arrived + n;
+  int* counts = reinterpret_cast<int*>(key_b + (counting ? 2 : 1) * (size_t)n);
   int* scan_tmp = counts + RADIX_BUCKETS * ntiles;
   // digits needed for the largest cell key
   int passes = 0;
   for (long long top = ncell > 1 ? ncell - 1 : 0; top > 0; top >>= RADIX_BITS) ++passes;
-  // ping-pong so that the last pass writes `out`: the gather fills `out` for
-  // an even count, the source array (no longer needed) for an odd one --
-  // except that the gather cannot write its own source, so an odd count
-  // starts in `out` and finishes with a copy
-  float4* va = out;
-  float4* vb = const_cast<float4*>(in);
+  float4* va = tmp;
+  float4* vb = sites;
+  const int nblk = (n + 255) / 256;
   if (n > 0) {
-    k_grid_gather<<<(n + 255) / 256, 256, 0, st>>>(in, n, probs, site_prob, lone, cell_start, key_a, va);
+    k_grid_gather<<<nblk, 256, 0, st>>>(sites, n, probs, site_prob, lone, cell_start, key_a, va,
+                                        counting ? arrived : nullptr);
     VGB_CUDA_TRY(cudaGetLastError());
   }
   if (scan_exclusive(cell_start, cell_start, ncell + 1, scan_tmp, st)) return -2;
-  if (n > 0) {
-    const int blocks = (int)((ntiles + RADIX_WARPS - 1) / RADIX_WARPS);
+  if (n > 0 && counting) {
+    k_grid_place<<<nblk, 256, 0, st>>>(key_a, arrived, n, cell_start, member);
+    k_grid_rank<<<nblk, 256, 0, st>>>(key_a, member, n, cell_start, va, vb);
+    VGB_CUDA_TRY(cudaGetLastError());
+    std::swap(va, vb);
+  } else if (n > 0) {
+    const int blocks = (int)((ntiles + RADIX_WARPS - 1) / RADIX_WARPS), tile = radix_tile(n);
     for (int ps = 0; ps < passes; ++ps) {
       const int shift = ps * RADIX_BITS;
-      k_radix_hist<<<blocks, RADIX_WARPS * 32, 0, st>>>(key_a, n, shift, (int)ntiles, counts);
+      k_radix_hist<<<blocks, RADIX_WARPS * 32, 0, st>>>(key_a, n, shift, tile, (int)ntiles, counts);
       VGB_CUDA_TRY(cudaGetLastError());
       if (scan_exclusive(counts, counts, (long long)RADIX_BUCKETS * ntiles, scan_tmp, st)) return -2;
-      k_radix_scatter<<<blocks, RADIX_WARPS * 32, 0, st>>>(key_a, va, n, shift, (int)ntiles, counts, key_b, vb);
+      k_radix_scatter<<<blocks, RADIX_WARPS * 32, 0, st>>>(key_a, va, n, shift, tile, (int)ntiles, counts, key_b, vb);
       VGB_CUDA_TRY(cudaGetLastError());
       std::swap(key_a, key_b);
       std::swap(va, vb);
     }
-    if (va != out) VGB_CUDA_TRY(cudaMemcpyAsync(out, va, sizeof(float4) * n, cudaMemcpyDeviceToDevice, st));
   }
+  *at = va;
+  return 0;
+}
+
+int grid_sort(const float4* in, float4* out, int n, long long ncell, const ProbDesc* probs, const int* site_prob,
+              const ProbDesc& lone, int* cell_start, int* work, cudaStream_t st) {
+  float4* at = nullptr;
+  const int rc = sort_sites(const_cast<float4*>(in), out, n, ncell, probs, site_prob, lone, cell_start, work, st, &at);
+  if (rc) return rc;
+  if (n > 0 && at != out) VGB_CUDA_TRY(cudaMemcpyAsync(out, at, sizeof(float4) * n, cudaMemcpyDeviceToDevice, st));
+  return 0;
+}
+
+int grid_sort_in_place(float4* sites, float4* tmp, int n, long long ncell, const ProbDesc* probs, const int* site_prob,
+                       const ProbDesc& lone, int* cell_start, int* work, cudaStream_t st) {
+  float4* at = nullptr;
+  const int rc = sort_sites(sites, tmp, n, ncell, probs, site_prob, lone, cell_start, work, st, &at);
+  if (rc) return rc;
+  if (n > 0 && at != sites) VGB_CUDA_TRY(cudaMemcpyAsync(sites, at, sizeof(float4) * n, cudaMemcpyDeviceToDevice, st));
   return 0;
 }
 

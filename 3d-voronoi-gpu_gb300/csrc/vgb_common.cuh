@@ -166,16 +166,30 @@ int scan_exclusive(const int* in, int* out, long long n, int* tmp, cudaStream_t 
 // in order and contiguous.  Stable radix sort of the sites in id order by
 // cell key; `in` is overwritten (scratch).
 //   cell_start: ncell + 1 ints; work: grid_sort_work_ints(n, ncell) ints.
+// Up to GRID_COUNT_MAX sites are placed by counting instead: a slot of its
+// cell for each site, then its rank among its cell's sites by id -- four
+// launches instead of ten to fifteen, the cost growing with the square of a
+// cell's sites, which so few bound (the kNN's does too).
 constexpr int RADIX_BITS = 8;
 constexpr int RADIX_BUCKETS = 1 << RADIX_BITS;
-constexpr int RADIX_TILE = 2048;  // keys per warp tile
-constexpr long long grid_sort_tiles(long long n) { return (n + RADIX_TILE - 1) / RADIX_TILE; }
+constexpr int GRID_COUNT_MAX = 65536;
+// Keys per warp tile: 16 warps an SM (2,432 tiles) where there are keys
+// enough, between 128 and 2,048 keys.
+constexpr int radix_tile(long long n) {
+  const long long t = (n / 2432 + 31) / 32 * 32;
+  return (int)(t < 128 ? 128 : t > 2048 ? 2048 : t);
+}
+constexpr long long grid_sort_tiles(long long n) { return (n + radix_tile(n) - 1) / radix_tile(n); }
 constexpr size_t grid_sort_work_ints(long long n, long long ncell) {
-  // two key arrays, the digit counts, the scan scratch (tiles of 2048 ints)
-  return (size_t)(2 * n + RADIX_BUCKETS * grid_sort_tiles(n) +
+  // two key arrays (counting: keys, arrival order and the cells' sites), the
+  // digit counts, the scan scratch (tiles of 2048 ints)
+  return (size_t)((n <= GRID_COUNT_MAX ? 3 : 2) * n + RADIX_BUCKETS * grid_sort_tiles(n) +
                   ((ncell + 1 > RADIX_BUCKETS * grid_sort_tiles(n) ? ncell + 1 : RADIX_BUCKETS * grid_sort_tiles(n)) +
                    2047) / 2048 + 1);
 }
+// The same with the result in `sites` (tmp: n entries of scratch).
+int grid_sort_in_place(float4* sites, float4* tmp, int n, long long ncell, const ProbDesc* probs, const int* site_prob,
+                       const ProbDesc& lone, int* cell_start, int* work, cudaStream_t st);
 int grid_sort(const float4* in, float4* out, int n, long long ncell, const ProbDesc* probs, const int* site_prob,
               const ProbDesc& lone, int* cell_start, int* work, cudaStream_t st);
 
