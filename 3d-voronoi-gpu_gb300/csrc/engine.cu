@@ -70,6 +70,9 @@ struct vgb_engine {
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // [update]
   cudaEvent_t ev[VGB_PHASES + 1] = {};
   cudaEvent_t tev[2] = {};
+  cudaStream_t st2 = nullptr;      // work beside the main stream inside a pass
+  cudaEvent_t fork = nullptr, join = nullptr;
+  int* bad_id = nullptr;           // page-locked: set by a readback that meets an id that is none
   bool timed = false;
 };
 
@@ -99,6 +102,32 @@ __global__ void k_get_positions(const float4* __restrict__ sites, int n, float* 
   xyz[3 * i] = p.x;
   xyz[3 * i + 1] = p.y;
   xyz[3 * i + 2] = p.z;
+}
+
+// Positions and ids in grid order; positions in input order.
+__global__ void k_get_sites(const float4* __restrict__ sites, int n, float* __restrict__ xyz, int* __restrict__ ids) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  float4 p = sites[i];
+  xyz[3 * i] = p.x;
+  xyz[3 * i + 1] = p.y;
+  xyz[3 * i + 2] = p.z;
+  if (ids) ids[i] = site_id(p);
+}
+
+// (bad: page-locked host int, written only for an id that is none)
+__global__ void k_get_original(const float4* __restrict__ sites, int n, float* __restrict__ xyz, int* bad) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  float4 p = sites[i];
+  const int id = site_id(p);
+  if (id < 0 || id >= n) {
+    *bad = 1;
+    return;
+  }
+  xyz[3 * id] = p.x;
+  xyz[3 * id + 1] = p.y;
+  xyz[3 * id + 2] = p.z;
 }
 
 __global__ void k_pack_mesh(const float* __restrict__ v, int nv, float4* __restrict__ out) {
@@ -184,6 +213,10 @@ void free_engine(vgb_engine* e) {
                   e->store.mnt, e->rec, e->last, e->beside};
   for (void* b : bufs)
     if (b) cudaFree(b);
+  if (e->fork) cudaEventDestroy(e->fork);
+  if (e->join) cudaEventDestroy(e->join);
+  if (e->st2) cudaStreamDestroy(e->st2);
+  if (e->bad_id) cudaFreeHost(e->bad_id);
   if (e->st) cudaStreamDestroy(e->st);
   delete e;
 }
@@ -199,6 +232,17 @@ int run_pass(vgb_engine* e, int update) {
     return VGB_ERR_CUDA;
   MARK(1);
   const bool exact = e->field != nullptr;
+  // the reach of the tets beside the kNN (both read the sorted sites only),
+  // unless the phases are timed
+  const bool aside = exact && !e->timed;
+  if (aside) {
+    VGB_CUDA_TRY(cudaEventRecord(e->fork, st));
+    VGB_CUDA_TRY(cudaStreamWaitEvent(e->st2, e->fork, 0));
+    if (tet_reach(e->sites, e->cell_start, nullptr, nullptr, e->prob, 1, e->tet_sph, e->n_tet, e->reach,
+                  e->reach_max, e->st2))
+      return VGB_ERR_CUDA;
+    VGB_CUDA_TRY(cudaEventRecord(e->join, e->st2));
+  }
   // the exact cell-tet form computes KNN_TIER neighbours first (the rest for
   // the sites that need them, in the clip phase)
   const int tier = (exact && e->cfg.method == VGB_METHOD_CELL_TET && e->K > KNN_TIER) ? KNN_TIER : 0;
@@ -206,8 +250,8 @@ int run_pass(vgb_engine* e, int update) {
                 st, tier, e->shape.knn_warps))
     return VGB_ERR_CUDA;
   MARK(2);
-  if (exact && tet_reach(e->sites, e->cell_start, nullptr, nullptr, e->prob, 1, e->tet_sph, e->n_tet, e->reach,
-                         e->reach_max, st))
+  if (exact && !aside && tet_reach(e->sites, e->cell_start, nullptr, nullptr, e->prob, 1, e->tet_sph, e->n_tet,
+                                   e->reach, e->reach_max, st))
     return VGB_ERR_CUDA;
   if (!exact &&
       knn_tet_centroids(e->sites, e->n, e->dim, e->cell_start, e->pos_of_id, e->verts, e->tets, e->tet_order,
@@ -224,6 +268,7 @@ int run_pass(vgb_engine* e, int update) {
   }
   VGB_CUDA_TRY(cudaMemsetAsync(e->stats, 0, sizeof(unsigned long long) * VGB_STAT_COUNT, st));
   if (e->cfg.method == VGB_METHOD_PLAIN) VGB_CUDA_TRY(cudaMemsetAsync(e->mom_f, 0, sizeof(float4) * e->n, st));
+  if (aside) VGB_CUDA_TRY(cudaStreamWaitEvent(st, e->join, 0));
   MARK(4);
   if (e->cfg.method != VGB_METHOD_PLAIN) {
     if (clip_site_major(e->cfg.method == VGB_METHOD_CELL_TET, e->sites, e->n, e->knn, nullptr, nullptr, e->prob,
@@ -418,7 +463,12 @@ int vgb_engine_create(vgb_engine** out, const vgb_config* cfg_in, const float* v
   if (ce != cudaSuccess) { set_error("cudaSetDevice(%d): %s", cfg.device, cudaGetErrorString(ce)); delete e; return VGB_ERR_CUDA; }
   if (knn_prepare() || clip_prepare()) { delete e; return VGB_ERR_CUDA; }
   ce = cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking);
-  if (ce != cudaSuccess) { set_error("stream: %s", cudaGetErrorString(ce)); delete e; return VGB_ERR_CUDA; }
+  if (exact_grid) {  // (only the exact form has work beside the main stream)
+    if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&e->st2, cudaStreamNonBlocking);
+    if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&e->fork, cudaEventDisableTiming);
+    if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&e->join, cudaEventDisableTiming);
+  }
+  if (ce != cudaSuccess) { set_error("stream: %s", cudaGetErrorString(ce)); free_engine(e); return VGB_ERR_CUDA; }
   int rc = VGB_OK;
   size_t pairs = (size_t)n_tet * e->tk;
   const bool exact_form = cfg.method == VGB_METHOD_CELL_TET && cfg.exact;
@@ -719,29 +769,25 @@ int vgb_engine_copy_buffer(vgb_engine* e, int which, void* host, size_t bytes) {
 
 int vgb_engine_get_sites(vgb_engine* e, float* xyz, int* ids) {
   if (!e || !xyz) { set_error("NULL argument"); return VGB_ERR_INVALID; }
-  std::vector<float> buf(4 * (size_t)e->n);
-  int rc = vgb_engine_copy_buffer(e, VGB_BUF_SITES, buf.data(), buf.size() * sizeof(float));
-  if (rc) return rc;
-  for (int i = 0; i < e->n; ++i) {
-    xyz[3 * (size_t)i] = buf[4 * (size_t)i];
-    xyz[3 * (size_t)i + 1] = buf[4 * (size_t)i + 1];
-    xyz[3 * (size_t)i + 2] = buf[4 * (size_t)i + 2];
-    if (ids) std::memcpy(ids + i, &buf[4 * (size_t)i + 3], sizeof(int));
-  }
+  // packed on the device, then straight to the caller's arrays
+  int* const d_ids = reinterpret_cast<int*>(e->sites_tmp);
+  k_get_sites<<<(e->n + 255) / 256, 256, 0, e->st>>>(e->sites, e->n, e->io_stage, ids ? d_ids : nullptr);
+  VGB_CUDA_TRY(cudaGetLastError());
+  VGB_CUDA_TRY(cudaMemcpyAsync(xyz, e->io_stage, sizeof(float) * 3 * e->n, cudaMemcpyDeviceToHost, e->st));
+  if (ids) VGB_CUDA_TRY(cudaMemcpyAsync(ids, d_ids, sizeof(int) * e->n, cudaMemcpyDeviceToHost, e->st));
+  VGB_CUDA_TRY(cudaStreamSynchronize(e->st));
   return VGB_OK;
 }
 
 int vgb_engine_get_sites_original(vgb_engine* e, float* xyz) {
   if (!e || !xyz) { set_error("NULL argument"); return VGB_ERR_INVALID; }
-  std::vector<float> buf(3 * (size_t)e->n);
-  std::vector<int> ids(e->n);
-  int rc = vgb_engine_get_sites(e, buf.data(), ids.data());
-  if (rc) return rc;
-  for (int i = 0; i < e->n; ++i) {
-    int id = ids[i];
-    if (id < 0 || id >= e->n) { set_error("corrupt site id %d", id); return VGB_ERR_STATE; }
-    std::memcpy(xyz + 3 * (size_t)id, &buf[3 * (size_t)i], 3 * sizeof(float));
-  }
+  if (!e->bad_id) VGB_CUDA_TRY(cudaHostAlloc((void**)&e->bad_id, sizeof(int), cudaHostAllocMapped));
+  *e->bad_id = 0;
+  k_get_original<<<(e->n + 255) / 256, 256, 0, e->st>>>(e->sites, e->n, e->io_stage, e->bad_id);
+  VGB_CUDA_TRY(cudaGetLastError());
+  VGB_CUDA_TRY(cudaMemcpyAsync(xyz, e->io_stage, sizeof(float) * 3 * e->n, cudaMemcpyDeviceToHost, e->st));
+  VGB_CUDA_TRY(cudaStreamSynchronize(e->st));
+  if (*static_cast<volatile int*>(e->bad_id)) { set_error("corrupt site id"); return VGB_ERR_STATE; }
   return VGB_OK;
 }
 
