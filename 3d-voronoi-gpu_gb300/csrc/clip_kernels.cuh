@@ -79,13 +79,13 @@ constexpr int CLIP_WARPS = 4;
 constexpr int BOX_PLANES = 6;
 // Resident blocks per SM the clip kernels are compiled for (the register
 // budget per thread is 65536 / (CLIP_WARPS * 32 * blocks)): measured, the
-// lone first pass is fastest at 8 (64 registers), the batched one at 7 (72,
-// where it spills nothing; 1% on the 256 Kuhn cubes).
+// first pass is fastest at 7 (72 registers, where it spills nothing; clip
+// phase of 1M relaxed sites 5.07 ms against 5.17 at 8), the one-warp pass at 8.
 #ifndef VGB_CLIP_MIN_BLOCKS
 #define VGB_CLIP_MIN_BLOCKS 8
 #endif
 #ifndef VGB_BUILD_MIN_BLOCKS
-#define VGB_BUILD_MIN_BLOCKS 8
+#define VGB_BUILD_MIN_BLOCKS 7
 #endif
 #ifndef VGB_BUILD_MIN_BLOCKS_BATCHED
 #define VGB_BUILD_MIN_BLOCKS_BATCHED 7

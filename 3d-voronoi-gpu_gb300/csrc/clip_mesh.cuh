@@ -27,13 +27,14 @@
 // exact near the site as a short one.
 //
 // One warp per site: lanes take candidate tets, then (tet, edge) pairs, then
-// faces.  Bound by instruction issue and the latency of its short loops, like
-// the pass it replaces, but a boundary cell (at 1M torus sites 36 edges, 20
+// faces.  Bound by instruction fetch and issue and the latency of its short
+// loops (loops are kept rolled: at 70 KB of code half the stalls were fetches
+// and the pass took 2.0 ms where it takes 1.4 at 50 KB).  A boundary cell (at 1M torus sites 36 edges, 20
 // tets, 6 open triangles) needs no vertices of its pieces, whose inner faces
 // only cancel.  Measured per Lloyd iteration: 1M sites in 1.96M tets 15.0 ->
-// 6.6 ms from random sites and 4.6 -> 2.4 ms once relaxed (the one-warp pass
+// 5.7 ms from random sites and 4.6 -> 1.8 ms once relaxed (the one-warp pass
 // before, now that pass without its tets and this one); 131k sites in 1.57M
-// tets 6.9 -> 2.5 ms and 1.6 -> 0.6 ms (pieces from the tets before).
+// tets 6.9 -> 2.3 ms and 1.6 -> 0.5 ms (pieces from the tets before).
 #pragma once
 
 #include "clip_warp.cuh"
@@ -43,7 +44,9 @@ namespace vgb {
 constexpr int MESH_WARPS = 4;
 // A cell of at most 64 vertices (three faces meet in each) has at most 34
 // faces and 96 edges.
-constexpr int MESH_FACES = 36, MESH_EDGES = 96;
+constexpr int MESH_FACES = 34, MESH_EDGES = 96;
+static_assert(MESH_EDGES == 3 * MESH_VERTS / 2 && MESH_FACES == MESH_VERTS / 2 + 2, "a simple polytope");
+constexpr int MESH_TETS = 16;  // tets in hand
 constexpr int MESH_IDS = 4 + MAX_SITE_K + 12 + MESH_EXT;  // plane ids a stored cell may use
 constexpr int MESH_ID_WORDS = (MESH_IDS + 31) / 32;
 // A cell whose terms from the site exceed this many times their sum is done
@@ -62,7 +65,7 @@ struct MeshSmem {
     struct {
       unsigned char loc[MESH_ID_WORDS * 32];  // plane id -> face
     };
-    float4 tp[WARP][4];  // the face planes of the tets in hand, in mesh order
+    float4 tp[MESH_TETS][4];  // the face planes of the tets in hand, in mesh order
   };
   union {
     unsigned char twin[MESH_FACES * MESH_FACES];  // (p, q) -> vertex, while the edges are made
@@ -73,8 +76,10 @@ struct MeshSmem {
   float4 epos[MESH_EDGES], edir[MESH_EDGES], eterm[MESH_EDGES];
   unsigned edge[MESH_EDGES];  // faces p, q and end vertices of each
   float3 vert[MESH_VERTS];    // the cell's vertices
-  int tidx[WARP];       // tets in hand: their record, and what is known of them
-  unsigned char tinf[WARP], thit[WARP];
+  float4 side[3][2];  // a triangle's sides: point and direction, end parameters in w
+  float at[3][MESH_FACES];  // where each face meets them
+  int tidx[MESH_TETS];  // tets in hand: their record, and what is known of them
+  unsigned char tinf[MESH_TETS], thit[MESH_TETS];
   int queue[2 * WARP];  // tets whose sphere meets the cell's
   int rng[2][WARP];     // the rows in hand: first tet, tets of the rows before
   unsigned cnt[WC_N];
@@ -149,7 +154,8 @@ struct Line {
 __device__ __forceinline__ Line line_of(float3 P, float3 Q) {
   Line L;
   const float3 d = sub_rn(Q, P);
-  const float il = __frsqrt_rn(dot_rn(d, d));
+  const float dd = dot_rn(d, d), r0 = rsqrtf(dd);
+  const float il = __fmul_rn(r0, __fmaf_rn(__fmul_rn(-0.5f * dd, r0), r0, 1.5f));  // (one Newton step)
   L.u = make_float3(__fmul_rn(d.x, il), __fmul_rn(d.y, il), __fmul_rn(d.z, il));
   L.a = dot_rn(P, L.u);
   L.b = dot_rn(Q, L.u);
@@ -219,7 +225,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
       }
     __syncwarp();
     int nf = 0;
-#pragma unroll
+#pragma unroll 1
     for (int w = 0; w < MESH_ID_WORDS; ++w) {
       const int id = w * WARP + lane;
       const bool has = S.loc[id] != 0;
@@ -240,7 +246,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
       nf += __popc(m);
     }
     __syncwarp();
-    bool bad = nf > MESH_FACES || nt < 4;
+    bool bad = nf > MESH_FACES || nt < 4 ;
     nf = min(nf, MESH_FACES);
     float lm = 0.f;
 #pragma unroll
@@ -282,6 +288,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
     bad |= ne > MESH_EDGES || ne < 6;
     ne = max(min(ne, MESH_EDGES), 1);
     __syncwarp();
+#pragma unroll 1
     for (int i = lane; i < ne; i += WARP) {
       const unsigned E = S.edge[i];
       const float4 P = S.plane[E & 0xffu], Q = S.plane[(E >> 8) & 0xffu];
@@ -315,14 +322,20 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
     };
     int nclip = 0;
     const float h = 1000.f / (float)dim;
-    const int j0 = grid_axis(seed.y - R, dim), k0 = grid_axis(seed.z - R, dim);
-    const int nj = grid_axis(seed.y + R, dim) - j0 + 1;
-    const int nrow = nj * (grid_axis(seed.z + R, dim) - k0 + 1);
+    // (the cell of a coordinate up to its rounding, well below the margins)
+    const float per = __fmul_rn((float)dim, 1e-3f);
+    auto cell_at = [&](float x) { return min(max((int)floorf(__fmul_rn(x, per)), 0), dim - 1); };
+    const int j0 = cell_at(seed.y - R), k0 = cell_at(seed.z - R);
+    const int nj = cell_at(seed.y + R) - j0 + 1;
+    const int nrow = nj * (cell_at(seed.z + R) - k0 + 1);
+    const float per_row = __fdividef(1.f, (float)nj);
+#pragma unroll 1
     for (int round = 0; round < 3 && !bad; ++round) {
       MeshSum sum;
       float far2 = 0.f;
       // a piece [a, b] of an edge: k = det(F1 - F0, p, u) (b - a), and the
       // moment k1 (F1 + a + b) - k0 (F0 + a + b)
+#pragma unroll 1
       for (int i = lane; i < ne; i += WARP) {
         const unsigned E = S.edge[i];
         const float3 F0 = foot_of(S.plane[E & 0xffu], X), F1 = foot_of(S.plane[(E >> 8) & 0xffu], X);
@@ -348,7 +361,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
             const int r = row0 + lane;
             int len = 0, rb = 0;
             if (r < nrow) {
-              const int j = j0 + r % nj, k = k0 + r / nj;
+              const int rk = (int)__fmul_rn((float)r + 0.5f, per_row), k = k0 + rk, j = j0 + r - rk * nj;
               // (the cells at the ends of the grid also hold what lies beyond)
               const float m = 0.01f;
               float lo = j == 0 ? -FLT_MAX : __fmaf_rn((float)j, h, -m);
@@ -359,10 +372,10 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
               const float dz = fmaxf(fmaxf(lo - seed.z, seed.z - hi), 0.f);
               const float left = __fmaf_rn(__fmul_rn(R, R), 1.0001f, -__fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
               if (left >= 0.f) {
-                const float w = __fadd_rn(sqrtf(left), m);
+                const float w = __fmaf_rn(left, rsqrtf(fmaxf(left, 1e-12f)), m);
                 const int row = cbase + dim * (j + dim * k);
-                rb = tet_cell_start[row + grid_axis(seed.x - w, dim)];
-                len = tet_cell_start[row + grid_axis(seed.x + w, dim) + 1] - rb;
+                rb = tet_cell_start[row + cell_at(seed.x - w)];
+                len = tet_cell_start[row + cell_at(seed.x + w) + 1] - rb;
               }
             }
             row0 += WARP;
@@ -394,9 +407,16 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
             // tet's reach: beyond it every point of the tet has a nearer site
             const float4 sp = tet_sph[idx];
             const float ex = sp.x - seed.x, ey = sp.y - seed.y, ez = sp.z - seed.z;
-            const float dm = sqrtf(dot3_rn(ex, ey, ez, ex, ey, ez));
-            meets = dm <= __fmaf_rn(__fadd_rn(Rc, sp.w), 1.0001f, 1e-3f);
-            if (meets) meets = REF ? candidate(idx) : dm <= __fmaf_rn(reach[idx], 1.0001f, 1e-2f);
+            const float d2 = dot3_rn(ex, ey, ez, ex, ey, ez), ds = __fmaf_rn(__fadd_rn(Rc, sp.w), 1.0001f, 1e-3f);
+            meets = d2 <= __fmul_rn(ds, ds);
+            if (meets) {
+              if (REF) {
+                meets = candidate(idx);
+              } else {
+                const float dr = __fmaf_rn(reach[idx], 1.0001f, 1e-2f);
+                meets = d2 <= __fmul_rn(dr, dr);
+              }
+            }
           }
           const unsigned m = __ballot_sync(FULL, meets);
           if (meets) S.queue[nq + __popc(m & lt_mask)] = idx;
@@ -425,6 +445,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
                      A2 = make_float3(r1.z, r1.w, r2.x), A3 = make_float3(r2.y, r2.z, r2.w);
         const float3 sd = make_float3(seed.x, seed.y, seed.z);
         const float3 c0 = sub_rn(A0, sd), c1 = sub_rn(A1, sd), c2 = sub_rn(A2, sd), c3 = sub_rn(A3, sd);
+#pragma unroll 2
         for (int f = 0; f < nf; ++f) {
           if (!__any_sync(FULL, alive)) break;
           const float4 P = S.plane[f];
@@ -432,21 +453,24 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
           alive &= !(e < 0.f);
         }
         const unsigned am = __ballot_sync(FULL, alive);
-        const int nb = __popc(am);
-        // the rest of the queue to its front
+        const int nb = min(__popc(am), MESH_TETS), place = __popc(am & lt_mask);
+        // the rest of the queue to its front, then what is more than can be
+        // held (those are looked at again)
         const int rest = nq - take;
         const int move = lane < rest ? S.queue[take + lane] : 0;
         __syncwarp();
         if (lane < rest) S.queue[lane] = move;
-        nq = rest;
+        if (alive && place >= MESH_TETS) S.queue[rest + place - MESH_TETS] = idx;
+        alive &= place < MESH_TETS;
+        nq = rest + __popc(am) - nb;
         if (lane == 0) {
-          if (!REF) S.cnt[WC_CULLED] += (unsigned)(take - nb);
+          if (!REF) S.cnt[WC_CULLED] += (unsigned)(take - __popc(am));
           if (!REF) S.cnt[WC_CLIPPED] += (unsigned)nb;
           S.cnt[WC_CULLTESTS] += (unsigned)(take * nf);
           S.cnt[WC_CONFLICT] += (unsigned)(8 * ne * nb);
         }
         if (alive) {
-          const int pos = __popc(am & lt_mask);
+          const int pos = place;
           auto face = [&](int i, float3 a, float3 b, float3 c, float3 ca) {
             const float3 n = cross_rn(sub_rn(b, a), sub_rn(c, a));
             S.tp[pos][i] = make_float4(n.x, n.y, n.z, -dot_rn(n, ca));
@@ -477,6 +501,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
         {
           int b = lane / ne, e = lane - b * ne;
           const int db = WARP / ne, de = WARP - db * ne;
+#pragma unroll 1
           for (int w = lane; w < nb * ne; w += WARP) {
             const float4 ep = S.epos[e], eu = S.edir[e];
             const float3 p = xyz(ep), u = xyz(eu);
@@ -511,9 +536,9 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
           }
         }
         __syncwarp();
-        const unsigned hits = __ballot_sync(FULL, lane < nb && S.thit[lane] != 0);
-        const unsigned farm = __ballot_sync(FULL, lane < nb && (S.tinf[lane] & 64u) != 0u);
-        unsigned open = __ballot_sync(FULL, lane < nb && (S.tinf[lane] & 15u) != 0u);
+        const unsigned hits = __ballot_sync(FULL, lane < nb && S.thit[lane & (MESH_TETS - 1)] != 0);
+        const unsigned farm = __ballot_sync(FULL, lane < nb && (S.tinf[lane & (MESH_TETS - 1)] & 64u) != 0u);
+        unsigned open = __ballot_sync(FULL, lane < nb && (S.tinf[lane & (MESH_TETS - 1)] & 15u) != 0u);
         nclip += nb;
         if (lane == 0) {
           S.cnt[WC_CONTRIB] += (unsigned)__popc(hits);
@@ -525,6 +550,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
         // tets' edges, one per lane; the cell's edges are in far2)
         if ((farm >> lane) & 1u) S.thit[__popc(farm & lt_mask)] = (unsigned char)lane;
         __syncwarp();
+#pragma unroll 1
         for (int w = lane; w < 6 * __popc(farm); w += WARP) {
           const int e = w % 6;
           const float4* q = rec + 4 * (size_t)S.tidx[S.thit[w / 6]];
@@ -534,6 +560,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
           const float3 P = e < 3 ? c0 : e < 5 ? c1 : c2, Q = e == 0 ? c1 : (e == 1 || e == 3) ? c2 : c3;
           const Line L = line_of(sub_rn(P, site), sub_rn(Q, site));
           float lo = L.a, hi = L.b;
+#pragma unroll 2
           for (int f = 0; f < nf; ++f) {
             bool up;
             const float t = line_at(S.plane[f], L.p, L.u, up);
@@ -556,6 +583,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
             // triangle (t0, t1, t2): face i, in mesh order
             const float3 t0 = i == 0 ? c[1] : c[0], t1 = i <= 1 ? c[2] : c[1], t2 = i <= 2 ? c[3] : c[2];
             bool out = false;
+#pragma unroll 1
             for (int f = lane; f < nf; f += WARP) {
               const float4 P = S.plane[f];
               out |= fmaxf(fmaxf(eval4(P, t0), eval4(P, t1)), eval4(P, t2)) < 0.f;
@@ -573,6 +601,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
             const unsigned up0 = __ballot_sync(FULL, lane < nt && eval4(PT, S.vert[lane]) >= 0.f);
             const unsigned up1 = __ballot_sync(FULL, lane + WARP < nt && eval4(PT, S.vert[lane + WARP]) >= 0.f);
             auto above = [&](unsigned v) { return ((v < WARP ? up0 : up1) >> (v & 31u)) & 1u; };
+#pragma unroll 1
             for (int e = lane; e < ne; e += WARP) {
               const unsigned E = S.edge[e];
               const bool end = above(E >> 24) != 0u;
@@ -586,42 +615,57 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
                 S.slot[1 - in][(E >> 8) & 0xffu] = make_float4(x.x, x.y, x.z, 1.f);
               }
             }
-            // its sides: 0 (t1, t2), 1 (t0, t2), 2 (t0, t1)
-            const Line L0 = line_of(t1, t2), L1 = line_of(t0, t2), L2 = line_of(t0, t1);
+            // its sides: 0 (t1, t2), 1 (t0, t2), 2 (t0, t1), a line each on
+            // lanes 0-2
+            if (lane < 3) {
+              const Line L = line_of(lane == 0 ? t1 : t0, lane == 2 ? t1 : t2);
+              S.side[lane][0] = make_float4(L.p.x, L.p.y, L.p.z, L.a);
+              S.side[lane][1] = make_float4(L.u.x, L.u.y, L.u.z, L.b);
+            }
             const float3 FT = foot_of(PT, X);
             __syncwarp();
-            float l0 = L0.a, h0 = L0.b, l1 = L1.a, h1 = L1.b, l2 = L2.a, h2 = L2.b;
+            float lo = 1.f, hi = -1.f;  // lanes 0-2: the side's part inside the cell
+#pragma unroll 1
+            for (int k = 0; k < 3; ++k) {
+              const float4 Lp = S.side[k][0], Lu = S.side[k][1];
+              float l = Lp.w, h = Lu.w;
+#pragma unroll 1
+              for (int f = lane; f < nf; f += WARP) {
+                bool up;
+                const float w = line_at(S.plane[f], xyz(Lp), xyz(Lu), up);
+                if (up) l = fmaxf(l, w); else h = fminf(h, w);
+                S.at[k][f] = w;
+              }
+              l = redux_max(l);
+              h = redux_min(h);
+              if (lane == k) lo = l, hi = h;
+            }
+            // its plane across each face, cut by the sides
+#pragma unroll 1
             for (int f = lane; f < nf; f += WARP) {
-              const float4 P = S.plane[f];
-              bool up0, up1, up2;
-              const float w0 = line_at(P, L0.p, L0.u, up0), w1 = line_at(P, L1.p, L1.u, up1),
-                          w2 = line_at(P, L2.p, L2.u, up2);
-              if (up0) l0 = fmaxf(l0, w0); else h0 = fminf(h0, w0);
-              if (up1) l1 = fmaxf(l1, w1); else h1 = fminf(h1, w1);
-              if (up2) l2 = fmaxf(l2, w2); else h2 = fminf(h2, w2);
               const float4 a4 = S.slot[0][f], b4 = S.slot[1][f];
               if (a4.w != 0.f && b4.w != 0.f) {
                 float3 a = xyz(a4), bb = xyz(b4);
                 bool keep = true;
-                // the side planes: the tet's faces that leave out t0, t1, t2
-                auto cut = [&](int o, const Line& L, float w) {
+#pragma unroll 1
+                for (int k = 0; k < 3; ++k) {
+                  // the side's other plane: the tet's face that leaves out its
+                  // opposite corner
+                  const int o = k < i ? k : k + 1;
                   const float4 PS = S.tp[b][o];
                   const bool pos = face_side(inf, o);
                   const float va = eval4(PS, a), vb = eval4(PS, bb);
                   const bool oa = pos ? va < 0.f : va > 0.f, ob = pos ? vb < 0.f : vb > 0.f;
                   keep &= !(oa && ob);
                   if (oa != ob) {
-                    const float3 y = along(L.p, w, L.u);
+                    const float3 y = along(xyz(S.side[k][0]), S.at[k][f], xyz(S.side[k][1]));
                     if (oa) a = y; else bb = y;
                   }
-                };
-                cut(i == 0 ? 1 : 0, L0, w0);
-                cut(i <= 1 ? 2 : 1, L1, w1);
-                cut(i <= 2 ? 3 : 2, L2, w2);
+                }
                 if (keep) {
                   const float3 aX = sub_rn(a, X), bX = sub_rn(bb, X);
                   const float3 cr = cross_rn(aX, bX), ab = make_float3(__fadd_rn(aX.x, bX.x), __fadd_rn(aX.y, bX.y), __fadd_rn(aX.z, bX.z));
-                  const float3 F = foot_of(P, X);
+                  const float3 F = foot_of(S.plane[f], X);
                   if (round == 1) {
                     sum.add(1.f, make_float3(0.f, 0.f, 0.f), ab);
                   } else {
@@ -631,19 +675,10 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
                 }
               }
             }
-            // the sides inside the cell (lanes 0-2), walked around the inward
-            // normal
-            l0 = redux_max(l0);
-            l1 = redux_max(l1);
-            l2 = redux_max(l2);
-            h0 = redux_min(h0);
-            h1 = redux_min(h1);
-            h2 = redux_min(h2);
-            const float lo = lane == 0 ? l0 : lane == 1 ? l1 : l2, hi = lane == 0 ? h0 : lane == 1 ? h1 : h2;
-            if (lane < 3 && hi > lo) {
-              const float3 p = lane == 0 ? L0.p : lane == 1 ? L1.p : L2.p, u = lane == 0 ? L0.u : lane == 1 ? L1.u : L2.u;
-              const float3 a = along(p, lo, u), bb = along(p, hi, u);
-              const float3 aX = sub_rn(a, X), bX = sub_rn(bb, X);
+            // the sides inside the cell, walked around the inward normal
+            if (hi > lo) {
+              const float3 p = xyz(S.side[lane][0]), u = xyz(S.side[lane][1]);
+              const float3 aX = sub_rn(along(p, lo, u), X), bX = sub_rn(along(p, hi, u), X);
               const float3 cr = cross_rn(aX, bX), ab = make_float3(__fadd_rn(aX.x, bX.x), __fadd_rn(aX.y, bX.y), __fadd_rn(aX.z, bX.z));
               const float k6 = dot_rn(FT, cr);
               sum.add(round == 1 ? 1.f : (side == (lane != 1)) ? -k6 : k6,

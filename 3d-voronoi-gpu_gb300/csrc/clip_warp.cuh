@@ -381,17 +381,21 @@ __device__ __forceinline__ void warp_moments(const WarpCell<SL>& c, const float4
   const float inv = __frcp_rn((float)c.nt);
   const float cx = __fmul_rn(warp_sum(sx), inv), cy = __fmul_rn(warp_sum(sy), inv), cz = __fmul_rn(warp_sum(sz), inv);
   float lv = 0.f, lmx = 0.f, lmy = 0.f, lmz = 0.f;
+#pragma unroll 1
+  for (int k = 0; k < SL; ++k) {  // (one copy of the vertex code, as group_moments)
+    unsigned vm = c.vm[0], T = c.tri[0];
+    float vx = c.vx[0], vy = c.vy[0], vz = c.vz[0];
 #pragma unroll
-  for (int k = 0; k < SL; ++k) {
-    if (c.vm[k] & lane_bit) {
-      const unsigned T = c.tri[k];
+    for (int j = 1; j < SL; ++j)
+      if (j == k) vm = c.vm[j], T = c.tri[j], vx = c.vx[j], vy = c.vy[j], vz = c.vz[j];
+    if (vm & lane_bit) {
       float4 q0 = planes[tri_at(T, 0)], q1 = planes[tri_at(T, 1)], q2 = planes[tri_at(T, 2)];
       q0.w = __fadd_rn(q0.w, dot3_rn(q0.x, q0.y, q0.z, cx, cy, cz));  // planes relative to the apex
       q1.w = __fadd_rn(q1.w, dot3_rn(q1.x, q1.y, q1.z, cx, cy, cz));
       q2.w = __fadd_rn(q2.w, dot3_rn(q2.x, q2.y, q2.z, cx, cy, cz));
       float v6;
       float3 m24;
-      vertex_moments(make_float3(c.vx[k] - cx, c.vy[k] - cy, c.vz[k] - cz), q0, q1, q2, v6, m24);
+      vertex_moments(make_float3(vx - cx, vy - cy, vz - cz), q0, q1, q2, v6, m24);
       lv += v6;
       lmx += m24.x;
       lmy += m24.y;
@@ -911,17 +915,23 @@ __device__ __forceinline__ void group_moments(const WarpCell<SL>& c, const float
   const float cx = __fmul_rn(group_sum<G>(sx), inv), cy = __fmul_rn(group_sum<G>(sy), inv),
               cz = __fmul_rn(group_sum<G>(sz), inv);
   float lv = 0.f, lmx = 0.f, lmy = 0.f, lmz = 0.f;
-#pragma unroll
+  // (one copy of the vertex code, its slot's registers picked: four copies
+  // are 15 KB of instructions, and their fetch showed in the stalls)
+#pragma unroll 1
   for (int k = 0; k < SL; ++k) {
-    if (c.vm[k] & lb) {
-      const unsigned T = c.tri[k];
+    unsigned vm = c.vm[0], T = c.tri[0];
+    float vx = c.vx[0], vy = c.vy[0], vz = c.vz[0];
+#pragma unroll
+    for (int j = 1; j < SL; ++j)
+      if (j == k) vm = c.vm[j], T = c.tri[j], vx = c.vx[j], vy = c.vy[j], vz = c.vz[j];
+    if (vm & lb) {
       float4 q0 = planes[tri_at(T, 0)], q1 = planes[tri_at(T, 1)], q2 = planes[tri_at(T, 2)];
       q0.w = __fadd_rn(q0.w, dot3_rn(q0.x, q0.y, q0.z, cx, cy, cz));  // planes relative to the apex
       q1.w = __fadd_rn(q1.w, dot3_rn(q1.x, q1.y, q1.z, cx, cy, cz));
       q2.w = __fadd_rn(q2.w, dot3_rn(q2.x, q2.y, q2.z, cx, cy, cz));
       float v6;
       float3 m24;
-      vertex_moments(make_float3(c.vx[k] - cx, c.vy[k] - cy, c.vz[k] - cz), q0, q1, q2, v6, m24);
+      vertex_moments(make_float3(vx - cx, vy - cy, vz - cz), q0, q1, q2, v6, m24);
       lv += v6;
       lmx += m24.x;
       lmy += m24.y;
