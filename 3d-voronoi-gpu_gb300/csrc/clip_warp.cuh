@@ -769,8 +769,8 @@ __device__ __forceinline__ int group_clip(WarpCell<SL>& c, const float4 P, const
 //   * every group tests planes until it has one that cuts its cell (a third
 //     of them do not; a group that has one waits);
 //   * the groups cut together: boundary edges by match_any as in group_clip,
-//     in two halves of the warp when the four cavities have more than 32
-//     edges; then one new vertex per lane, kept in shared memory, and each
+//     in turns when the four cavities have more than 32 edges (one round in
+//     three; a group that has ended tests on, unheard); then one new vertex per lane, kept in shared memory, and each
 //     freed slot takes its own.  (Each slot computing its own vertex runs the
 //     vertex code once per slot a cavity has freed, for one or two lanes at a
 //     time.)
@@ -794,6 +794,7 @@ __device__ __forceinline__ void build_cells(WarpCell<4>& c, const float4* plane,
   unsigned V = c.vm[0];
   float r2 = c.r2;
   int nt = c.nt, pi = 4;
+  unsigned tested = 1u + ((unsigned)nt << 16);  // a plane's share of the counters
   float4 P = building ? plane[pi] : none;
   for (;;) {
     // the next plane that cuts, for every group
@@ -807,19 +808,17 @@ __device__ __forceinline__ void build_cells(WarpCell<4>& c, const float4* plane,
       const bool miss = building && M == 0u;
       if (!__any_sync(FULL, miss)) break;
       if (miss) {
-        seq_cnt += 1u + ((unsigned)nt << 16);
         // |neighbour - site|^2 > 4 max|v - site|^2
-        if (2.f * P.w > 4.f * r2) {
-          secmiss = false;
-          building = false;
-        } else if (++pi == pend) {
-          building = false;
-        }
-        P = building ? plane[pi] : none;
+        const bool secure = P.w > 2.f * r2;
+        secmiss = secmiss && !secure;
+        building = !secure && pi + 1 < pend;
+        seq_cnt += tested;
+        pi += building;
+        P = plane[pi];
       }
     }
     if (!__any_sync(FULL, building)) break;
-    if (building) seq_cnt += 1u + ((unsigned)nt << 16);
+    if (building) seq_cnt += tested;
     if (building && M == V) {  // nothing left
       state = 1;
       building = false;
@@ -838,83 +837,50 @@ __device__ __forceinline__ void build_cells(WarpCell<4>& c, const float4* plane,
     const int E = 3 * R;
     const int E0 = __shfl_sync(FULL, E, 0), E1 = __shfl_sync(FULL, E, 8), E2 = __shfl_sync(FULL, E, 16),
               E3 = __shfl_sync(FULL, E, 24);
-    const int npass = E0 + E1 + E2 + E3 <= WARP ? 1 : (E0 + E1 <= WARP && E2 + E3 <= WARP) ? 2 : 0;
-    int nb = 0;
-    bool bad = false;
-    if (npass > 0) {
-      const bool large = __any_sync(FULL, R > 3);
-      for (int pass = 0; pass < npass; ++pass) {
-        // the edges of this pass's groups as one run over the warp
-        const bool lo = npass == 1 || pass == 0, hi = npass == 1 || pass == 1;
-        const int c1 = lo ? E0 : 0, c2 = c1 + (lo ? E1 : 0), c3 = c2 + (hi ? E2 : 0), tot = c3 + (hi ? E3 : 0);
-        const int gi = lane >= c3 ? 3 : lane >= c2 ? 2 : lane >= c1 ? 1 : 0;
-        const int go = lane >= c3 ? c3 : lane >= c2 ? c2 : lane >= c1 ? c1 : 0;
-        const int mine = gid == 3 ? c3 : gid == 2 ? c2 : gid == 1 ? c1 : 0;
-        const bool has_e = lane < tot;
-        const int shift = (gi - gid) * gstride;
-        unsigned dir = 0u, key = 0x80000000u | (unsigned)lane;
-        if (has_e) {
-          const int e = lane - go, tr = (e * 11) >> 5, es = e - 3 * tr;
-          const unsigned T = conf[shift + tr];
-          dir = __byte_perm(T, 0u, es == 0 ? 0x4410 : es == 1 ? 0x4421 : 0x4402);  // ea | eb << 8
-          const unsigned ea = dir & 0xffu, eb = dir >> 8;
-          key = ((unsigned)gi << 16) | min(ea, eb) | (max(ea, eb) << 8);
-        }
-        const unsigned same = __match_any_sync(FULL, key);
-        const bool isb = has_e && __popc(same) == 1;
-        const unsigned bm = __ballot_sync(FULL, isb);
-        if (isb) bedge[shift + __popc(bm & ((1u << lane) - 1u) & ~((1u << go) - 1u))] = dir;
-        const bool in = gid < 2 ? lo : hi;
-        const unsigned gmask = in && E > 0 ? (E >= WARP ? FULL : ((1u << E) - 1u) << mine) : 0u;
-        if (in) nb = __popc(bm & gmask);
-        if (large) {
-          // each boundary vertex starts exactly one edge
-          const unsigned skey = isb ? (((unsigned)gi << 16) | (dir & 0xffu)) : (0x80000000u | (unsigned)lane);
-          const unsigned starts = __match_any_sync(FULL, skey);
-          const bool dup = isb && __popc(starts) != 1;
-          bad |= (__ballot_sync(FULL, dup) & gmask) != 0u;
-        }
+    // as many groups at a time as have 32 edges between them (a cavity of more
+    // than ten triangles, which no lane is left for, is dropped: the one-warp
+    // pass builds that cell)
+    const bool large = __any_sync(FULL, R > 3);
+    const int end1 = E0, end2 = E0 + E1, end3 = end2 + E2, end4 = end3 + E3;
+    int nb = 0, from = 0;
+    bool bad = E > WARP;
+#pragma unroll 1
+    while (from < end4) {
+      // the edges [from, to) of the warp's run, whole groups
+      const int to = end4 - from <= WARP ? end4
+                     : end3 > from && end3 - from <= WARP ? end3
+                     : end2 > from && end2 - from <= WARP ? end2
+                     : end1 > from && end1 - from <= WARP ? end1
+                     : end1 > from ? end1 : end2 > from ? end2 : end3 > from ? end3 : end4;
+      const int at = from + lane;  // this lane's edge
+      const int gi = at >= end3 ? 3 : at >= end2 ? 2 : at >= end1 ? 1 : 0;
+      const int go = (at >= end3 ? end3 : at >= end2 ? end2 : at >= end1 ? end1 : 0) - from;
+      const int mine = (gid == 3 ? end3 : gid == 2 ? end2 : gid == 1 ? end1 : 0) - from;
+      const bool has_e = at < to;
+      const int shift = (gi - gid) * gstride;
+      unsigned dir = 0u, key = 0x80000000u | (unsigned)lane;
+      if (has_e) {
+        const int e = lane - go, tr = (e * 11) >> 5, es = e - 3 * tr;
+        const unsigned T = conf[shift + tr];
+        dir = __byte_perm(T, 0u, es == 0 ? 0x4410 : es == 1 ? 0x4421 : 0x4402);  // ea | eb << 8
+        const unsigned ea = dir & 0xffu, eb = dir >> 8;
+        key = ((unsigned)gi << 16) | min(ea, eb) | (max(ea, eb) << 8);
       }
-    } else {
-      // more edges than that: each group searches its removed triangles, 8
-      // edges at a time
-      const int Emax = (int)__reduce_max_sync(FULL, (unsigned)E);
-      for (int e0 = 0; e0 < Emax; e0 += G) {
-        const int e = e0 + gl;
-        bool isb = false;
-        unsigned dir = 0u;
-        if (e < E) {
-          const unsigned T = conf[e / 3];
-          const int es = e % 3;
-          dir = __byte_perm(T, 0u, es == 0 ? 0x4410 : es == 1 ? 0x4421 : 0x4402);
-          const unsigned tw = __byte_perm(dir, 0u, 0x4401);
-          bool twin = false;
-          for (int q = 0; q < R; ++q) {
-            const unsigned U = conf[q];
-            twin |= ((U & 0xffffu) == tw) | (((U >> 8) & 0xffffu) == tw) | (__byte_perm(U, 0u, 0x4402u) == tw);
-          }
-          isb = !twin;
-        }
-        const unsigned bm = (__ballot_sync(FULL, isb) >> gbase) & 0xffu;
-        if (isb) {
-          const int r = nb + __popc(bm & ((1u << gl) - 1u));
-          if (r < CAP) bedge[r] = dir;
-        }
-        nb += __popc(bm);
+      const unsigned same = __match_any_sync(FULL, key);
+      const bool isb = has_e && __popc(same) == 1;
+      const unsigned bm = __ballot_sync(FULL, isb);
+      if (isb) bedge[shift + __popc(bm & ((1u << lane) - 1u) & ~((1u << max(go, 0)) - 1u))] = dir;
+      const bool in = E > 0 && E <= WARP && mine >= 0 && mine + E <= to - from;
+      const unsigned gmask = in ? ((1u << E) - 1u) << mine : 0u;
+      if (in) nb = __popc(bm & gmask);
+      if (large) {
+        // each boundary vertex starts exactly one edge
+        const unsigned skey = isb ? (((unsigned)gi << 16) | (dir & 0xffu)) : (0x80000000u | (unsigned)lane);
+        const unsigned starts = __match_any_sync(FULL, skey);
+        const bool dup = isb && __popc(starts) != 1;
+        bad |= (__ballot_sync(FULL, dup) & gmask) != 0u;
       }
-      __syncwarp();
-      const int nbc = (building && R > 3 && nb <= CAP) ? nb : 0;
-      const int NBmax = (int)__reduce_max_sync(FULL, (unsigned)nbc);
-      for (int e0 = 0; e0 < NBmax; e0 += G) {
-        const int e = e0 + gl;
-        if (e < nbc) {
-          const unsigned a = bedge[e] & 0xffu;
-          int starts = 0;
-          for (int q = 0; q < nbc; ++q) starts += (bedge[q] & 0xffu) == a;
-          bad |= starts != 1;
-        }
-      }
-      bad = ((__ballot_sync(FULL, bad) >> gbase) & 0xffu) != 0u;
+      from = to;
     }
     if (R <= 3) bad = !cavity_disk_small(R, nb);
     const int nt2 = nt - R + nb;
@@ -973,6 +939,7 @@ __device__ __forceinline__ void build_cells(WarpCell<4>& c, const float4* plane,
     if (building) {
       V = keep | N;
       nt = nt2;
+      tested = 1u + ((unsigned)nt << 16);
       r2 = lm;
       seq_cnt += 1u << 8;
       if (gl == 0) *nnew += (unsigned)nb;
@@ -980,14 +947,14 @@ __device__ __forceinline__ void build_cells(WarpCell<4>& c, const float4* plane,
         // (nearly) parallel planes: the conflict decisions were inconsistent
         state = 2;
         building = false;
-      } else if (2.f * P.w > 4.f * r2) {
-        secmiss = false;
-        building = false;
-      } else if (++pi == pend) {
-        building = false;
+      } else {
+        const bool secure = P.w > 2.f * r2;
+        secmiss = secmiss && !secure;
+        building = !secure && pi + 1 < pend;
+        pi += building;
+        P = plane[pi];
       }
     }
-    P = building ? plane[pi] : none;
   }
 #pragma unroll
   for (int k = 0; k < SL; ++k) c.vm[k] = (V >> (8 * k)) & 0xffu;
