@@ -49,9 +49,12 @@ static_assert(MESH_EDGES == 3 * MESH_VERTS / 2 && MESH_FACES == MESH_VERTS / 2 +
 constexpr int MESH_TETS = 16;  // tets in hand
 constexpr int MESH_IDS = 4 + MAX_SITE_K + 12 + MESH_EXT;  // plane ids a stored cell may use
 constexpr int MESH_ID_WORDS = (MESH_IDS + 31) / 32;
-// A cell whose terms from the site exceed this many times their sum is done
-// again from a point of what is left of it (sites outside the mesh).
-constexpr float MESH_APEX_RATIO = 32.f;
+// A cell whose terms exceed this many times their sum keeps a sliver of
+// itself in the mesh (one in a thousand of the boundary cells of random sites,
+// the site mostly outside): the terms' rounding, 1e-7 of a cell, would show in
+// it, so the 128-vertex pass clips it by each tet.  A completed cell, which
+// no pass follows, is summed again from a point of the sliver.
+constexpr float MESH_APEX_RATIO = 64.f;
 // A sum below this fraction of its terms (rounded to 1e-7 of them each) is
 // rounding: the cell only touches the mesh, and its site stays where it is.
 constexpr float MESH_NOISE = 1e-6f;
@@ -307,7 +310,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
 
     // -----------------------------------------------------------------
     // the tets.  When the first apex (the site) turns out far from what is left
-    // of the cell: again for a mean of its points (lengths of its edges and
+    // of a completed cell: again for a mean of its points (lengths of its edges and
     // moments of them in place of their terms), and then from that point
     float3 X = make_float3(0.f, 0.f, 0.f);
     float pr2 = 0.f, vol = 0.f, mx = 0.f, my = 0.f, mz = 0.f, v6 = 0.f, mag = 0.f;
@@ -705,19 +708,14 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
       mz = __fmaf_rn(z24, 1.f / 24.f, __fmul_rn(vol, X.z));
       // large terms for a small sum: the apex is far from what is left
       if (mag <= MESH_APEX_RATIO * v6 || mag == 0.f) break;
+      if (out_list) bad = true;
     }
     // a sum within its terms' rounding is none (a tet that only touches)
     if (!(v6 > MESH_NOISE * mag)) vol = mx = my = mz = v6 == v6 ? 0.f : v6;
-    if (REF && lane == 0) {
-      const unsigned nc = (unsigned)(site_start[s + 1] - site_start[s]);
-      S.cnt[WC_CAND] += nc;
-      S.cnt[WC_CLIPPED] += min((unsigned)nclip, nc);
-      S.cnt[WC_CULLED] += nc - min((unsigned)nclip, nc);
-    }
     bad |= !(isfinite(vol) && isfinite(mx) && isfinite(my) && isfinite(mz));
     if (bad) {
-      // degenerate: the 128-vertex pass clips a copy of the cell by each tet
-      // (a completed cell keeps its earlier moments)
+      // degenerate, or a sliver: the 128-vertex pass clips a copy of the cell by
+      // each tet (a completed cell keeps its earlier moments)
       if (lane == 0) {
         if (out_list) {
           out_list[atomicAdd(out_count, 1)] = s;
@@ -731,6 +729,12 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
       }
       __syncwarp();
       continue;
+    }
+    if (REF && lane == 0) {
+      const unsigned nc = (unsigned)(site_start[s + 1] - site_start[s]);
+      S.cnt[WC_CAND] += nc;
+      S.cnt[WC_CLIPPED] += min((unsigned)nclip, nc);
+      S.cnt[WC_CULLED] += nc - min((unsigned)nclip, nc);
     }
     if (lane == 0) {
       unsigned f = flags | SITE_HANDED;

@@ -62,7 +62,8 @@ enum vgb_stat {
   VGB_STAT_CULL_TESTS = 12,     /* tet-vs-plane tests of the separation pass          */
   VGB_STAT_NEW_VERTICES = 13,   /* vertices created by clipping                       */
   VGB_STAT_INTERIOR = 14,       /* sites whose whole cell lies inside the mesh        */
-  VGB_STAT_REDO = 15,           /* sites redone at 128 vertices (outgrew 64)          */
+  VGB_STAT_REDO = 15,           /* sites redone at 128 vertices (outgrew 64, or left a
+                                   sliver to the mesh pass)                           */
   VGB_STAT_NEEDS_EXACT = 16,    /* robust_predicates: vertex-vs-plane tests decided by
                                    the exact determinants (the reference's status
                                    needs_exact_predicates, voronoi_defs.h:10)          */
