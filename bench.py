@@ -98,22 +98,32 @@ WORKLOADS = {
 DEFAULT_WORKLOAD = "torus128_uniform_1m"
 # kernels per Lloyd iteration besides the grid sort: exact form -- position
 # map, kNN (first tier), tet reach, first clip pass, kNN of the listed sites
-# (K > 32 only), one-warp, 128-vertex and completion clip passes, update;
-# reference cell-tet form -- position map, site kNN, centroid kNN, candidate
-# count, scan (3), fill, the two clip passes, update; tet-cell: one clip
-# pass; plain: the thread-per-pair clip and its update
-LAUNCHES_PER_STEP = {"exact": 9, "cell_tet": 11, "site_major": 10, "plain": 5}
+# (K > 32 only), one-warp pass, mesh pass, 128-vertex pass, completion (64 and
+# 256 vertices), the completed cells' mesh pass, update; reference forms
+# (cell-tet, tet-cell) -- position map, site kNN, centroid kNN, last
+# candidates, candidate count, fill (and their scan, below), first pass,
+# one-warp, mesh and 128-vertex passes, update; plain: the thread-per-pair clip
+# and its update
+LAUNCHES_PER_STEP = {"exact": 12, "cell_tet": 11, "site_major": 11, "plain": 5}
 
 
-def grid_sort_launches(ncell: int) -> int:
-    """Gather + cell-count scan (3), then per 8-bit digit of the cell key a
-    histogram, a scan (3) and a scatter."""
+def scan_launches(n: int) -> int:
+    """One block up to 32,768 values, three launches above."""
+    return 1 if n <= 32768 else 3
+
+
+def grid_sort_launches(n: int, ncell: int) -> int:
+    """Gather and cell-count scan, then up to 65,536 sites the placement and the
+    ranks, above that per 8-bit digit of the cell key a histogram, a scan (3)
+    and a scatter."""
+    if n <= 65536:
+        return 3 + scan_launches(ncell + 1)
     passes = 0
     top = max(ncell - 1, 0)
     while top > 0:
         passes += 1
         top >>= 8
-    return 4 + 5 * passes
+    return 1 + scan_launches(ncell + 1) + 5 * passes
 
 # algorithmic FP32 work of the clip phase, per event its kernels count
 FLOPS_CONFLICT = 7      # plane test of one cell vertex: 3 FMA + compare
@@ -209,12 +219,13 @@ def measured_peaks():
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) per launch of
 # the rooflined kernels on the default workload, from one-pass ncu captures
-# of one launch each: the clip phase's two large kernels (first pass
-# 253.5 MB, one-warp pass 502.1 MB) and the first kNN tier (93.1 MB).
+# of one launch each on relaxed sites: the clip phase's three large kernels
+# (first pass 222.4 MB, one-warp pass 66.7 MB, mesh pass 111.1 MB) and the
+# first kNN tier (90.2 MB).
 TRAFFIC = {
-    ("clip", "torus128_uniform_1m"): (755_616_512, "ncu one-pass capture, k_build<0,8,4,0> + "
-                                                  "k_clip_site<1,0,2,0,0>, one launch each"),
-    ("knn", "torus128_uniform_1m"): (93_052_672, "ncu one-pass capture, k_knn<1,0,8>, one launch"),
+    ("clip", "torus128_uniform_1m"): (400_200_000, "ncu one-pass capture, k_build<0,8,4,0> + "
+                                                  "k_clip_site<1,0,2,0,0,1> + k_cell_mesh<0,0>, one launch each"),
+    ("knn", "torus128_uniform_1m"): (90_200_000, "ncu one-pass capture, k_knn<1,0,8>, one launch"),
 }
 
 
@@ -429,10 +440,12 @@ def run_ours(args):
     clip_flops = (FLOPS_CONFLICT * stats["conflict_tests"] + FLOPS_CULL * stats["cull_tests"] +
                   FLOPS_NEW_VERTEX * stats["new_vertices"] + FLOPS_FINAL_VERTEX * stats["final_vertices"])
     clip_tf = clip_flops / (phases["clip"] / 1e3) / 1e12
-    # the clip phase: the exact form runs the lane-group first pass (k_build),
-    # the one-warp pass over the sites it hands on and the 128-vertex pass
-    kname = ("k_build + k_clip_site<cell_tet> x2 (clip phase)" if exact else
-             {"cell_tet": "k_clip_site<cell_tet> x2 (clip phase)", "site_major": "k_clip_site<tet_cell>",
+    # the clip phase: the lane-group first pass (k_build), the one-warp pass
+    # over the sites it hands on, the mesh pass and the passes for large and
+    # open cells
+    kname = ("k_build + k_clip_site + k_cell_mesh (clip phase)" if exact else
+             {"cell_tet": "k_build + k_clip_site + k_cell_mesh (clip phase)",
+              "site_major": "k_build + k_clip_site + k_cell_mesh (clip phase)",
               "plain": "k_clip_plain"}[args.method])
     tr_clip = TRAFFIC.get(("clip", args.workload)) if exact else None
     roofline = {"kernel": kname,
@@ -515,7 +528,8 @@ def run_ours(args):
                                              "no flush",
                    "parallelism": f"replicas x{world}"},
         "gpu_launches": (LAUNCHES_PER_STEP["exact" if exact else args.method] - (1 if exact and K <= 32 else 0) +
-                         grid_sort_launches(grid_dim ** 3)) * args.steps,
+                         grid_sort_launches(n, grid_dim ** 3) +
+                         (0 if exact or args.method == "plain" else scan_launches(n + 1))) * args.steps,
         "e2e": e2e,
         "roofline": roofline,
         "roofline_knn": roofline_knn,
@@ -729,7 +743,7 @@ def run_batch(args):
                    "grid_density": round(dens, 2), "form": "exact, batched (one launch per kernel per iteration)",
                    "cuda_graph": True, "create_s": round(create_s, 2), "l2": "inputs larger than L2, no flush",
                    "parallelism": f"replicas x{world}"},
-        "gpu_launches": (LAUNCHES_PER_STEP["exact"] + grid_sort_launches(n_cells)) * args.steps,
+        "gpu_launches": (LAUNCHES_PER_STEP["exact"] + grid_sort_launches(B.n_site, n_cells)) * args.steps,
         "e2e": None,
         "sites_per_s": round(n_site * value / world, 1),
         "stats": stats,
