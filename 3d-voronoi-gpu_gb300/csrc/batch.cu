@@ -349,7 +349,7 @@ int vgb_batch_create(vgb_batch** out, const vgb_config* cfg_in, int n_prob, cons
       (rc = balloc(&b->cell_fill, cell_cap)) || (rc = balloc(&b->site_cell, grid_sort_work_ints(b->n, cell_cap))) ||
       (rc = balloc(&b->scan_tmp, scan_tmp_ints((long long)scan_n))) || (rc = balloc(&b->pos_of_id, b->n)) ||
       (rc = balloc(&b->tet_order, b->n_tet)) || (rc = balloc(&b->tet_cell_start, cell_cap + 1)) ||
-      (rc = balloc(&b->tcell, b->n_tet)) || (rc = balloc(&b->knn, knn_cap)) || (rc = balloc(&b->mom, b->n)) ||
+      (rc = balloc(&b->tcell, 2 * (size_t)b->n_tet)) || (rc = balloc(&b->knn, knn_cap)) || (rc = balloc(&b->mom, b->n)) ||
       (rc = balloc(&b->stats, VGB_STAT_COUNT)) || (rc = balloc(&b->field, f_off)) ||
       (rc = balloc(&b->field_sat, q_off)) || (rc = balloc(&b->reach, b->n_tet)) ||
       (rc = balloc(&b->tet_sph, b->n_tet)) || (rc = balloc(&b->reach_max, n_prob)) ||

@@ -517,7 +517,7 @@ int vgb_engine_create(vgb_engine** out, const vgb_config* cfg_in, const float* v
   if (ce == cudaSuccess) {
     // tets by centroid cell, once per mesh and grid
     int* tcell = nullptr;
-    if (dalloc(&tcell, n_tet) != VGB_OK) { free_engine(e); return VGB_ERR_NOMEM; }
+    if (dalloc(&tcell, 2 * (size_t)n_tet) != VGB_OK) { free_engine(e); return VGB_ERR_NOMEM; }
     if (tets_by_cell(e->verts, e->tets, n_tet, e->ncell, nullptr, nullptr, e->prob, e->tet_cell_start, e->cell_fill,
                      tcell, e->tet_order,
                      e->scan_tmp, e->st)) {

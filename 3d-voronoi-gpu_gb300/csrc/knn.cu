@@ -915,22 +915,26 @@ __global__ void k_tet_scatter(const int* __restrict__ tcell, int n_tet, const in
   order[start[c] + atomicAdd(fill + c, 1)] = t;
 }
 
-// Tets of each cell in id order (insertion sort; a few dozen per cell), so
-// the order in which a cell's pieces are summed does not depend on the
-// scatter's atomics.
-__global__ void k_tet_cell_order(int* __restrict__ order, const int* __restrict__ start, long long ncell) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncell) return;
+// Tets of each cell in id order, so the order in which a cell's pieces are
+// summed does not depend on the scatter's atomics: each by its rank among the
+// members (the lanes of a warp mostly share a cell and read the same words).
+// One thread sorting each cell by insertion, as before, moved words as often
+// as this compares them, in one serial chain a cell: a reference-form engine
+// of 1,293 sites in 64,848 tets (a thousand tets a cell) was made in 27.9 ms,
+// now 0.9; 3,000 sites in 245k tets 114 ms, now 1.6; 162k tets in one cell
+// 87 s, now 6 ms.  One compare per pair of tets of a cell remains: an engine
+// with 1M tets in one cell is made in 0.15 s.
+__global__ void k_tet_rank(const int* __restrict__ member, const int* __restrict__ tcell, int n_tet,
+                           const int* __restrict__ start, int* __restrict__ order) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n_tet) return;
+  const int t = member[p];
+  const int c = tcell[t];
   const int b = start[c], e = start[c + 1];
-  for (int i = b + 1; i < e; ++i) {
-    const int x = order[i];
-    int j = i - 1;
-    while (j >= b && order[j] > x) {
-      order[j + 1] = order[j];
-      --j;
-    }
-    order[j + 1] = x;
-  }
+  int r = 0;
+#pragma unroll 8
+  for (int q = b; q < e; ++q) r += member[q] < t;
+  order[b + r] = t;
 }
 
 // Bounding sphere (centroid, largest corner distance) of each tet, in
@@ -1169,8 +1173,9 @@ int tets_by_cell(const float4* verts, const int4* tets, int n_tet, long long nce
   k_tet_cells<<<(n_tet + 255) / 256, 256, 0, st>>>(verts, tets, n_tet, probs, tet_prob, lone, tet_cell_start, tcell);
   VGB_CUDA_TRY(cudaGetLastError());
   if (scan_exclusive(tet_cell_start, tet_cell_start, nc + 1, scan_tmp, st)) return -2;
-  k_tet_scatter<<<(n_tet + 255) / 256, 256, 0, st>>>(tcell, n_tet, tet_cell_start, cell_fill, tet_order);
-  k_tet_cell_order<<<(unsigned)((nc + 255) / 256), 256, 0, st>>>(tet_order, tet_cell_start, nc);
+  int* const member = tcell + n_tet;
+  k_tet_scatter<<<(n_tet + 255) / 256, 256, 0, st>>>(tcell, n_tet, tet_cell_start, cell_fill, member);
+  k_tet_rank<<<(n_tet + 255) / 256, 256, 0, st>>>(member, tcell, n_tet, tet_cell_start, tet_order);
   VGB_CUDA_TRY(cudaGetLastError());
   return 0;
 }

@@ -246,7 +246,7 @@ int last_candidates(const float4* sites, const float4* tet_sph, const int* tet_o
                     int tk, float2* last, unsigned* reach_max_bits, cudaStream_t st);
 // Tets sorted by the grid cell of their float32 centroid in their problem's
 // grid (once per mesh): tet_cell_start ncell + 1 ints, cell_fill ncell
-// scratch, tcell n_tet scratch, tet_order n_tet ints.
+// scratch, tcell 2 n_tet scratch, tet_order n_tet ints.
 int tets_by_cell(const float4* verts, const int4* tets, int n_tet, long long ncell, const ProbDesc* probs,
                  const int* tet_prob, const ProbDesc& lone, int* tet_cell_start, int* cell_fill, int* tcell,
                  int* tet_order, int* scan_tmp, cudaStream_t st);
@@ -309,9 +309,10 @@ constexpr int MESH_VERTS = 64;
 constexpr int MESH_EXT = PIECE_REC;
 
 // Whether a problem (or batch) runs the mesh pass (clip_mesh.cuh): the exact
-// form and the reference forms do, with float predicates.  It is faster than clipping by each tet
-// at every size and mesh measured (Lloyd iteration, us: 20k sites in 48k tets
-// 610 -> 290, 100k in 6 tets 1,955 -> 1,020, 1M in 1.96M 10,100 -> 7,400); the
+// form and the reference forms do, with float predicates.  It is faster than
+// clipping by each tet at every size and mesh measured (Lloyd iteration with
+// nothing else changed, us: 20k sites in 48k tets 610 -> 290, 100k in 6 tets
+// 1,955 -> 1,020, 1M in 1.96M 10,100 -> 7,400); the
 // pieces pass is left to callers who ask for it on a mesh of fewer than a tet
 // per 256 sites, where its pieces outgrow their lane groups and the counters
 // say so (3,000 sites in 6 tets: 350 us, with the mesh pass 280).
