@@ -770,13 +770,14 @@ __device__ __forceinline__ int group_clip(WarpCell<SL>& c, const float4 P, const
 //     of them do not; a group that has one waits);
 //   * the groups cut together: boundary edges by match_any as in group_clip,
 //     in turns when the four cavities have more than 32 edges (one round in
-//     three; a group that has ended tests on, unheard); then one new vertex per lane, kept in shared memory, and each
-//     freed slot takes its own.  (Each slot computing its own vertex runs the
-//     vertex code once per slot a cavity has freed, for one or two lanes at a
-//     time.)
-// Bound by the ALU pipe and issue (73% and 74% busy).  The first pass with it
-// against the loop of group_clip calls: 1M random torus sites 5.02 -> 3.98 ms,
-// relaxed 3.85 -> 3.45; 20k sites 145 -> 124 us.  conf and bedge: the group's
+//     three; a group that has ended tests on, unheard); then one new vertex
+//     per lane, kept in shared memory, and each freed slot takes its own.
+//     (Each slot computing its own vertex runs the vertex code once per slot
+//     a cavity has freed, for one or two lanes at a time.)
+// Bound by instruction issue (78% of cycles; the ALU pipe 65% busy).  The
+// first pass with it against the loop of group_clip calls: 1M random torus
+// sites 5.02 -> 3.75 ms, relaxed 3.85 -> 3.17; with the edges in turns as
+// well, the clip phase of 1M relaxed sites 5.07 -> 4.92.  conf and bedge: the group's
 // 32-entry scratch arrays (conf 16-byte aligned), gstride words after the
 // previous group's.
 __device__ __forceinline__ void build_cells(WarpCell<4>& c, const float4* plane, unsigned* conf, unsigned* bedge,

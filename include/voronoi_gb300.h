@@ -139,7 +139,8 @@ typedef struct vgb_config {
   int autotune; /* exact cell-tet form.  1: at creation, time the launch shapes and
                    keep the fastest -- warps per kNN block (4 or 8), lanes per site in
                    the first clip pass (8 or 16), vertices per cell in the one-warp
-                   clip pass (64 or 96) -- and the clip form (tet_pieces); results do
+                   clip pass (64 or 96) -- and the clip form (tet_pieces); the last
+                   two only where cells are clipped by each tet.  Results do
                    not depend on them beyond float rounding.  The choices are timed
                    on the sites after two Lloyd steps (the initial sites are put
                    back).  0: the defaults (8, 8, 64, the configured clip form).  The
@@ -264,7 +265,7 @@ int vgb_clipped_voro_diagram(const float* vertices, int n_vert, const int* indic
  * d_knn (n x k) holds the k nearest points of each point in grid order, as
  * grid positions, and d_perm (n) maps grid position -> input index.  All
  * pointers are device memory owned by the caller; d_points is n x 3 floats.
- * Intermediate arrays live in one static device array of about 2.9 MB, held
+ * Intermediate arrays live in one static device array of about 3.7 MB, held
  * by every GPU that loads the library until the process exits, so n is at
  * most VGB_NOALLOC_MAX_POINTS (larger n returns VGB_ERR_INVALID) and
  * 1 <= k <= 128, k < n.  Work is queued on `stream` (a cudaStream_t, NULL for
