@@ -87,6 +87,13 @@ constexpr int BOX_PLANES = 6;
 #ifndef VGB_BUILD_MIN_BLOCKS
 #define VGB_BUILD_MIN_BLOCKS 7
 #endif
+// The robust kernels at 6 (80 registers): at 8 they spill 200-400 B a thread
+// (the pairs of floats of a vertex), at 5 they spill next to nothing but hold
+// fewer warps.  Two robust steps, ms, at the float kernels' 7 and 8 / at 6:
+// 1,500 sites 1.12 / 1.10, 20k 3.61 / 3.40, 125k 16.5 / 15.7, 1M 102.4 / 96.0.
+#ifndef VGB_ROBUST_MIN_BLOCKS
+#define VGB_ROBUST_MIN_BLOCKS 6
+#endif
 #ifndef VGB_BUILD_MIN_BLOCKS_BATCHED
 #define VGB_BUILD_MIN_BLOCKS_BATCHED 7
 #endif
@@ -268,7 +275,7 @@ __device__ __forceinline__ void store_master(const WarpCell<SL>& c, SiteSmem<SL,
 // MESH (exact form, float): a cell that is not inside the mesh goes to the
 // mesh pass (clip_mesh.cuh) instead of being clipped by each tet.
 template <bool CELL_TET, bool BATCHED, int SL, bool ROBUST, bool COMPLETE = false, bool MESH = false>
-__global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : SL >= 4 || COMPLETE ? 6 : VGB_CLIP_MIN_BLOCKS) k_clip_site(
+__global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_ROBUST_MIN_BLOCKS : SL >= 4 || COMPLETE ? 6 : VGB_CLIP_MIN_BLOCKS) k_clip_site(
     const float4* __restrict__ sites, int n, const unsigned* __restrict__ knn, const ProbDesc* __restrict__ probs,
     const int* __restrict__ site_prob, const ProbDesc lone, const float4* __restrict__ verts,
     const int4* __restrict__ tets, const int* __restrict__ site_start, const int* __restrict__ site_tets,
@@ -1093,7 +1100,7 @@ struct PieceSmem {
 };
 
 template <bool BATCHED, bool ROBUST>
-__global__ void __launch_bounds__(CLIP_WARPS * WARP, VGB_PIECE_MIN_BLOCKS) k_clip_pieces(
+__global__ void __launch_bounds__(CLIP_WARPS * WARP, ROBUST ? VGB_ROBUST_MIN_BLOCKS : VGB_PIECE_MIN_BLOCKS) k_clip_pieces(
     const float4* __restrict__ sites, const unsigned* __restrict__ knn, const ProbDesc* __restrict__ probs,
     const int* __restrict__ site_prob, const ProbDesc lone, const float4* __restrict__ verts,
     const int4* __restrict__ tets, const int* __restrict__ site_start, const int* __restrict__ site_tets,
@@ -1465,7 +1472,7 @@ __host__ __device__ constexpr int build_plane_stride(int kmax) { return 4 + kmax
 // counter independently; a warp's groups run one instruction stream, a
 // group whose cell is done passing its turn in each clip.
 template <bool BATCHED, int G, int SL, bool ROBUST>
-__global__ void __launch_bounds__(CLIP_WARPS * WARP, BATCHED ? VGB_BUILD_MIN_BLOCKS_BATCHED : VGB_BUILD_MIN_BLOCKS) k_build(
+__global__ void __launch_bounds__(CLIP_WARPS * WARP, ROBUST ? VGB_ROBUST_MIN_BLOCKS : BATCHED ? VGB_BUILD_MIN_BLOCKS_BATCHED : VGB_BUILD_MIN_BLOCKS) k_build(
     const float4* __restrict__ sites, int n, const unsigned* __restrict__ knn, const ProbDesc* __restrict__ probs,
     const int* __restrict__ site_prob, const ProbDesc lone, dmom4* __restrict__ mom,
     unsigned long long* __restrict__ stats, const unsigned char* __restrict__ field,
