@@ -27,7 +27,10 @@
 //     cell (stored, resumed, or built), its bound by the domain box when its
 //     security radius was missed, then the candidate tets;
 //   * k_clip_site with 4 slots (128 vertices) over the sites whose cell
-//     outgrew 64.
+//     outgrew 64 or which the mesh pass gives back;
+//   * the completion of the cells that the K neighbours leave open: k_clip_site
+//     again at 64 vertices, k_cell_mesh over what it finishes, and 8 slots (256
+//     vertices) over the rest, clipped by each tet.
 //   The tet-cell method is k_clip_site with 3 slots (96 vertices, the
 //   reference's triangle capacity).  Within a warp or group:
 //   * the K bisector planes of the site are computed once, in coordinates
@@ -272,8 +275,10 @@ __device__ __forceinline__ void store_master(const WarpCell<SL>& c, SiteSmem<SL,
 // and the completion pass (COMPLETE) clips its cell by every site within
 // twice that radius beyond its K nearest before it clips the tets again.
 //
-// MESH (exact form, float): a cell that is not inside the mesh goes to the
-// mesh pass (clip_mesh.cuh) instead of being clipped by each tet.
+// MESH (exact form, float): a cell of at most 64 vertices that is not inside
+// the mesh goes to the mesh pass (clip_mesh.cuh) instead of being clipped by
+// each tet; the last completion pass (256 vertices) takes what that one and
+// the mesh pass leave and clips it by each tet.
 template <bool CELL_TET, bool BATCHED, int SL, bool ROBUST, bool COMPLETE = false, bool MESH = false>
 __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_ROBUST_MIN_BLOCKS : SL >= 4 || COMPLETE ? 6 : VGB_CLIP_MIN_BLOCKS) k_clip_site(
     const float4* __restrict__ sites, int n, const unsigned* __restrict__ knn, const ProbDesc* __restrict__ probs,
@@ -286,8 +291,7 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
     const int* __restrict__ in_list, const int* __restrict__ in_count, int* __restrict__ out_list,
     int* __restrict__ out_count, int* __restrict__ work, const CellStore store, int k_tier,
     const int* __restrict__ cell_start, int* __restrict__ esc_list, float* __restrict__ esc_r2,
-    int* __restrict__ esc_count, int* __restrict__ piece_list, int* __restrict__ piece_count,
-    float* __restrict__ out_r2) {
+    int* __restrict__ esc_count, int* __restrict__ piece_list, int* __restrict__ piece_count) {
   constexpr int NPLANE = COMPLETE ? COMPLETE_PLANES : SITE_PLANES;
   constexpr int PWORDS = (NPLANE + 31) / 32;
   __shared__ SiteSmem<SL, NPLANE> smem_all[CLIP_WARPS];
@@ -305,7 +309,10 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
   // take the next item from it in a single wave of resident blocks, so a warp
   // that drew cheap sites takes more; without, items are dealt round-robin.
   const int n_items = in_list ? *in_count : n;
+  // (COMPLETE with MESH: the site again, without its completion)
+  bool again = false;
   auto next_item = [&](int cur) {
+    if (COMPLETE && MESH && again) return cur;
     if (work) {
       int v = 0;
       if (lane == 0) v = atomicAdd(work, 1);
@@ -317,6 +324,9 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
     const int s = in_list ? in_list[it] : it;
     bool abandon = false;
     bool emitted = false;  // handed to the pieces pass
+    bool lost = false;     // completion pass: a piece of the cell failed
+    // completing the cell (not so once its pieces proved to be lost, see below)
+    const bool completing = COMPLETE && !again;
     // the cell the first pass built, when it stored one
     if (lane == 0) S.stored = (CELL_TET && store.nt) ? store.nt[s] : 0;
     __syncwarp();
@@ -351,7 +361,7 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
     // outcome bits of the site (cell-tet method): this pass built its cell
     if (lane == 0) {
       S.site_flags = SITE_HANDED | (SL > 2 ? SITE_REDO : 0);
-      S.pr2 = COMPLETE ? esc_r2[it] : 0.f;
+      S.pr2 = completing ? esc_r2[s] : 0.f;
       S.unchanged = 0;
       S.Rc = 0.f;
       S.nfaces = 0;
@@ -633,7 +643,18 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
       if (abandon) break;
       if (job == 2 && bis && state == 0 && secmiss && lane == 0) S.cnt[WC_SECMISS]++;
       // the completion pass keeps the earlier moments of a site that loses a piece
-      if (COMPLETE && job == 2 && state == 2 && lane == 0) S.site_flags |= SITE_UNRESOLVED;
+      // (MESH: those are no sum of pieces -- a mesh pass that skips the tets out
+      // of reach has their faces missing -- so the larger pass takes the site,
+      // and that one clips its tets again from the cell of its K neighbours)
+      if (completing && job == 2 && state == 2) {
+        if (MESH && out_list) {
+          abandon = true;
+          break;
+        }
+        lost = true;
+        if (lane == 0) S.site_flags |= SITE_UNRESOLVED;
+        if (MESH) break;
+      }
 
       // ---------------------------------------------------------------
       bool take = state == 0, interior = false;
@@ -672,7 +693,7 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
         // |K-th neighbour - site|^2 > 4 max|v - site|^2 over the bounded cell
         const bool secmiss = build_miss && !(2.f * S.plane[4 + K - 1].w > 4.f * c.r2);
         bool cdone = false;  // completion pass: the cell was completed
-        if (COMPLETE) {
+        if (completing) {
           // Clip the cell by every site within 2R (R: the bound of its pieces
           // from the earlier pass) that is not among its K nearest: after
           // that no site can cut its pieces.  Such a site z (|z| >= |z_K|)
@@ -888,8 +909,10 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
           // outcome so far) goes to it and the site is done here; the
           // pieces pass clips each candidate tet by the faces crossing it.
           emitted = CELL_TET && !COMPLETE && !MESH && piece_list != nullptr && nfaces <= PIECE_FACES;
-          int nt_out = MESH ? c.nt : MESH_VERTS + 1;
-          if (MESH && COMPLETE) {
+          // (the last completion pass clips every cell that it is given itself)
+          constexpr bool to_mesh = MESH && WARP * SL <= MESH_VERTS;
+          int nt_out = to_mesh ? c.nt : MESH_VERTS + 1;
+          if (to_mesh && COMPLETE) {
             // the sites beyond the K nearest by rank among the cell's faces
             // (S.faces is ascending): id -> 4 + K + 12 + rank, the site in
             // the cell's record
@@ -908,7 +931,7 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
             __syncwarp();
             if (nfaces - own > MESH_EXT || !cdone) nt_out = MESH_VERTS + 1;
           }
-          if (MESH && nt_out <= MESH_VERTS) {
+          if (to_mesh && nt_out <= MESH_VERTS) {
             emitted = true;
             int base = 0;
 #pragma unroll
@@ -996,11 +1019,7 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
     if (abandon) {
       // the larger-capacity pass redoes this site from scratch
       if (COMPLETE) {
-        if (lane == 0) {
-          const int pos = atomicAdd(out_count, 1);
-          out_list[pos] = s;
-          out_r2[pos] = esc_r2[it];
-        }
+        if (lane == 0) out_list[atomicAdd(out_count, 1)] = s;
       } else if (lane == 0) {
         out_list[atomicAdd(out_count, 1)] = s;
         S.cnt[WC_REDO]++;
@@ -1010,11 +1029,17 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
       continue;
     }
     if (emitted) continue;  // the pieces pass finishes the site
+    if (COMPLETE && MESH) {
+      // a completion that lost a piece: the site's tets again, clipped from the
+      // cell of its K neighbours
+      again = lost && !again;
+      if (again) continue;
+    }
     if (lane == 0) {
       unsigned f = S.site_flags;
-      // a completion that failed keeps the earlier pass's moments
-      // (in the mesh form those are good only where the K neighbours were
-      // enough: a failed completion leaves what it clipped)
+      // a completion that failed keeps the earlier pass's moments; in the mesh
+      // form, which has none to keep (above), one whose search gave up leaves
+      // the pieces of the cell as far as it was cut
       const bool keep_old = COMPLETE && ((f & (MESH ? SITE_DROPPED : SITE_UNRESOLVED | SITE_DROPPED)) || S.unchanged);
       if (!keep_old)
         mom[s] = make_dmom4((double)S.acc[0] + (double)S.acc[4], (double)S.acc[1] + (double)S.acc[5],
@@ -1027,9 +1052,8 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
           const float4 seed = S.seed;
           const float dK2 = dist2(seed, sites[knn[PD(knn_off) + (size_t)(s - PD(site_off)) * K + K - 1]]);
           if (!(dK2 > __fmaf_rn(4.f * S.pr2, 1.0001f, 1e-4f))) {
-            const int pos = atomicAdd(esc_count, 1);
-            esc_list[pos] = s;
-            esc_r2[pos] = S.pr2;
+            esc_list[atomicAdd(esc_count, 1)] = s;
+            esc_r2[s] = S.pr2;
             f |= SITE_UNRESOLVED;
           }
         }
@@ -1425,9 +1449,8 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, ROBUST ? VGB_ROBUST_MIN_BLO
         const int K = PD(K);
         const float dK2 = dist2(S.seed, sites[knn[PD(knn_off) + (size_t)(s - PD(site_off)) * K + K - 1]]);
         if (!(dK2 > __fmaf_rn(4.f * S.pr2, 1.0001f, 1e-4f))) {
-          const int pos = atomicAdd(esc_count, 1);
-          esc_list[pos] = s;
-          esc_r2[pos] = S.pr2;
+          esc_list[atomicAdd(esc_count, 1)] = s;
+          esc_r2[s] = S.pr2;
           f |= SITE_UNRESOLVED;
         }
       }
@@ -1808,7 +1831,7 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
     k_clip_site<false, false, SLOTS_TET_CELL, R><<<(int)(want < need ? want : need), CLIP_WARPS * WARP, 0, st>>>(
         sites, n, knn, probs, site_prob, lone, verts, tets, site_start, site_tets, mom, stats, nullptr, nullptr,
         nullptr, nullptr, nullptr, nullptr, nullptr, prob_secmiss, nullptr, nullptr, nullptr, nullptr, nullptr,
-        CellStore{}, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+        CellStore{}, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
     VGB_CUDA_TRY(cudaGetLastError());
     return 0;
   }
@@ -1819,12 +1842,13 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
   // [9] their kNN's work counter, [10] sites to complete, [11] the
   // completion pass's work counter; lists: [0, n) the hand-offs to the
   // 128-vertex pass, [n, 2n) the first pass's, [2n, 3n) the deep sites,
-  // [3n, 4n) the sites to complete, [4n, 5n) their pieces' squared radius
-  // bounds (float) and [5n, 6n) the pieces pass's sites or the mesh pass's;
+  // [3n, 4n) the sites to complete, [4n, 5n) by site: the squared radius bound
+  // of its pieces (float) and [5n, 6n) the pieces pass's sites or the mesh pass's;
   // [12] the mesh pass's sites, [13] its work counter, [14, 15] the same for
   // its second launch, over completed cells (their list: [n, 2n) again),
-  // [16] the cells the completion pass finds above 64 vertices (in [0, n), the
-  // bounds in [2n, 3n)), [17] the work counter of the pass that takes them
+  // [16] the sites to complete at 256 vertices: those that the completion pass
+  // of 64 or the second mesh launch hands on (in [0, n) again), [17] the work
+  // counter of the pass that takes them
   const bool exact = tet_order != nullptr;
   int* const redo = lists;
   int* const rest = lists + n;
@@ -1851,7 +1875,7 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
         sites, n, knn, probs, site_prob, lone, verts, tets, site_start, site_tets, mom, stats, field, field_sat,
         tet_order, tet_cell_start, tet_sph, reach, reach_max_bits, prob_secmiss, in_list, in_count, out_list,
         out_count, work, cs, kt, cell_start, esc, esc_r2, exact ? counters + 10 : nullptr,
-        emit ? piece_list : nullptr, emit ? counters + 6 : nullptr, nullptr);
+        emit ? piece_list : nullptr, emit ? counters + 6 : nullptr);
   };
   // the pieces pass over the sites the one-warp pass handed on
   auto launch_pieces = [&](auto kernel, int variant) {
@@ -1890,30 +1914,28 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
   if constexpr (!R) {
     if (mesh) {
       auto pass = [&](auto kernel, int variant, const int* in_list, int* in_count, int* out_list, int* out_count,
-                      int* work, int* to_list, int* to_count, float* r2 = nullptr, float* out_r2 = nullptr) {
+                      int* work, int* to_list, int* to_count) {
         kernel<<<g_clip_resident_blocks[variant], CLIP_WARPS * WARP, 0, st>>>(
             sites, n, knn, probs, site_prob, lone, verts, tets, site_start, site_tets, mom, stats, field, field_sat,
             tet_order, tet_cell_start, tet_sph, reach, reach_max_bits, prob_secmiss, in_list, in_count, out_list,
-            out_count, work, cs, kt, cell_start, esc, r2 ? r2 : esc_r2, exact ? counters + 10 : nullptr, to_list,
-            to_count, out_r2);
+            out_count, work, cs, kt, cell_start, esc, esc_r2, exact ? counters + 10 : nullptr, to_list,
+            to_count);
       };
       auto mesh_pass = [&](const int* in_list, int* in_count, int* work, bool last) {
         auto go = [&](auto kernel, int variant) {
           kernel<<<g_clip_resident_blocks[variant], MESH_WARPS * WARP, 0, st>>>(
               sites, knn, probs, site_prob, lone, cs.rec, tet_cell_start, tet_sph, reach, reach_max_bits, mom, stats,
-              prob_secmiss, in_list, in_count, work, last ? nullptr : redo, counters + 1, cs, last ? nullptr : esc,
+              prob_secmiss, in_list, in_count, work, redo, counters + (last ? 16 : 1), cs, last ? nullptr : esc,
               esc_r2, counters + 10, site_start);
         };
         if (ref_mesh) go(k_cell_mesh<false, true>, 17);
         else if (probs) go(k_cell_mesh<true, false>, 12);
         else go(k_cell_mesh<false, false>, 11);
       };
-      // (cells the completion pass finds above 64 vertices: their bounds, in
-      // the deep sites' place)
-      float* const large_r2 = reinterpret_cast<float*>(deep);
       // the cells the first pass left, finished or taken whole; then what of
       // each lies in the mesh; then the cells above 64 vertices, and those
-      // their K neighbours left unresolved
+      // their K neighbours left unresolved: at 64 vertices and through the mesh
+      // pass, then what neither could finish at 256, clipped by each tet
       if (probs) {
         pass(k_clip_site<true, true, SLOTS_FAST, false, false, true>, 14, rest, counters + 0, redo, counters + 1,
              counters + 3, mesh_list, counters + 12);
@@ -1921,9 +1943,10 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
         pass(k_clip_site<true, true, SLOTS_REDO, false>, 4, redo, counters + 1, nullptr, nullptr, counters + 4,
              nullptr, nullptr);
         pass(k_clip_site<true, true, SLOTS_FAST, false, true, true>, 19, esc, counters + 10, redo, counters + 16,
-             counters + 11, rest, counters + 14, nullptr, large_r2);
+             counters + 11, rest, counters + 14);
+        mesh_pass(rest, counters + 14, counters + 15, true);
         pass(k_clip_site<true, true, SLOTS_COMPLETE, false, true, true>, 16, redo, counters + 16, nullptr, nullptr,
-             counters + 17, rest, counters + 14, large_r2);
+             counters + 17, nullptr, nullptr);
       } else {
         pass(k_clip_site<true, false, SLOTS_FAST, false, false, true>, 13, rest, counters + 0, redo, counters + 1,
              counters + 3, mesh_list, counters + 12);
@@ -1935,11 +1958,11 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
           return 0;
         }
         pass(k_clip_site<true, false, SLOTS_FAST, false, true, true>, 18, esc, counters + 10, redo, counters + 16,
-             counters + 11, rest, counters + 14, nullptr, large_r2);
+             counters + 11, rest, counters + 14);
+        mesh_pass(rest, counters + 14, counters + 15, true);
         pass(k_clip_site<true, false, SLOTS_COMPLETE, false, true, true>, 15, redo, counters + 16, nullptr, nullptr,
-             counters + 17, rest, counters + 14, large_r2);
+             counters + 17, nullptr, nullptr);
       }
-      mesh_pass(rest, counters + 14, counters + 15, true);
       VGB_CUDA_TRY(cudaGetLastError());
       return 0;
     }

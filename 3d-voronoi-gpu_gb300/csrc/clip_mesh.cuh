@@ -53,12 +53,8 @@ constexpr int MESH_ID_WORDS = (MESH_IDS + 31) / 32;
 // A cell whose terms exceed this many times their sum keeps a sliver of
 // itself in the mesh (one in a thousand of the boundary cells of random sites,
 // the site mostly outside): the terms' rounding, 1e-7 of a cell, would show in
-// it, so the 128-vertex pass clips it by each tet.  A completed cell, which
-// no pass follows, is summed again from a point of the sliver.
-constexpr float MESH_APEX_RATIO = 64.f;
-// A sum below this fraction of its terms (rounded to 1e-7 of them each) is
-// rounding: the cell only touches the mesh, and its site stays where it is.
-constexpr float MESH_NOISE = 1e-6f;
+// it, so a pass that follows clips it by each tet.
+constexpr float MESH_RATIO = 64.f;
 #ifndef VGB_MESH_MIN_BLOCKS
 #define VGB_MESH_MIN_BLOCKS 5
 #endif
@@ -118,7 +114,7 @@ __device__ __forceinline__ float line_at(float4 P, float3 p, float3 u, bool& ahe
 }
 
 // Signed tets of the piece [a, b] on the line of faces 0 and 1 (feet F0, F1;
-// all apex-relative; c = a x b, ab = a + b).
+// all relative to the apex, which is the site; c = a x b, ab = a + b).
 struct MeshSum {
   float v = 0.f, x = 0.f, y = 0.f, z = 0.f, mag = 0.f;
   __device__ __forceinline__ void add(float k, float3 F, float3 ab) {
@@ -130,10 +126,10 @@ struct MeshSum {
   }
 };
 
-// Foot of the apex X on plane P, relative to X.
-__device__ __forceinline__ float3 foot_of(float4 P, float3 X) {
+// Foot of the site on plane P.
+__device__ __forceinline__ float3 foot_of(float4 P) {
   const float nn = dot3_rn(P.x, P.y, P.z, P.x, P.y, P.z);
-  const float l = __fdividef(-eval4(P, X), nn);
+  const float l = __fdividef(-P.w, nn);
   return make_float3(__fmul_rn(l, P.x), __fmul_rn(l, P.y), __fmul_rn(l, P.z));
 }
 
@@ -310,11 +306,8 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
     __syncwarp();
 
     // -----------------------------------------------------------------
-    // the tets.  When the first apex (the site) turns out far from what is left
-    // of a completed cell: again for a mean of its points (lengths of its edges and
-    // moments of them in place of their terms), and then from that point
-    float3 X = make_float3(0.f, 0.f, 0.f);
-    float pr2 = 0.f, vol = 0.f, mx = 0.f, my = 0.f, mz = 0.f, v6 = 0.f, mag = 0.f;
+    // the tets
+    float pr2 = 0.f, vol = 0.f, mx = 0.f, my = 0.f, mz = 0.f;
     const int dim = PD(dim), cbase = PD(cell_off);
     const float rt = REF ? __uint_as_float(reach_max_bits[1]) : PD(rt_max);
     const float R = __fadd_rn(fminf(__fmaf_rn(rt, 1.001f, Rc), __uint_as_float(reach_max_bits[pidx])), 0.01f);
@@ -333,8 +326,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
     const int nj = cell_at(seed.y + R) - j0 + 1;
     const int nrow = nj * (cell_at(seed.z + R) - k0 + 1);
     const float per_row = __fdividef(1.f, (float)nj);
-#pragma unroll 1
-    for (int round = 0; round < 3 && !bad; ++round) {
+    if (!bad) {
       MeshSum sum;
       float far2 = 0.f;
       // a piece [a, b] of an edge: k = det(F1 - F0, p, u) (b - a), and the
@@ -342,13 +334,12 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
 #pragma unroll 1
       for (int i = lane; i < ne; i += WARP) {
         const unsigned E = S.edge[i];
-        const float3 F0 = foot_of(S.plane[E & 0xffu], X), F1 = foot_of(S.plane[(E >> 8) & 0xffu], X);
-        const float3 p = sub_rn(xyz(S.epos[i]), X), cr = cross_rn(p, xyz(S.edir[i]));
+        const float3 F0 = foot_of(S.plane[E & 0xffu]), F1 = foot_of(S.plane[(E >> 8) & 0xffu]);
+        const float3 p = xyz(S.epos[i]), cr = cross_rn(p, xyz(S.edir[i]));
         const float k0 = dot_rn(F0, cr), k1 = dot_rn(F1, cr), k = __fsub_rn(k1, k0), k2 = 2.f * k;
-        S.eterm[i] = round == 1 ? make_float4(2.f * p.x, 2.f * p.y, 2.f * p.z, 1.f)
-                                : make_float4(__fmaf_rn(k2, p.x, cross_term(k1, F1.x, k0, F0.x)),
-                                              __fmaf_rn(k2, p.y, cross_term(k1, F1.y, k0, F0.y)),
-                                              __fmaf_rn(k2, p.z, cross_term(k1, F1.z, k0, F0.z)), k);
+        S.eterm[i] = make_float4(__fmaf_rn(k2, p.x, cross_term(k1, F1.x, k0, F0.x)),
+                                 __fmaf_rn(k2, p.y, cross_term(k1, F1.y, k0, F0.y)),
+                                 __fmaf_rn(k2, p.z, cross_term(k1, F1.z, k0, F0.z)), k);
       }
       __syncwarp();
       int nq = 0, row0 = 0, f0 = 0, total = 0, incl = 0;
@@ -626,7 +617,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
               S.side[lane][0] = make_float4(L.p.x, L.p.y, L.p.z, L.a);
               S.side[lane][1] = make_float4(L.u.x, L.u.y, L.u.z, L.b);
             }
-            const float3 FT = foot_of(PT, X);
+            const float3 FT = foot_of(PT);
             __syncwarp();
             float lo = 1.f, hi = -1.f;  // lanes 0-2: the side's part inside the cell
 #pragma unroll 1
@@ -667,66 +658,45 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
                   }
                 }
                 if (keep) {
-                  const float3 aX = sub_rn(a, X), bX = sub_rn(bb, X);
-                  const float3 cr = cross_rn(aX, bX), ab = make_float3(__fadd_rn(aX.x, bX.x), __fadd_rn(aX.y, bX.y), __fadd_rn(aX.z, bX.z));
-                  const float3 F = foot_of(S.plane[f], X);
-                  if (round == 1) {
-                    sum.add(1.f, make_float3(0.f, 0.f, 0.f), ab);
-                  } else {
-                    sum.add(dot_rn(F, cr), F, ab);
-                    sum.add(-dot_rn(FT, cr), FT, ab);
-                  }
+                  const float3 cr = cross_rn(a, bb), ab = make_float3(__fadd_rn(a.x, bb.x), __fadd_rn(a.y, bb.y), __fadd_rn(a.z, bb.z));
+                  const float3 F = foot_of(S.plane[f]);
+                  sum.add(dot_rn(F, cr), F, ab);
+                  sum.add(-dot_rn(FT, cr), FT, ab);
                 }
               }
             }
             // the sides inside the cell, walked around the inward normal
             if (hi > lo) {
               const float3 p = xyz(S.side[lane][0]), u = xyz(S.side[lane][1]);
-              const float3 aX = sub_rn(along(p, lo, u), X), bX = sub_rn(along(p, hi, u), X);
-              const float3 cr = cross_rn(aX, bX), ab = make_float3(__fadd_rn(aX.x, bX.x), __fadd_rn(aX.y, bX.y), __fadd_rn(aX.z, bX.z));
+              const float3 a = along(p, lo, u), bb = along(p, hi, u);
+              const float3 cr = cross_rn(a, bb), ab = make_float3(__fadd_rn(a.x, bb.x), __fadd_rn(a.y, bb.y), __fadd_rn(a.z, bb.z));
               const float k6 = dot_rn(FT, cr);
-              sum.add(round == 1 ? 1.f : (side == (lane != 1)) ? -k6 : k6,
-                      round == 1 ? make_float3(0.f, 0.f, 0.f) : FT, ab);
+              sum.add((side == (lane != 1)) ? -k6 : k6, FT, ab);
             }
             __syncwarp();
           }
         }
         __syncwarp();
       }
-      v6 = warp_sum(sum.v);
-      mag = warp_sum(sum.mag);
-      const float x24 = warp_sum(sum.x), y24 = warp_sum(sum.y), z24 = warp_sum(sum.z);
-      pr2 = fmaxf(pr2, warp_max_nonneg(far2));
-      if (round == 1) {
-        if (!(v6 > 0.f)) break;
-        const float w = __fdividef(0.5f, v6);
-        X = make_float3(__fmul_rn(x24, w), __fmul_rn(y24, w), __fmul_rn(z24, w));
-        continue;
-      }
+      const float v6 = warp_sum(sum.v), mag = warp_sum(sum.mag);
+      pr2 = warp_max_nonneg(far2);
       vol = __fmul_rn(v6, 1.f / 6.f);
-      mx = __fmaf_rn(x24, 1.f / 24.f, __fmul_rn(vol, X.x));
-      my = __fmaf_rn(y24, 1.f / 24.f, __fmul_rn(vol, X.y));
-      mz = __fmaf_rn(z24, 1.f / 24.f, __fmul_rn(vol, X.z));
-      // large terms for a small sum: the apex is far from what is left
-      if (mag <= MESH_APEX_RATIO * v6 || mag == 0.f) break;
-      if (out_list) bad = true;
+      mx = __fmul_rn(warp_sum(sum.x), 1.f / 24.f);
+      my = __fmul_rn(warp_sum(sum.y), 1.f / 24.f);
+      mz = __fmul_rn(warp_sum(sum.z), 1.f / 24.f);
+      // large terms for a small sum: a sliver, or a cell that only touches the
+      // mesh (or no number at all)
+      bad = !(mag <= MESH_RATIO * v6 || mag == 0.f);
     }
-    // a sum within its terms' rounding is none (a tet that only touches)
-    if (!(v6 > MESH_NOISE * mag)) vol = mx = my = mz = v6 == v6 ? 0.f : v6;
     bad |= !(isfinite(vol) && isfinite(mx) && isfinite(my) && isfinite(mz));
     if (bad) {
-      // degenerate, or a sliver: the 128-vertex pass clips a copy of the cell by
-      // each tet (a completed cell keeps its earlier moments)
+      // degenerate, or a sliver: the pass that follows clips a copy of the cell by
+      // each tet (at 128 vertices; of a completed cell at 256)
       if (lane == 0) {
-        if (out_list) {
-          out_list[atomicAdd(out_count, 1)] = s;
-          S.cnt[WC_REDO]++;
-          store.nt[s] = 0;
-          if (store.flags) store.flags[s] = (unsigned char)(flags | SITE_HANDED | SITE_REDO);
-        } else {
-          S.cnt[WC_UNRESOLVED]++;
-          if (store.flags) store.flags[s] = (unsigned char)(flags | SITE_UNRESOLVED);
-        }
+        out_list[atomicAdd(out_count, 1)] = s;
+        if (!(flags & SITE_COMPLETED)) S.cnt[WC_REDO]++;
+        store.nt[s] = 0;
+        if (store.flags) store.flags[s] = (unsigned char)(flags | SITE_HANDED | SITE_REDO);
       }
       __syncwarp();
       continue;
@@ -744,9 +714,8 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
         // exact where it meets the mesh when that lies within half the K-th
         // neighbour's distance; else completed by the completion pass
         if (!(dK2 > __fmaf_rn(4.f * pr2, 1.0001f, 1e-4f))) {
-          const int pos = atomicAdd(esc_count, 1);
-          esc_list[pos] = s;
-          esc_r2[pos] = pr2;
+          esc_list[atomicAdd(esc_count, 1)] = s;
+          esc_r2[s] = pr2;
           f |= SITE_UNRESOLVED;
         }
       }
