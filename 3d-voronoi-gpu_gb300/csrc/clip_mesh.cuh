@@ -71,8 +71,8 @@ struct MeshSmem {
     unsigned char twin[MESH_FACES * MESH_FACES];  // (p, q) -> vertex, while the edges are made
     float4 slot[2][MESH_FACES];  // a triangle's plane across each face: first and second point
   };
-  // the cell's edges: point nearest the site and direction, with the end
-  // parameters; the terms of a unit of its length (volume in w)
+  // the cell's edges: point nearest the site and direction, with the smaller
+  // and the larger end parameter; the terms of a unit of its length (volume in w)
   float4 epos[MESH_EDGES], edir[MESH_EDGES], eterm[MESH_EDGES];
   unsigned edge[MESH_EDGES];  // faces p, q and end vertices of each
   float3 vert[MESH_VERTS];    // the cell's vertices
@@ -297,11 +297,24 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
       const float3 a = cross_rn(xyz(P), D), b = cross_rn(D, xyz(Q));
       const float i2 = __fdividef(-1.f, dd), i1 = rsqrtf(dd);
       const float3 u = make_float3(__fmul_rn(D.x, i1), __fmul_rn(D.y, i1), __fmul_rn(D.z, i1));
-      S.epos[i] = make_float4(__fmul_rn(i2, __fmaf_rn(Q.w, a.x, __fmul_rn(P.w, b.x))),
-                              __fmul_rn(i2, __fmaf_rn(Q.w, a.y, __fmul_rn(P.w, b.y))),
-                              __fmul_rn(i2, __fmaf_rn(Q.w, a.z, __fmul_rn(P.w, b.z))),
-                              dot_rn(S.vert[(E >> 16) & 0xffu], u));
-      S.edir[i] = make_float4(u.x, u.y, u.z, dot_rn(S.vert[E >> 24], u));
+      const float3 p = make_float3(__fmul_rn(i2, __fmaf_rn(Q.w, a.x, __fmul_rn(P.w, b.x))),
+                                   __fmul_rn(i2, __fmaf_rn(Q.w, a.y, __fmul_rn(P.w, b.y))),
+                                   __fmul_rn(i2, __fmaf_rn(Q.w, a.z, __fmul_rn(P.w, b.z))));
+      // Where planes nearly share a line, rounding may place a vertex beyond
+      // its neighbour: an edge from its end back to its start, whose terms
+      // count against those of the edges that reach too far
+      const float t0 = dot_rn(S.vert[(E >> 16) & 0xffu], u), t1 = dot_rn(S.vert[E >> 24], u);
+      S.epos[i] = make_float4(p.x, p.y, p.z, fminf(t0, t1));
+      S.edir[i] = make_float4(u.x, u.y, u.z, fmaxf(t0, t1));
+      // a piece [a, b] of an edge: k = det(F1 - F0, p, u) (b - a), and the
+      // moment k1 (F1 + a + b) - k0 (F0 + a + b)
+      const float sg = t1 < t0 ? -1.f : 1.f;
+      const float3 F0 = foot_of(P), F1 = foot_of(Q), cr = cross_rn(p, u);
+      const float k0 = __fmul_rn(sg, dot_rn(F0, cr)), k1 = __fmul_rn(sg, dot_rn(F1, cr)), k = __fsub_rn(k1, k0);
+      const float k2 = 2.f * k;
+      S.eterm[i] = make_float4(__fmaf_rn(k2, p.x, cross_term(k1, F1.x, k0, F0.x)),
+                               __fmaf_rn(k2, p.y, cross_term(k1, F1.y, k0, F0.y)),
+                               __fmaf_rn(k2, p.z, cross_term(k1, F1.z, k0, F0.z)), k);
     }
     __syncwarp();
 
@@ -329,19 +342,6 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
     if (!bad) {
       MeshSum sum;
       float far2 = 0.f;
-      // a piece [a, b] of an edge: k = det(F1 - F0, p, u) (b - a), and the
-      // moment k1 (F1 + a + b) - k0 (F0 + a + b)
-#pragma unroll 1
-      for (int i = lane; i < ne; i += WARP) {
-        const unsigned E = S.edge[i];
-        const float3 F0 = foot_of(S.plane[E & 0xffu]), F1 = foot_of(S.plane[(E >> 8) & 0xffu]);
-        const float3 p = xyz(S.epos[i]), cr = cross_rn(p, xyz(S.edir[i]));
-        const float k0 = dot_rn(F0, cr), k1 = dot_rn(F1, cr), k = __fsub_rn(k1, k0), k2 = 2.f * k;
-        S.eterm[i] = make_float4(__fmaf_rn(k2, p.x, cross_term(k1, F1.x, k0, F0.x)),
-                                 __fmaf_rn(k2, p.y, cross_term(k1, F1.y, k0, F0.y)),
-                                 __fmaf_rn(k2, p.z, cross_term(k1, F1.z, k0, F0.z)), k);
-      }
-      __syncwarp();
       int nq = 0, row0 = 0, f0 = 0, total = 0, incl = 0;
       bool more = true;
       while (more || nq > 0) {

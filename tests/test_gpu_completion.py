@@ -45,3 +45,20 @@ def test_a_completion_that_loses_a_piece_leaves_a_whole_sum(pkg, meshgen, n_side
     assert given_up.sum() == st["unresolved"] > 3
     off = np.abs(v / vol - 1)[given_up]
     assert off.max() < 6 * MOVED / np.cbrt(vol).min(), np.flatnonzero(given_up)[off.argmax()]
+
+
+@pytest.mark.parametrize("site_k", [12, 32])
+@pytest.mark.parametrize("n_side", [8, 10, 11, 13, 18, 19])
+def test_cells_with_vertices_placed_beyond_their_neighbours(pkg, meshgen, n_side, site_k):
+    """Three faces that nearly share a line meet in a vertex that rounding moves
+    far along it, past the edge's other end: such a cell's edges count with
+    their sign, and one that a mesh plane meets more than twice on a face is
+    clipped by each tet.  Cells that were not dropped or given up are their
+    lattice boxes, with the bound of the test above."""
+    pkg.build()
+    P, sites, vol, h = near_lattice(meshgen, n_side)
+    v, f, _ = cells(pkg, P, sites, site_k=site_k)
+    ok = (f & (pkg.SITE_DROPPED | pkg.SITE_UNRESOLVED)) == 0
+    assert ok.mean() > 0.99
+    off = np.where(ok, np.abs(v / vol - 1), 0.0)
+    assert off.max() < 6 * MOVED / np.cbrt(vol).min(), off.argmax()
