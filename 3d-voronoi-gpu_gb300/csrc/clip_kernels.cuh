@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
     // outcome bits of the site (cell-tet method): this pass built its cell
     if (lane == 0) {
       S.site_flags = SITE_HANDED | (SL > 2 ? SITE_REDO : 0);
-      S.pr2 = completing ? esc_r2[s] : 0.f;
+      S.pr2 = completing ? fabsf(esc_r2[s]) : 0.f;
       S.unchanged = 0;
       S.Rc = 0.f;
       S.nfaces = 0;
@@ -812,7 +812,7 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
               }
           if (abandon) break;
           cdone = !fail;
-          if (cdone && ncut == 0) {
+          if (cdone && ncut == 0 && !(MESH && esc_r2[s] < 0.f)) {
             // nothing beyond the K nearest cuts the cell: the earlier pass's
             // pieces were exact; keep them and clip no tet again
             if (lane == 0) {

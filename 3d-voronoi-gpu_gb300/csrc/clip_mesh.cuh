@@ -24,7 +24,10 @@
 // of the cell meets a triangle (on the edge), where a side of a triangle meets
 // a face of the cell (on the side).  Lines are kept as their point nearest
 // the site and a unit direction, so that a long edge of an open cell is as
-// exact near the site as a short one.
+// exact near the site as a short one.  Where that is not enough (an edge and a
+// triangle's side within rounding of each other, a face in a triangle's plane)
+// the lines of a face or a triangle no longer close, which one more sum over
+// the pieces tells (face_mark): the cell is given back and clipped by each tet.
 //
 // One warp per site: lanes take candidate tets, then (tet, edge) pairs, then
 // faces.  Bound by latency (issuing on 63% of cycles, five blocks of four warps
@@ -55,6 +58,14 @@ constexpr int MESH_ID_WORDS = (MESH_IDS + 31) / 32;
 // the site mostly outside): the terms' rounding, 1e-7 of a cell, would show in
 // it, so a pass that follows clips it by each tet.
 constexpr float MESH_RATIO = 64.f;
+// So it does with a cell whose faces' lines leave more than these parts of its
+// radius and of all their lengths open: the ends of pieces are rounded to 1e-7
+// of the radius each, their sum to as much of what it went through.
+// Where three planes nearly share a line and that line nearly lies in one of the
+// mesh's planes (sites of a lattice along the mesh's axes), the sides that
+// rounding gives a point of an edge and of a triangle may disagree, and a piece
+// is lost, or counted twice.
+constexpr float MESH_CLOSED = 2e-5f, MESH_WAY = 5e-7f;
 #ifndef VGB_MESH_MIN_BLOCKS
 #define VGB_MESH_MIN_BLOCKS 5
 #endif
@@ -75,6 +86,7 @@ struct MeshSmem {
   // and the larger end parameter; the terms of a unit of its length (volume in w)
   float4 epos[MESH_EDGES], edir[MESH_EDGES], eterm[MESH_EDGES];
   unsigned edge[MESH_EDGES];  // faces p, q and end vertices of each
+  float eopen[MESH_EDGES];    // what a unit of its length leaves open (face_mark)
   float3 vert[MESH_VERTS];    // the cell's vertices
   float4 side[3][2];  // a triangle's sides: point and direction, end parameters in w
   float at[3][MESH_FACES];  // where each face meets them
@@ -116,7 +128,11 @@ __device__ __forceinline__ float line_at(float4 P, float3 p, float3 u, bool& ahe
 // Signed tets of the piece [a, b] on the line of faces 0 and 1 (feet F0, F1;
 // all relative to the apex, which is the site; c = a x b, ab = a + b).
 struct MeshSum {
-  float v = 0.f, x = 0.f, y = 0.f, z = 0.f, mag = 0.f;
+  float v = 0.f, x = 0.f, y = 0.f, z = 0.f, mag = 0.f, open = 0.f, way = 0.f;
+  __device__ __forceinline__ void close(float o) {
+    open = __fadd_rn(open, o);
+    way = __fadd_rn(way, fabsf(o));
+  }
   __device__ __forceinline__ void add(float k, float3 F, float3 ab) {
     v = __fadd_rn(v, k);
     mag = __fadd_rn(mag, fabsf(k));
@@ -125,6 +141,15 @@ struct MeshSum {
     z = __fmaf_rn(k, __fadd_rn(F.z, ab.z), z);
   }
 };
+
+// Around each face of a cell, and around each triangle, the pieces of its lines
+// close: their vectors sum to nothing.  One sum checks them all, each piece by
+// its product with a vector of its face (hashed, components within 1).
+__device__ __forceinline__ float3 face_mark(unsigned f) {
+  const unsigned h = (f + 1u) * 0x9e3779b1u;
+  return make_float3(0x1p-31f * (float)(int)(h << 24), 0x1p-31f * (float)(int)(h << 16),
+                     0x1p-31f * (float)(int)(h << 8));
+}
 
 // Foot of the site on plane P.
 __device__ __forceinline__ float3 foot_of(float4 P) {
@@ -315,12 +340,14 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
       S.eterm[i] = make_float4(__fmaf_rn(k2, p.x, cross_term(k1, F1.x, k0, F0.x)),
                                __fmaf_rn(k2, p.y, cross_term(k1, F1.y, k0, F0.y)),
                                __fmaf_rn(k2, p.z, cross_term(k1, F1.z, k0, F0.z)), k);
+      S.eopen[i] = __fmul_rn(sg, dot_rn(u, sub_rn(face_mark((E >> 8) & 0xffu), face_mark(E & 0xffu))));
     }
     __syncwarp();
 
     // -----------------------------------------------------------------
     // the tets
     float pr2 = 0.f, vol = 0.f, mx = 0.f, my = 0.f, mz = 0.f;
+    bool open = false;  // its faces' lines do not close
     const int dim = PD(dim), cbase = PD(cell_off);
     const float rt = REF ? __uint_as_float(reach_max_bits[1]) : PD(rt_max);
     const float R = __fadd_rn(fminf(__fmaf_rn(rt, 1.001f, Rc), __uint_as_float(reach_max_bits[pidx])), 0.01f);
@@ -342,6 +369,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
     if (!bad) {
       MeshSum sum;
       float far2 = 0.f;
+      int skew = 0;  // ends of crossing edges, less the faces' slots they took
       int nq = 0, row0 = 0, f0 = 0, total = 0, incl = 0;
       bool more = true;
       while (more || nq > 0) {
@@ -516,6 +544,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
               const float d = __fsub_rn(hi, lo), m = __fadd_rn(hi, lo), k = __fmul_rn(T4.w, d), km = __fmul_rn(k, m);
               sum.v = __fadd_rn(sum.v, k);
               sum.mag = __fadd_rn(sum.mag, fabsf(k));
+              sum.close(__fmul_rn(d, S.eopen[e]));
               sum.x = __fadd_rn(sum.x, __fmaf_rn(km, u.x, __fmul_rn(d, T4.x)));
               sum.y = __fadd_rn(sum.y, __fmaf_rn(km, u.y, __fmul_rn(d, T4.y)));
               sum.z = __fadd_rn(sum.z, __fmaf_rn(km, u.z, __fmul_rn(d, T4.z)));
@@ -591,8 +620,10 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
             const bool side = face_side(inf, i);
             // the cell's edges across its plane: where each face's line with
             // it begins and ends.  The side of each vertex is decided once for
-            // all its edges, so that every face has its two ends or none (the
-            // box that bounds an open cell has edges that lie in mesh planes)
+            // all its edges, so that a face has as many beginnings as ends (the
+            // box that bounds an open cell has edges that lie in mesh planes):
+            // one of each or none, else (skew) a slot is taken twice and the cell
+            // given back
             const unsigned up0 = __ballot_sync(FULL, lane < nt && eval4(PT, S.vert[lane]) >= 0.f);
             const unsigned up1 = __ballot_sync(FULL, lane + WARP < nt && eval4(PT, S.vert[lane + WARP]) >= 0.f);
             auto above = [&](unsigned v) { return ((v < WARP ? up0 : up1) >> (v & 31u)) & 1u; };
@@ -608,6 +639,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
                 const int in = end == side ? 0 : 1;
                 S.slot[in][E & 0xffu] = make_float4(x.x, x.y, x.z, 1.f);
                 S.slot[1 - in][(E >> 8) & 0xffu] = make_float4(x.x, x.y, x.z, 1.f);
+                skew += 2;
               }
             }
             // its sides: 0 (t1, t2), 1 (t0, t2), 2 (t0, t1), a line each on
@@ -617,7 +649,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
               S.side[lane][0] = make_float4(L.p.x, L.p.y, L.p.z, L.a);
               S.side[lane][1] = make_float4(L.u.x, L.u.y, L.u.z, L.b);
             }
-            const float3 FT = foot_of(PT);
+            const float3 FT = foot_of(PT), mark = face_mark(MESH_FACES + 4 * b + i);
             __syncwarp();
             float lo = 1.f, hi = -1.f;  // lanes 0-2: the side's part inside the cell
 #pragma unroll 1
@@ -639,6 +671,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
 #pragma unroll 1
             for (int f = lane; f < nf; f += WARP) {
               const float4 a4 = S.slot[0][f], b4 = S.slot[1][f];
+              skew -= (a4.w != 0.f) + (b4.w != 0.f);
               if (a4.w != 0.f && b4.w != 0.f) {
                 float3 a = xyz(a4), bb = xyz(b4);
                 bool keep = true;
@@ -661,6 +694,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
                   const float3 cr = cross_rn(a, bb), ab = make_float3(__fadd_rn(a.x, bb.x), __fadd_rn(a.y, bb.y), __fadd_rn(a.z, bb.z));
                   const float3 F = foot_of(S.plane[f]);
                   sum.add(dot_rn(F, cr), F, ab);
+                  sum.close(dot_rn(sub_rn(bb, a), sub_rn(face_mark(f), mark)));
                   sum.add(-dot_rn(FT, cr), FT, ab);
                 }
               }
@@ -672,6 +706,8 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
               const float3 cr = cross_rn(a, bb), ab = make_float3(__fadd_rn(a.x, bb.x), __fadd_rn(a.y, bb.y), __fadd_rn(a.z, bb.z));
               const float k6 = dot_rn(FT, cr);
               sum.add((side == (lane != 1)) ? -k6 : k6, FT, ab);
+              const float op = dot_rn(sub_rn(bb, a), mark);
+              sum.close((side == (lane != 1)) ? -op : op);
             }
             __syncwarp();
           }
@@ -687,8 +723,15 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
       // large terms for a small sum: a sliver, or a cell that only touches the
       // mesh (or no number at all)
       bad = !(mag <= MESH_RATIO * v6 || mag == 0.f);
+      const float tol = __fmaf_rn(MESH_CLOSED, pr2 > 0.f ? sqrtf(pr2) : Rc, MESH_WAY * warp_sum(sum.way));
+      open = !(fabsf(warp_sum(sum.open)) <= tol) || __reduce_add_sync(FULL, skew) != 0;
     }
     bad |= !(isfinite(vol) && isfinite(mx) && isfinite(my) && isfinite(mz));
+    // exact where it meets the mesh when that lies within half the K-th
+    // neighbour's distance; else completed by the completion pass (and open as
+    // long as tets out of the true cell's reach are left out)
+    const bool beyond = esc_list && miss && !(dK2 > __fmaf_rn(4.f * pr2, 1.0001f, 1e-4f));
+    bad |= open && !beyond;
     if (bad) {
       // degenerate, or a sliver: the pass that follows clips a copy of the cell by
       // each tet (at 128 vertices; of a completed cell at 256)
@@ -710,14 +753,11 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
     if (lane == 0) {
       unsigned f = flags | SITE_HANDED;
       mom[s] = make_dmom4((double)vol, (double)mx, (double)my, (double)mz);
-      if (esc_list && miss) {
-        // exact where it meets the mesh when that lies within half the K-th
-        // neighbour's distance; else completed by the completion pass
-        if (!(dK2 > __fmaf_rn(4.f * pr2, 1.0001f, 1e-4f))) {
-          esc_list[atomicAdd(esc_count, 1)] = s;
-          esc_r2[s] = pr2;
-          f |= SITE_UNRESOLVED;
-        }
+      if (beyond) {
+        // (a bound below zero: these moments are not to be kept)
+        esc_list[atomicAdd(esc_count, 1)] = s;
+        esc_r2[s] = open ? -pr2 : pr2;
+        f |= SITE_UNRESOLVED;
       }
       if (miss) {
         S.cnt[WC_SECMISS]++;
