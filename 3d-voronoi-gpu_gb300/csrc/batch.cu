@@ -419,7 +419,7 @@ int vgb_batch_create(vgb_batch** out, const vgb_config* cfg_in, int n_prob, cons
         return VGB_ERR_CUDA;
       }
   }
-  if (b->rec && face_info(b->verts, b->tets, b->n_vert, b->n_tet, b->face_info, nullptr, b->st)) {
+  if (b->rec && face_info(b->verts, b->tets, b->tet_prob, b->n_vert, b->n_tet, b->face_info, nullptr, b->st)) {
     free_batch(b);
     return VGB_ERR_CUDA;
   }

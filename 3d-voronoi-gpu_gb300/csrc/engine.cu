@@ -546,7 +546,7 @@ int vgb_engine_create(vgb_engine** out, const vgb_config* cfg_in, const float* v
       free_engine(e);
       return rc;
     }
-    if (face_info(e->verts, e->tets, n_vert, n_tet, info, across, e->st) ||
+    if (face_info(e->verts, e->tets, nullptr, n_vert, n_tet, info, across, e->st) ||
         (across && tets_beside(e->tet_order, across, n_tet, (int*)info + n_tet, e->beside, e->st)) ||
         tet_records(e->verts, e->tets, e->tet_order, info, n_tet, e->rec, e->st) ||
         tet_spheres(e->verts, e->tets, e->tet_order, n_tet, e->tet_sph, e->st)) {

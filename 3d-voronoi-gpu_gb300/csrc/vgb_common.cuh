@@ -224,19 +224,21 @@ int tet_reach(const float4* sites, const int* cell_start, const ProbDesc* probs,
               unsigned* reach_max_bits, cudaStream_t st);
 // Bounding spheres (centroid, radius) of the tets in centroid-cell order.
 int tet_spheres(const float4* verts, const int4* tets, const int* tet_order, int n_tet, float4* sph, cudaStream_t st);
-// The tets for the mesh pass, in centroid-cell order: corners by ascending
-// vertex index (12 floats), an info word (bits 0-3: the face that leaves out
-// the i-th corner is open; 4: that corner order is an even permutation of a
-// positively oriented tet; 5: not positively oriented), 3 spare words.
-// info: bits 0-5 per tet in input order, from face_info.
+// The tets for the mesh pass, in centroid-cell order: corners by ascending name
+// (12 floats; a vertex's name is the smallest index at its position), an info
+// word (bits 0-3: the face that leaves out the i-th corner is open; 4: that
+// corner order is an even permutation of a positively oriented tet; 5: not
+// positively oriented), 3 spare words.  info: one word per tet in input order,
+// from face_info.
 int tet_records(const float4* verts, const int4* tets, const int* tet_order, const unsigned* info, int n_tet,
                 float4* rec, cudaStream_t st);
-// Which faces of each tet are open (no other tet shares them from the other
-// side) and the tets' orientations: the info words of tet_records, input
-// order.  Allocates its scratch; synchronises.
+// Which faces of each tet are open (no other tet of its problem has it from the
+// other side), the tets' orientations and the order of their corners: the info
+// words of tet_records, input order.  Allocates its scratch; synchronises.
+// tet_prob (may be null): the tets' problems; problems share no vertex.
 // beside (may be null): the tet across each face, input order, -1 where open.
-int face_info(const float4* verts, const int4* tets, int n_vert, int n_tet, unsigned* info, int4* beside,
-              cudaStream_t st);
+int face_info(const float4* verts, const int4* tets, const int* tet_prob, int n_vert, int n_tet, unsigned* info,
+              int4* beside, cudaStream_t st);
 // The same in centroid-cell order; where: n_tet ints scratch.
 int tets_beside(const int* tet_order, const int4* beside, int n_tet, int* where, int4* out, cudaStream_t st);
 // Reference form: last[q] = (squared distance from its centroid, id) of the
