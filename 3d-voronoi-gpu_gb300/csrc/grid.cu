@@ -4,8 +4,8 @@
 // count needs: 3 at 1M sites); cell starts come from an atomic count and a
 // device exclusive scan.  Up to 65,536 sites are placed by counting instead:
 // the gather's atomic gives each site a slot of its cell, and a site's place
-// is its rank by id among its cell's (launch-bound sizes: 20k sites 160 -> 25
-// us, 500 sites 45 -> 20; above that the radix passes, whose cost does not
+// is its rank by id among its cell's, counted in bits where a cell holds many
+// (launch-bound sizes: 20k sites 160 -> 25 us, 500 sites 45 -> 20; above that the radix passes, whose cost does not
 // depend on how many sites share a cell, with tiles small enough to fill the
 // chip: 125k sites 46 -> 11 us a pass).  Replaces kn_firstbuild's count / reserve / store
 // (knearests.cu:29-57, 149-198), whose `reserve` hands out cell ranges in
@@ -202,18 +202,60 @@ __global__ void k_grid_place(const unsigned* __restrict__ key, const int* __rest
   if (i < n) member[cell_start[key[i]] + arrived[i]] = i;
 }
 
-__global__ void k_grid_rank(const unsigned* __restrict__ key, const int* __restrict__ member, int n,
-                            const int* __restrict__ cell_start, const float4* __restrict__ val,
-                            float4* __restrict__ out) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const int i = member[p];
-  const unsigned c = key[i];
-  const int b = cell_start[c], e = cell_start[c + 1];
-  int r = 0;
-  for (int q = b; q < e; ++q) r += member[q] < i;
-  out[b + r] = val[i];
+// Cells of at most GRID_RANK_MAX sites: by looking at all of them (1 us for a
+// hundred).  Larger ones, a block's one after the other: the cell's sites as bits
+// of one word per 32 sites (all sites, so few there are), the bits before each
+// word summed, and a site's rank is its word's sum and the bits below its own.
+// (65,000 sites, all but 1,300 in one cell: the whole sort 1.12 -> 0.10 ms, half
+// of 20,000 0.20 -> 0.04; by the radix passes 0.15 and 0.13.)
+constexpr int GRID_RANK_MAX = 256, RANK_THREADS = 256, RANK_WORDS = GRID_COUNT_MAX / 32;
+__global__ void __launch_bounds__(RANK_THREADS) k_grid_rank(const unsigned* __restrict__ key,
+                                                            const int* __restrict__ member, int n,
+                                                            const int* __restrict__ cell_start,
+                                                            const float4* __restrict__ val, float4* __restrict__ out) {
+  __shared__ unsigned bits[RANK_WORDS];
+  __shared__ int before[RANK_WORDS / 8];  // bits before each 8 words
+  __shared__ int ws[32];
+  __shared__ unsigned next;
+  const int p = blockIdx.x * RANK_THREADS + threadIdx.x;
+  const int i = p < n ? member[p] : 0;
+  const unsigned c = p < n ? key[i] : 0xffffffffu;
+  const int b = p < n ? cell_start[c] : 0, e = p < n ? cell_start[c + 1] : 0;
+  const bool large = e - b > GRID_RANK_MAX;
+  if (p < n && !large) {
+    int r = 0;
+    for (int q = b; q < e; ++q) r += member[q] < i;
+    out[b + r] = val[i];
+  }
+  bool todo = large;
+  while (__syncthreads_or(todo)) {
+    // the lowest cell left (the block's sites are in the order of their cells)
+    if (threadIdx.x == 0) next = 0xffffffffu;
+    for (int w = threadIdx.x; w < RANK_WORDS; w += RANK_THREADS) bits[w] = 0u;
+    __syncthreads();
+    if (todo) atomicMin(&next, c);
+    __syncthreads();
+    const unsigned cell = next;
+    const int cb = cell_start[cell], ce = cell_start[cell + 1];
+    for (int q = cb + (int)threadIdx.x; q < ce; q += RANK_THREADS) {
+      const int m = member[q];
+      atomicOr(bits + (m >> 5), 1u << (m & 31));
+    }
+    __syncthreads();
+    int total, s = 0;
+    for (int w = 0; w < 8; ++w) s += __popc(bits[threadIdx.x * 8 + w]);
+    before[threadIdx.x] = block_exclusive_scan(s, ws, total);
+    __syncthreads();
+    if (todo && c == cell) {
+      const int w = i >> 5;
+      int r = before[w >> 3] + __popc(bits[w] & ((1u << (i & 31)) - 1u));
+      for (int u = w & ~7; u < w; ++u) r += __popc(bits[u]);
+      out[b + r] = val[i];
+      todo = false;
+    }
+  }
 }
+static_assert(RANK_WORDS == 8 * RANK_THREADS, "eight words a thread");
 
 // Digit histogram of one tile of keys per warp, written bucket-major
 // (counts[digit * ntiles + tile]) so one exclusive scan gives every tile's
@@ -297,7 +339,7 @@ static int sort_sites(float4* sites, float4* tmp, int n, long long ncell, const 
   if (scan_exclusive(cell_start, cell_start, ncell + 1, scan_tmp, st)) return -2;
   if (n > 0 && counting) {
     k_grid_place<<<nblk, 256, 0, st>>>(key_a, arrived, n, cell_start, member);
-    k_grid_rank<<<nblk, 256, 0, st>>>(key_a, member, n, cell_start, va, vb);
+    k_grid_rank<<<nblk, RANK_THREADS, 0, st>>>(key_a, member, n, cell_start, va, vb);
     VGB_CUDA_TRY(cudaGetLastError());
     std::swap(va, vb);
   } else if (n > 0) {

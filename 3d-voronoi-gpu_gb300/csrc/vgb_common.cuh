@@ -168,8 +168,7 @@ int scan_exclusive(const int* in, int* out, long long n, int* tmp, cudaStream_t 
 //   cell_start: ncell + 1 ints; work: grid_sort_work_ints(n, ncell) ints.
 // Up to GRID_COUNT_MAX sites are placed by counting instead: a slot of its
 // cell for each site, then its rank among its cell's sites by id -- four
-// launches instead of ten to fifteen, the cost growing with the square of a
-// cell's sites, which so few bound (the kNN's does too).
+// launches instead of ten to fifteen.
 constexpr int RADIX_BITS = 8;
 constexpr int RADIX_BUCKETS = 1 << RADIX_BITS;
 constexpr int GRID_COUNT_MAX = 65536;
