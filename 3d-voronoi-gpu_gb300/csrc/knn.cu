@@ -324,6 +324,9 @@ __global__ void __launch_bounds__(W * 32, 32 / W) k_knn(const float4* __restrict
     // the ball, only keys inside it taken: when K are found they are the K
     // nearest, and the walk below is not needed.  A radius too small (3% of
     // the queries of random sites, fewer of relaxed ones) costs the look.
+    // Not beside a crowd (a block of 27 K sites or more): the ball would be one
+    // for sites spread over the block, and its rows read the crowd in vain
+    // (65,000 sites, a fifth of them in one cell: 0.62 ms, 0.77 with the look).
     // About 45 keys then reach the list at K = 32, instead of 77: first tier at
     // 1M uniform sites 1.76 -> 1.45 ms, the rows of 64 of its deep sites 2.46
     // -> 1.83 ms, 60,000 points at K = 64 358 -> 314 us.
@@ -341,7 +344,7 @@ __global__ void __launch_bounds__(W * 32, 32 / W) k_knn(const float4* __restrict
         }
       }
       const int block = __reduce_add_sync(KFULL, nj);
-      if (block > 0) {
+      if (block > 0 && block < 27 * K) {
         // K + 2.2 sqrt(K) sites: two deviations above K when they are random
         const float want = (float)K + 2.2f * sqrtf((float)K);
         // (cells beyond the grid count as empty, as the ball's part there is)

@@ -29,3 +29,24 @@ def test_order_within_crowded_cells(pkg, n, sizes):
     kn.close()
     c = np.floor(p * np.float32(dim) / np.float32(1000.0)).astype(np.int64).clip(0, dim - 1)
     assert np.array_equal(perm, np.lexsort((np.arange(n), c[:, 0] + dim * (c[:, 1] + dim * c[:, 2]))))
+
+
+@pytest.mark.parametrize("k", [16, 32, 64])
+@pytest.mark.parametrize("n,sizes,width", [(20_000, [800, 900, 1500], 20.0), (20_000, [10_000], 0.5), (66_000, [30_000, 2000], 25.0)])
+def test_neighbours_beside_a_crowd(pkg, n, sizes, width, k):
+    """Queries in and around the crowds, on both sides of the line at 27 K sites
+    in a block, against brute force."""
+    pkg.build()
+    p = crowds(n, sizes, width, seed=k)
+    kn = pkg.KnProblem(p, k=k)
+    kn.solve()
+    perm, rows = kn.permutation().astype(np.int64), kn.knearests().astype(np.int64)
+    kn.close()
+    d = p.astype(np.float64)
+    _, block = np.unique(np.floor(d / 60.0), axis=0, return_inverse=True)
+    full = np.bincount(block)[block]
+    near = np.argsort(-full[perm], kind="stable")
+    for q in np.concatenate([near[::len(near) // 60], np.random.default_rng(1).choice(n, 40, replace=False)]):
+        d2 = ((d - d[perm[q]]) ** 2).sum(1)
+        d2[perm[q]] = np.inf
+        assert np.allclose(np.sort(d2[perm[rows[q]]]), np.sort(d2)[:k], rtol=1e-6, atol=0.0)
