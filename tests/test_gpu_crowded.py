@@ -50,3 +50,39 @@ def test_neighbours_beside_a_crowd(pkg, n, sizes, width, k):
         d2 = ((d - d[perm[q]]) ** 2).sum(1)
         d2[perm[q]] = np.inf
         assert np.allclose(np.sort(d2[perm[rows[q]]]), np.sort(d2)[:k], rtol=1e-6, atol=0.0)
+
+
+@pytest.mark.parametrize("n,sizes,width", [(6000, [3000], 2.0), (20_000, [6000, 200], 10.0), (30_000, [12_000], 0.5)])
+def test_cells_beside_a_crowd(pkg, meshgen, oracle, n, sizes, width):
+    """Cells that the K neighbours left open, completed by the 64-vertex pass or,
+    where the search spans the grid, by the 256-vertex pass, against the
+    oracle's exact cells.  Points are rounded to u = 2^-24 of a cell's radius R,
+    and further along the line that planes at a small angle nearly share: a cell
+    at the rim of a crowd is a needle sqrt(V / R) wide, with faces at that angle
+    over R, and its points are good to u R over the angle along it, which is
+    u R^3 / V of its volume, and of R for its barycentre."""
+    pkg.build()
+    P = meshgen.cube_problem(8, 10, seed=3)
+    sites = crowds(n, sizes, width, seed=n)
+    with pkg.Engine(P.verts, P.tets, sites, site_k=64, tet_k=20, exact=True) as e:
+        e.iterate(1, update=False)
+        vol, mom = e.moments()
+        _, ids = e.sites()
+        fl, st = e.buffer("site_flags"), e.stats()
+    v, m, f = np.empty_like(vol), np.empty_like(mom), np.empty_like(fl)
+    v[ids], m[ids], f[ids] = vol, mom, fl
+    done = np.flatnonzero((f & pkg.SITE_COMPLETED) != 0)
+    large = (f[done] & pkg.SITE_REDO) != 0
+    # (a few whose search a float cut ends, as for the 256-vertex pass alone, say so)
+    assert st["unresolved"] < 5 and large.any() and (~large).any()
+    # the largest of those at 256 vertices, and a sample of the others
+    q = np.concatenate([done[large][np.argsort(-v[done[large]])][:60], done[~large][:: max(1, (~large).sum() // 200)]])
+    r = oracle.complete_cells(sites, q, P.verts, P.tets, k0=256, kmax=16_384)
+    ok = r["complete"] & (r["vol"] > 0)  # (the oracle drops cells beyond its capacity)
+    assert ok.sum() > 60
+    vol, bary = r["vol"][ok], r["mom"][ok] / r["vol"][ok, None]
+    radius = np.cbrt(vol) + 2.0 * np.linalg.norm(bary - sites[q][ok], axis=1)
+    bound = np.maximum(1e-5, 2.0 ** -24 * radius ** 3 / vol)
+    assert (np.abs(v[q][ok] / vol - 1) / bound).max() < 1.0
+    off = np.linalg.norm(m[q][ok] / v[q][ok, None] - bary, axis=1)
+    assert (off / (radius * bound)).max() < 1.0
