@@ -104,6 +104,22 @@ __global__ void k_get_positions(const float4* __restrict__ sites, int n, float* 
   xyz[3 * i + 2] = p.z;
 }
 
+// The engine's device while an entry point that may be called with another one
+// current launches on its stream (a copy works from any device, a kernel launch
+// is refused).
+struct OnDevice {
+  int back = -1;
+  explicit OnDevice(int device) {
+    if (cudaGetDevice(&back) == cudaSuccess && back != device) cudaSetDevice(device);
+    else back = -1;
+  }
+  ~OnDevice() {
+    if (back >= 0) cudaSetDevice(back);
+  }
+  OnDevice(const OnDevice&) = delete;
+  OnDevice& operator=(const OnDevice&) = delete;
+};
+
 // Positions and ids in grid order; positions in input order.
 __global__ void k_get_sites(const float4* __restrict__ sites, int n, float* __restrict__ xyz, int* __restrict__ ids) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -769,6 +785,7 @@ int vgb_engine_copy_buffer(vgb_engine* e, int which, void* host, size_t bytes) {
 
 int vgb_engine_get_sites(vgb_engine* e, float* xyz, int* ids) {
   if (!e || !xyz) { set_error("NULL argument"); return VGB_ERR_INVALID; }
+  const OnDevice on(e->cfg.device);
   // packed on the device, then straight to the caller's arrays
   int* const d_ids = reinterpret_cast<int*>(e->sites_tmp);
   k_get_sites<<<(e->n + 255) / 256, 256, 0, e->st>>>(e->sites, e->n, e->io_stage, ids ? d_ids : nullptr);
@@ -781,6 +798,7 @@ int vgb_engine_get_sites(vgb_engine* e, float* xyz, int* ids) {
 
 int vgb_engine_get_sites_original(vgb_engine* e, float* xyz) {
   if (!e || !xyz) { set_error("NULL argument"); return VGB_ERR_INVALID; }
+  const OnDevice on(e->cfg.device);
   if (!e->bad_id) VGB_CUDA_TRY(cudaHostAlloc((void**)&e->bad_id, sizeof(int), cudaHostAllocMapped));
   *e->bad_id = 0;
   k_get_original<<<(e->n + 255) / 256, 256, 0, e->st>>>(e->sites, e->n, e->io_stage, e->bad_id);
