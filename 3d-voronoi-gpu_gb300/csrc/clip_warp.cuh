@@ -14,6 +14,7 @@
 
 #include "vgb_common.cuh"
 #include "exact_pred.cuh"
+#include "pair_float.cuh"
 
 namespace vgb {
 
@@ -63,44 +64,6 @@ __device__ __forceinline__ float3 vertex_of(float4 a, float4 b, float4 c) {
 // |x|^2, with the same rounding everywhere
 __device__ __forceinline__ float norm2_rn(float3 x) { return dot3_rn(x.x, x.y, x.z, x.x, x.y, x.z); }
 
-// Pairs of floats (h + l, 48 bits): products split by fma, sums by Knuth's
-// TwoSum, every operation rounded on its own.
-struct Pair {
-  float h, l;
-};
-__device__ __forceinline__ Pair pair_fast(float h, float l) {  // |h| >= |l|
-  const float s = __fadd_rn(h, l);
-  return {s, __fsub_rn(l, __fsub_rn(s, h))};
-}
-__device__ __forceinline__ Pair pair_sum(float a, float b) {
-  const float s = __fadd_rn(a, b), bv = __fsub_rn(s, a);
-  return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bv)), __fsub_rn(b, bv))};
-}
-__device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
-  const Pair s = pair_sum(a.h, b.h);
-  return pair_fast(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
-}
-__device__ __forceinline__ Pair pair_cross(float p, float q, float r, float t) {  // p q - r t
-  const float a = __fmul_rn(p, q), b = __fmul_rn(r, t);
-  const float ea = __fmaf_rn(p, q, -a), eb = __fmaf_rn(r, t, -b);
-  const Pair s = pair_sum(a, -b);
-  return pair_fast(s.h, __fadd_rn(s.l, __fsub_rn(ea, eb)));
-}
-__device__ __forceinline__ Pair pair_mul(float a, Pair b) {
-  const float p = __fmul_rn(a, b.h);
-  return pair_fast(p, __fmaf_rn(a, b.l, __fmaf_rn(a, b.h, -p)));
-}
-__device__ __forceinline__ Pair pair_dot(float a0, float a1, float a2, Pair b0, Pair b1, Pair b2) {
-  return pair_add(pair_add(pair_mul(a0, b0), pair_mul(a1, b1)), pair_mul(a2, b2));
-}
-// -n / d, with r near 1 / d.h
-__device__ __forceinline__ float pair_ratio(Pair n, Pair d, float r) {
-  const float q = __fmul_rn(n.h, r), p = __fmul_rn(q, d.h);
-  const float e = __fmaf_rn(q, d.h, -p);
-  const float rest = __fadd_rn(__fsub_rn(__fsub_rn(n.h, p), e), __fmaf_rn(-q, d.l, n.l));
-  return -__fmaf_rn(rest, r, q);
-}
-
 // Robust-predicate variants (the ROBUST instantiations of the clips).  A
 // vertex-vs-plane test is decided in float unless |P(v)| lies within
 // ROBUST_BAND of the sum of its terms' magnitudes; such a test is decided
@@ -112,39 +75,6 @@ __device__ __forceinline__ float pair_ratio(Pair n, Pair d, float r) {
 // determinant cancels, so new vertices are computed in double.  The exact
 // and double paths are out of line.
 constexpr float ROBUST_BAND = 1e-4f;
-
-// Sign of P at the vertex of A, B, C where pairs of floats tell it: with
-// V = -num / det (Cramer), the sign of det (P.w det - P.n num), each factor's
-// error below 2^-44 of the sum T of its terms' magnitudes; 0 when either is
-// within 2^-40 of T.  (Sites from a lattice are cospherical up to the rounding
-// of their positions, 2^-24: all but the exactly degenerate tests end here,
-// for 450 FP32 operations instead of some thousands in FP64.)
-__device__ __forceinline__ int pair_side(float4 a, float4 b, float4 c, float4 P) {
-  const Pair bcx = pair_cross(b.y, c.z, b.z, c.y), bcy = pair_cross(b.z, c.x, b.x, c.z),
-             bcz = pair_cross(b.x, c.y, b.y, c.x);
-  const Pair cax = pair_cross(c.y, a.z, c.z, a.y), cay = pair_cross(c.z, a.x, c.x, a.z),
-             caz = pair_cross(c.x, a.y, c.y, a.x);
-  const Pair abx = pair_cross(a.y, b.z, a.z, b.y), aby = pair_cross(a.z, b.x, a.x, b.z),
-             abz = pair_cross(a.x, b.y, a.y, b.x);
-  auto m = [](float p, float q, float r, float t) { return fabsf(p * q) + fabsf(r * t); };
-  const float mbx = m(b.y, c.z, b.z, c.y), mby = m(b.z, c.x, b.x, c.z), mbz = m(b.x, c.y, b.y, c.x);
-  const float mcx = m(c.y, a.z, c.z, a.y), mcy = m(c.z, a.x, c.x, a.z), mcz = m(c.x, a.y, c.y, a.x);
-  const float max_ = m(a.y, b.z, a.z, b.y), may = m(a.z, b.x, a.x, b.z), maz = m(a.x, b.y, a.y, b.x);
-  const Pair det = pair_dot(a.x, a.y, a.z, bcx, bcy, bcz);
-  const float md = fabsf(a.x) * mbx + fabsf(a.y) * mby + fabsf(a.z) * mbz;
-  const Pair nx = pair_dot(a.w, b.w, c.w, bcx, cax, abx), ny = pair_dot(a.w, b.w, c.w, bcy, cay, aby),
-             nz = pair_dot(a.w, b.w, c.w, bcz, caz, abz);
-  const float aw = fabsf(a.w), bw = fabsf(b.w), cw = fabsf(c.w);
-  const Pair pn = pair_dot(P.x, P.y, P.z, nx, ny, nz), pd = pair_mul(P.w, det);
-  const Pair D = pair_add(pd, Pair{-pn.h, -pn.l});
-  const float T = fabsf(P.w) * md + fabsf(P.x) * (aw * mbx + bw * mcx + cw * max_) +
-                  fabsf(P.y) * (aw * mby + bw * mcy + cw * may) + fabsf(P.z) * (aw * mbz + bw * mcz + cw * maz);
-  constexpr float eps = 1.f / (1048576.f * 1048576.f);  // 2^-40
-  // (1e-20: the low parts must stay clear of underflow)
-  if (!(fabsf(D.h) > eps * T && fabsf(det.h) > eps * md && fabsf(D.h) > 1e-20f && fabsf(det.h) > 1e-20f && T < 1e35f))
-    return 0;
-  return (D.h > 0.f) == (det.h > 0.f) ? 1 : -1;
-}
 
 static __device__ __noinline__ bool exact_outside(float4 A, float4 B, float4 C, float4 P) {
   const int side = pair_side(A, B, C, P);
@@ -178,29 +108,11 @@ static __device__ __noinline__ float3 vertex_of_d(float4 a, float4 b, float4 c) 
 // The robust variants compute every new vertex beyond float: a float vertex
 // from planes that nearly share a line carries an error up to its condition
 // number times float rounding, enough to put a later float test on the wrong
-// side of the exact band.  Pairs of floats carry it to about 2^-46 of its
-// terms' size; when the determinant is more than 2^-12 of the sum of its
-// terms (and far from underflow), that is 2^-34 of the vertex's distance,
-// below the rounding to float that follows as it does in double.  Otherwise
-// (one vertex in a thousand) in double.  GB300 issues 64 FP32 operations for
-// one in FP64: the vertex takes about 350 instead of 65 x 64.
+// side of the exact band.  Where pairs of floats do not give each coordinate to
+// its own rounding (a few vertices in a thousand), in double.
 __device__ __forceinline__ float3 vertex_of_robust(float4 a, float4 b, float4 c) {
-  const Pair bcx = pair_cross(b.y, c.z, b.z, c.y), bcy = pair_cross(b.z, c.x, b.x, c.z),
-             bcz = pair_cross(b.x, c.y, b.y, c.x);
-  const Pair det = pair_dot(a.x, a.y, a.z, bcx, bcy, bcz);
-  const float mag = fabsf(a.x) * (fabsf(b.y * c.z) + fabsf(b.z * c.y)) +
-                    fabsf(a.y) * (fabsf(b.z * c.x) + fabsf(b.x * c.z)) +
-                    fabsf(a.z) * (fabsf(b.x * c.y) + fabsf(b.y * c.x));
-  const float ad = fabsf(det.h);
-  if (!(ad > mag * (1.f / 4096.f) && ad > 1e-22f && ad < 1e30f)) return vertex_of_d(a, b, c);
-  const Pair cax = pair_cross(c.y, a.z, c.z, a.y), cay = pair_cross(c.z, a.x, c.x, a.z),
-             caz = pair_cross(c.x, a.y, c.y, a.x);
-  const Pair abx = pair_cross(a.y, b.z, a.z, b.y), aby = pair_cross(a.z, b.x, a.x, b.z),
-             abz = pair_cross(a.x, b.y, a.y, b.x);
-  const float r = __frcp_rn(det.h);
-  return make_float3(pair_ratio(pair_dot(a.w, b.w, c.w, bcx, cax, abx), det, r),
-                     pair_ratio(pair_dot(a.w, b.w, c.w, bcy, cay, aby), det, r),
-                     pair_ratio(pair_dot(a.w, b.w, c.w, bcz, caz, abz), det, r));
+  float3 x;
+  return pair_vertex(a, b, c, x) ? x : vertex_of_d(a, b, c);
 }
 
 // Plane through three points, normal (p1-p0)x(p2-p0): positive inside a
