@@ -309,6 +309,7 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
   const unsigned lane_bit = 1u << lane, lt_mask = lane_bit - 1u;
   if (lane < WC_N) S.cnt[lane] = 0u;
   const bool exact = CELL_TET && tet_order != nullptr;
+#define MISS_BY_PIECE (CELL_TET && !exact && store.flags == nullptr)
   __syncwarp();
 
   // The sites in_list names (in_count of them), or every site.  A site whose
@@ -1010,7 +1011,11 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
           for (int k = 0; k < SL; ++k)
             if (c.vm[k] & lane_bit) lm = fmaxf(lm, c.vw[k]);
           lm = warp_max_nonneg(lm);
-          if (lane == 0) S.pr2 = fmaxf(S.pr2, lm);
+          if (lane == 0) {
+            S.pr2 = fmaxf(S.pr2, lm);
+            // (a site of the tet-cell method: its misses are its pieces')
+            if (MISS_BY_PIECE && !(2.f * S.plane[4 + K - 1].w > 4.f * lm)) S.cnt[WC_SECMISS]++;
+          }
         }
         float vol, mx, my, mz;
         warp_moments(c, S.plane, lane, vol, mx, my, mz);
@@ -1070,7 +1075,7 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
           }
         }
         if (store.flags) store.flags[s] = (unsigned char)f;
-        if (!COMPLETE && (f & SITE_SECMISS)) {
+        if (!COMPLETE && (f & SITE_SECMISS) && !MISS_BY_PIECE) {
           S.cnt[WC_SECMISS]++;
           if (prob_secmiss) atomicAdd(prob_secmiss + pidx, 1u);
         }
@@ -1080,6 +1085,7 @@ __global__ void __launch_bounds__(CLIP_WARPS * WARP, SL >= 8 ? 2 : ROBUST ? VGB_
     __syncwarp();
 #undef PD
   }
+#undef MISS_BY_PIECE
   if (stats && lane < WC_N && S.cnt[lane]) atomicAdd(stats + stat_slot(lane), (unsigned long long)S.cnt[lane]);
 }
 
@@ -1740,10 +1746,10 @@ struct ClipPasses {
   // the 96-vertex fast pass lone / batched, the pieces pass lone / batched,
   // and of the float exact form the mesh pass, the one-warp pass and the
   // completion pass that hand on to it, lone / batched each, then the mesh
-  // pass of the reference form, and the completion pass of 64 vertices, lone
-  // / batched
+  // pass of the reference form, the completion pass of 64 vertices, lone /
+  // batched, and the mesh pass of the tet-cell method
   static int* resident() {
-    static int r[20] = {};
+    static int r[21] = {};
     return r;
   }
   static int prepare();
@@ -1779,6 +1785,7 @@ int ClipPasses<R>::prepare() {
     if (resident_blocks(k_cell_mesh<false, false>, sms, r + 11) ||
         resident_blocks(k_cell_mesh<true, false>, sms, r + 12) ||
         resident_blocks(k_cell_mesh<false, true>, sms, r + 17) ||
+        resident_blocks(k_cell_mesh<false, true, true>, sms, r + 20) ||
         resident_blocks(k_clip_site<true, false, SLOTS_FAST, false, false, true>, sms, r + 13) ||
         resident_blocks(k_clip_site<true, true, SLOTS_FAST, false, false, true>, sms, r + 14) ||
         resident_blocks(k_clip_site<true, false, SLOTS_FAST, false, true, true>, sms, r + 18) ||
@@ -1940,7 +1947,8 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
               prob_secmiss, in_list, in_count, work, redo, counters + (last ? 16 : 1), cs, last ? nullptr : esc,
               esc_r2, counters + 10, site_start);
         };
-        if (ref_mesh) go(k_cell_mesh<false, true>, 17);
+        if (ref_mesh && !cell_tet) go(k_cell_mesh<false, true, true>, 20);
+        else if (ref_mesh) go(k_cell_mesh<false, true>, 17);
         else if (probs) go(k_cell_mesh<true, false>, 12);
         else go(k_cell_mesh<false, false>, 11);
       };

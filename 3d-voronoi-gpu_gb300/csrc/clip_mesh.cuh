@@ -108,6 +108,8 @@ struct MeshSmem {
   int queue[2 * WARP];  // tets whose sphere meets the cell's
   int rng[2][WARP];     // the rows in hand: first tet, tets of the rows before
   unsigned cnt[WC_N];
+  unsigned here[WC_N], spare[WC_N];  // of the site in hand; of its second sum (not counted)
+  unsigned tr2[MESH_TETS];           // tet-cell method: how far each tet's piece reaches (squared, float bits)
 };
 
 // dot product ending in + c, the same rounding in every kernel
@@ -232,8 +234,9 @@ __device__ __forceinline__ bool face_side(unsigned info, int i) { return ((info 
 
 // REF (reference form): a site's sum is over the tets it is a candidate of
 // (one of the tet_k nearest sites of their centroid), and the face between
-// such a tet and one it is no candidate of is open.
-template <bool BATCHED, bool REF>
+// such a tet and one it is no candidate of is open.  PAIRS (tet-cell method): the
+// counter of misses is of its pieces, not of cells.
+template <bool BATCHED, bool REF, bool PAIRS = false>
 __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell_mesh(
     const float4* __restrict__ sites, const unsigned* __restrict__ knn, const ProbDesc* __restrict__ probs,
     const int* __restrict__ site_prob, const ProbDesc lone, const float4* __restrict__ rec,
@@ -265,7 +268,8 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
     const int K = PD(K);
     const unsigned* const krow = knn + PD(knn_off) + (size_t)(s - PD(site_off)) * K;
     const bool miss = (flags & SITE_SECMISS) && !(flags & SITE_COMPLETED);
-    const float dK2 = miss && !REF ? dist2(seed, sites[krow[K - 1]]) : FLT_MAX;
+    const float dK2 = miss && (!REF || PAIRS) ? dist2(seed, sites[krow[K - 1]]) : FLT_MAX;
+    if (lane < WC_N) S.here[lane] = 0u;
 
     // -----------------------------------------------------------------
     // the cell: its faces, vertices and edges
@@ -388,7 +392,6 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
       const float d2 = dist2(tet_sph[q], seed);
       return d2 < z.x || (d2 == z.x && site_id(seed) <= __float_as_int(z.y));
     };
-    int nclip = 0;
     const float h = 1000.f / (float)dim;
     // (the cell of a coordinate up to its rounding, well below the margins)
     const float per = __fmul_rn((float)dim, 1e-3f);
@@ -401,6 +404,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
     for (bool again = false; !bad;) {
       MeshSum sum;
       float far2 = 0.f;
+      unsigned* const here = again ? S.spare : S.here;
       int skew = 0;  // ends of crossing edges, less the faces' slots they took
       // a piece [a, b] of an edge: k = det(F1 - F0, p, u) (b - a), and the
       // moment k1 (F1 + a + b) - k0 (F0 + a + b), all relative to X
@@ -491,7 +495,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
           const unsigned m = __ballot_sync(FULL, meets);
           if (meets) S.queue[nq + __popc(m & lt_mask)] = idx;
           nq += __popc(m);
-          if (!REF && lane == 0) S.cnt[WC_CAND] += (unsigned)min(WARP, total - f0);
+          if (!REF && lane == 0) here[WC_CAND] += (unsigned)min(WARP, total - f0);
           f0 += WARP;
         }
         if (nq == 0) break;
@@ -515,13 +519,16 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
                      A2 = make_float3(r1.z, r1.w, r2.x), A3 = make_float3(r2.y, r2.z, r2.w);
         const float3 sd = make_float3(seed.x, seed.y, seed.z);
         const float3 c0 = sub_rn(A0, sd), c1 = sub_rn(A1, sd), c2 = sub_rn(A2, sd), c3 = sub_rn(A3, sd);
+        unsigned tests = 0u;
 #pragma unroll 2
         for (int f = 0; f < nf; ++f) {
           if (!__any_sync(FULL, alive)) break;
+          tests += alive;
           const float4 P = S.plane[f];
           const float e = fmaxf(fmaxf(eval4(P, c0), eval4(P, c1)), fmaxf(eval4(P, c2), eval4(P, c3)));
           alive &= !(e < 0.f);
         }
+        const unsigned tested = __reduce_add_sync(FULL, tests);
         const unsigned am = __ballot_sync(FULL, alive);
         const int nb = min(__popc(am), MESH_TETS), place = __popc(am & lt_mask);
         // the rest of the queue to its front, then what is more than can be
@@ -534,10 +541,9 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
         alive &= place < MESH_TETS;
         nq = rest + __popc(am) - nb;
         if (lane == 0) {
-          if (!REF) S.cnt[WC_CULLED] += (unsigned)(take - __popc(am));
-          if (!REF) S.cnt[WC_CLIPPED] += (unsigned)nb;
-          S.cnt[WC_CULLTESTS] += (unsigned)(take * nf);
-          S.cnt[WC_CONFLICT] += (unsigned)(8 * ne * nb);
+          here[WC_CLIPPED] += (unsigned)nb;
+          here[WC_CULLTESTS] += tested;
+          here[WC_CONFLICT] += (unsigned)(8 * ne * nb);
         }
         if (alive) {
           const int pos = place;
@@ -550,7 +556,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
           face(2, A0, A1, A3, c0);
           face(3, A0, A1, A2, c0);
           unsigned far = 0u;
-          if (miss && !REF) {
+          if (miss && (!REF || PAIRS)) {
             const float m2 = fmaxf(fmaxf(dot_rn(c0, c0), dot_rn(c1, c1)), fmaxf(dot_rn(c2, c2), dot_rn(c3, c3)));
             far = !(dK2 > __fmaf_rn(4.f * m2, 1.0001f, 1e-4f)) ? 64u : 0u;
           }
@@ -564,6 +570,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
           }
           S.tinf[pos] = (unsigned char)((info & 31u) | far);
           S.thit[pos] = 0;
+          if (PAIRS) S.tr2[pos] = 0u;
         }
         __syncwarp();
 
@@ -575,7 +582,8 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
           for (int w = lane; w < nb * ne; w += WARP) {
             const float4 ep = S.epos[e], eu = S.edir[e];
             const float3 p = xyz(ep), u = xyz(eu);
-            const bool even = (S.tinf[b] & REC_EVEN) != 0u;  // sides: -, +, -, + of an even tet
+            const unsigned inf = S.tinf[b];
+            const bool even = (inf & REC_EVEN) != 0u;  // sides: -, +, -, + of an even tet
             float lo = ep.w, hi = eu.w;
             bool up;
             float t = line_at(S.tp[b][0], p, u, up);
@@ -592,8 +600,10 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
               sum.add(k, __fmaf_rn(km, u.x, __fmul_rn(d, T4.x)), __fmaf_rn(km, u.y, __fmul_rn(d, T4.y)),
                       __fmaf_rn(km, u.z, __fmul_rn(d, T4.z)));
               sum.close(__fmul_rn(d, S.eopen[e]));
-              far2 = fmaxf(far2, __fadd_rn(dot_rn(p, p), fmaxf(lo * lo, hi * hi)));
+              const float r2 = __fadd_rn(dot_rn(p, p), fmaxf(lo * lo, hi * hi));
+              far2 = fmaxf(far2, r2);
               S.thit[b] = 1;
+              if (PAIRS && (inf & 64u)) atomicMax(S.tr2 + b, __float_as_uint(r2));
             }
             b += db;
             e += de;
@@ -604,24 +614,11 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
           }
         }
         __syncwarp();
-        const unsigned hits = __ballot_sync(FULL, lane < nb && S.thit[lane & (MESH_TETS - 1)] != 0);
-        const unsigned farm = __ballot_sync(FULL, lane < nb && (S.tinf[lane & (MESH_TETS - 1)] & 64u) != 0u);
-        unsigned open = __ballot_sync(FULL, lane < nb && (S.tinf[lane & (MESH_TETS - 1)] & 15u) != 0u);
-        nclip += nb;
-        if (lane == 0) {
-          S.cnt[WC_CONTRIB] += (unsigned)__popc(hits);
-          S.cnt[WC_EMPTY] += (unsigned)(nb - __popc(hits));
-        }
         const float3 site = make_float3(seed.x, seed.y, seed.z);
-        // the tets reaching beyond half the K-th neighbour's distance, of a
-        // cell its K neighbours left open: how far their pieces reach (the
-        // tets' edges, one per lane; the cell's edges are in far2)
-        if ((farm >> lane) & 1u) S.thit[__popc(farm & lt_mask)] = (unsigned char)lane;
-        __syncwarp();
-#pragma unroll 1
-        for (int w = lane; w < 6 * __popc(farm); w += WARP) {
-          const int e = w % 6;
-          const float4* q = rec + 4 * (size_t)S.tidx[S.thit[w / 6]];
+        // the part of edge e (0-5) of tet b inside the cell: how far it reaches
+        // (squared, below zero where there is none)
+        auto tet_edge = [&](int b, int e) {
+          const float4* q = rec + 4 * (size_t)S.tidx[b];
           const float4 r0 = q[0], r1 = q[1], r2 = q[2];
           const float3 c0 = make_float3(r0.x, r0.y, r0.z), c1 = make_float3(r0.w, r1.x, r1.y),
                        c2 = make_float3(r1.z, r1.w, r2.x), c3 = make_float3(r2.y, r2.z, r2.w);
@@ -634,8 +631,41 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
             const float t = line_at(S.plane[f], L.p, L.u, up);
             if (up) lo = fmaxf(lo, t); else hi = fminf(hi, t);
           }
-          if (hi > lo) far2 = fmaxf(far2, __fadd_rn(dot_rn(L.p, L.p), fmaxf(lo * lo, hi * hi)));
+          return hi > lo ? __fadd_rn(dot_rn(L.p, L.p), fmaxf(lo * lo, hi * hi)) : -1.f;
+        };
+        if (PAIRS && miss) {
+          // the pieces that reach beyond half the K-th neighbour's distance (of
+          // tets that do, alone)
+          const unsigned reach = __ballot_sync(FULL, lane < nb && (S.tinf[lane & (MESH_TETS - 1)] & 64u) != 0u);
+#pragma unroll 1
+          for (int w = lane; w < 6 * nb; w += WARP) {
+            const int b = w / 6;
+            const float r2 = (reach >> b) & 1u ? tet_edge(b, w - 6 * b) : -1.f;
+            if (r2 >= 0.f) {
+              S.thit[b] = 1;
+              atomicMax(S.tr2 + b, __float_as_uint(r2));
+            }
+          }
+          __syncwarp();
+          const unsigned beyond_k = __ballot_sync(
+              FULL, ((reach >> lane) & 1u) && S.thit[lane & (MESH_TETS - 1)] != 0 &&
+                        !(dK2 > 4.f * __uint_as_float(S.tr2[lane & (MESH_TETS - 1)])));
+          if (lane == 0) here[WC_SECMISS] += (unsigned)__popc(beyond_k);
         }
+        const unsigned hits = __ballot_sync(FULL, lane < nb && S.thit[lane & (MESH_TETS - 1)] != 0);
+        const unsigned farm = REF ? 0u : __ballot_sync(FULL, lane < nb && (S.tinf[lane & (MESH_TETS - 1)] & 64u) != 0u);
+        unsigned open = __ballot_sync(FULL, lane < nb && (S.tinf[lane & (MESH_TETS - 1)] & 15u) != 0u);
+        if (lane == 0) {
+          here[WC_CONTRIB] += (unsigned)__popc(hits);
+          here[WC_EMPTY] += (unsigned)(nb - __popc(hits));
+        }
+        // the tets reaching beyond half the K-th neighbour's distance, of a
+        // cell its K neighbours left open: how far their pieces reach (the
+        // tets' edges, one per lane; the cell's edges are in far2)
+        if ((farm >> lane) & 1u) S.thit[__popc(farm & lt_mask)] = (unsigned char)lane;
+        __syncwarp();
+#pragma unroll 1
+        for (int w = lane; w < 6 * __popc(farm); w += WARP) far2 = fmaxf(far2, tet_edge(S.thit[w / 6], w % 6));
 
         for (; open != 0u; open &= open - 1u) {
           const int b = __ffs(open) - 1;
@@ -809,12 +839,16 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
       continue;
     }
     if (lane < 4) reinterpret_cast<double*>(mom + s)[lane] = moment;
-    if (REF && lane == 0) {
-      const unsigned nc = (unsigned)(site_start[s + 1] - site_start[s]);
-      S.cnt[WC_CAND] += nc;
-      S.cnt[WC_CLIPPED] += min((unsigned)nclip, nc);
-      S.cnt[WC_CULLED] += nc - min((unsigned)nclip, nc);
+    // (counted now that the site is done here; a cell that is given back is
+    // counted by the pass that takes it)
+    if (lane == 0) {
+      const unsigned nc = REF ? (unsigned)(site_start[s + 1] - site_start[s]) : S.here[WC_CAND];
+      S.here[WC_CAND] = nc;
+      S.here[WC_CULLED] = nc - min(S.here[WC_CLIPPED], nc);
     }
+    __syncwarp();
+    if (lane < WC_N) S.cnt[lane] += S.here[lane];
+    __syncwarp();
     if (lane == 0) {
       unsigned f = flags | SITE_HANDED;
       if (beyond) {
@@ -824,7 +858,7 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
         f |= SITE_UNRESOLVED;
       }
       if (miss) {
-        S.cnt[WC_SECMISS]++;
+        if (!PAIRS) S.cnt[WC_SECMISS]++;
         if (prob_secmiss) atomicAdd(prob_secmiss + pidx, 1u);
       }
       if (flags & SITE_COMPLETED) S.cnt[WC_COMPLETED]++;

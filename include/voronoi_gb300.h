@@ -50,22 +50,23 @@ enum vgb_stat {
   VGB_STAT_CLIPPED = 2,         /* run through the full clip                          */
   VGB_STAT_EMPTY = 3,           /* clipped to nothing (mesh pass: no edge of the cell in it) */
   VGB_STAT_CONTRIB = 4,         /* contributed volume (mesh pass: an edge of the cell in it) */
-  VGB_STAT_SECURITY_MISS = 5,   /* contributed without reaching the security radius
-                                   (mesh pass: cells, otherwise pairs in the tet-cell
-                                   method)                                            */
+  VGB_STAT_SECURITY_MISS = 5,   /* contributed without reaching the security radius:
+                                   cells, in the tet-cell method pairs                */
   VGB_STAT_TRI_OVERFLOW = 6,    /* dropped: more cell vertices than the capacity      */
   VGB_STAT_BOUNDARY_FAIL = 7,   /* dropped: cavity boundary not one loop              */
   VGB_STAT_PLANES = 8,          /* bisector planes applied                            */
   VGB_STAT_CLIPS = 9,           /* planes that removed a vertex                       */
-  VGB_STAT_FINAL_VERTICES = 10, /* cell vertices decomposed into sub-tets             */
+  VGB_STAT_FINAL_VERTICES = 10, /* cell vertices decomposed into sub-tets (the mesh pass
+                                   decomposes none: it sums over edges)               */
   VGB_STAT_CONFLICT_TESTS = 11, /* vertex-vs-plane tests while clipping               */
   VGB_STAT_CULL_TESTS = 12,     /* tet-vs-plane tests of the separation pass          */
   VGB_STAT_NEW_VERTICES = 13,   /* vertices created by clipping                       */
   VGB_STAT_INTERIOR = 14,       /* sites whose whole cell lies inside the mesh        */
   VGB_STAT_REDO = 15,           /* sites redone at 128 vertices (outgrew 64, or left a
                                    sliver to the mesh pass)                           */
-  VGB_STAT_NEEDS_EXACT = 16,    /* robust_predicates: vertex-vs-plane tests decided by
-                                   the exact determinants (the reference's status
+  VGB_STAT_NEEDS_EXACT = 16,    /* robust_predicates: vertex-vs-plane tests too close to
+                                   zero for float, decided by pairs of floats or the
+                                   exact determinants (the reference's status
                                    needs_exact_predicates, voronoi_defs.h:10)          */
   VGB_STAT_COMPLETED = 17,      /* exact form: sites whose K neighbours left their cell
                                    unresolved, completed by every site within twice the
