@@ -592,7 +592,7 @@ int vgb_batch_shape(const vgb_batch* b, int* knn_warps, int* build_lanes, int* f
   if (knn_warps) *knn_warps = b->shape.knn_warps;
   if (build_lanes) *build_lanes = b->shape.build_g;
   if (fast_slots) *fast_slots = b->shape.fast_sl;
-  if (tet_pieces) *tet_pieces = b->shape.pieces;
+  if (tet_pieces) *tet_pieces = b->store.rec ? 0 : b->shape.pieces;  // (the mesh pass has no pieces)
   return VGB_OK;
 }
 

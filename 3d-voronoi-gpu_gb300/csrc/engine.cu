@@ -854,7 +854,7 @@ int vgb_engine_shape(vgb_engine* e, int* knn_warps, int* build_lanes, int* fast_
   if (knn_warps) *knn_warps = e->shape.knn_warps;
   if (build_lanes) *build_lanes = e->shape.build_g;
   if (fast_slots) *fast_slots = e->shape.fast_sl;
-  if (tet_pieces) *tet_pieces = e->shape.pieces;
+  if (tet_pieces) *tet_pieces = e->store.rec ? 0 : e->shape.pieces;  // (the mesh pass has no pieces)
   return VGB_OK;
 }
 

@@ -233,8 +233,9 @@ int vgb_engine_info(vgb_engine* e, int* n_site, int* n_tet, int* site_k, int* te
 
 /* Launch shapes in use (autotuned with cfg.autotune): warps per kNN block,
  * lanes per site in the first clip pass, triangle slots per lane of the
- * one-warp clip pass (32 x slots vertices), and the clip form (1: pieces
- * built from their tets, 0: copies of the cell clipped by each tet; see
+ * one-warp clip pass (32 x slots vertices), and the clip form in use (1: pieces
+ * built from their tets, 0: copies of the cell clipped by each tet, or neither,
+ * where a cell's edges and the mesh's open triangles are summed; see
  * vgb_config.tet_pieces).  Any pointer may be NULL. */
 int vgb_engine_shape(vgb_engine* e, int* knn_warps, int* build_lanes, int* fast_slots, int* tet_pieces);
 
