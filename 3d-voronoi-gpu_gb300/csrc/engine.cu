@@ -489,7 +489,7 @@ int vgb_engine_create(vgb_engine** out, const vgb_config* cfg_in, const float* v
   size_t pairs = (size_t)n_tet * e->tk;
   const bool exact_form = cfg.method == VGB_METHOD_CELL_TET && cfg.exact;
   const bool mesh_form = cfg.method != VGB_METHOD_PLAIN &&
-                         runs_mesh_pass(cfg.robust_predicates != 0, cfg.tet_pieces != 0, n_tet, n_site);
+                         runs_mesh_pass(cfg.robust_predicates != 0, exact_form && cfg.tet_pieces != 0, n_tet, n_site);
   size_t scan_n = std::max((size_t)e->ncell + 1, (size_t)n_site + 1);
   if ((rc = dalloc(&e->verts, n_vert)) || (rc = dalloc(&e->tets, n_tet)) || (rc = dalloc(&e->sites, n_site)) ||
       (rc = dalloc(&e->sites_tmp, n_site)) || (rc = dalloc(&e->cell_start, e->ncell + 1)) ||

@@ -309,16 +309,17 @@ constexpr int PIECE_REC = 4 + PIECE_FACES / 4;
 constexpr int MESH_VERTS = 64;
 constexpr int MESH_EXT = PIECE_REC;
 
-// Whether a problem (or batch) runs the mesh pass (clip_mesh.cuh): the exact
-// form and the reference forms do, with float predicates.  It is faster than
+// Whether a problem (or batch, by its totals) runs the mesh pass (clip_mesh.cuh):
+// with float predicates all forms but the plain method do.  It is faster than
 // clipping by each tet at every size and mesh measured (Lloyd iteration with
 // nothing else changed, us: 20k sites in 48k tets 610 -> 290, 100k in 6 tets
-// 1,955 -> 1,020, 1M in 1.96M 10,100 -> 7,400); the
-// pieces pass is left to callers who ask for it on a mesh of fewer than a tet
-// per 256 sites, where its pieces outgrow their lane groups and the counters
-// say so (3,000 sites in 6 tets: 350 us, with the mesh pass 280).
-inline bool runs_mesh_pass(bool robust, bool tet_pieces, long long n_tet, long long n_site) {
-  return !robust && !(tet_pieces && n_tet * 256 < n_site);
+// 1,955 -> 1,020, 1M in 1.96M 10,100 -> 7,400).  The pieces pass, slower on such a
+// mesh as well (3,000 sites in 6 tets: 409 us, with the mesh pass 238), runs only
+// where the exact form's option asks for it by name on fewer than a tet per 256
+// sites: what callers read from it there is how many pieces outgrow their lane
+// groups (VGB_STAT_REDO), which the mesh pass has no like of.
+inline bool runs_mesh_pass(bool robust, bool exact_pieces, long long n_tet, long long n_site) {
+  return !robust && !(exact_pieces && n_tet * 256 < n_site);
 }
 
 // Counters of the clip passes (clip_kernels.cuh lists them).
