@@ -97,9 +97,6 @@ constexpr int BOX_PLANES = 6;
 #ifndef VGB_ROBUST_MIN_BLOCKS
 #define VGB_ROBUST_MIN_BLOCKS 6
 #endif
-#ifndef VGB_BUILD_MIN_BLOCKS_BATCHED
-#define VGB_BUILD_MIN_BLOCKS_BATCHED 7
-#endif
 
 enum WarpCount : int {
   WC_CAND = 0, WC_CULLED, WC_CLIPPED, WC_EMPTY, WC_CONTRIB, WC_SECMISS, WC_OVERFLOW, WC_BOUNDARY, WC_PLANES,
@@ -1513,7 +1510,7 @@ __host__ __device__ constexpr int build_plane_stride(int kmax) { return 4 + kmax
 // counter independently; a warp's groups run one instruction stream, a
 // group whose cell is done passing its turn in each clip.
 template <bool BATCHED, int G, int SL, bool ROBUST>
-__global__ void __launch_bounds__(CLIP_WARPS * WARP, ROBUST ? VGB_ROBUST_MIN_BLOCKS : BATCHED ? VGB_BUILD_MIN_BLOCKS_BATCHED : VGB_BUILD_MIN_BLOCKS) k_build(
+__global__ void __launch_bounds__(CLIP_WARPS * WARP, ROBUST ? VGB_ROBUST_MIN_BLOCKS : VGB_BUILD_MIN_BLOCKS) k_build(
     const float4* __restrict__ sites, int n, const unsigned* __restrict__ knn, const ProbDesc* __restrict__ probs,
     const int* __restrict__ site_prob, const ProbDesc lone, dmom4* __restrict__ mom,
     unsigned long long* __restrict__ stats, const unsigned char* __restrict__ field,
@@ -1770,8 +1767,9 @@ int ClipPasses<R>::prepare() {
   VGB_CUDA_TRY(cudaGetDevice(&dev));
   VGB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   int* r = resident();
-  if (resident_blocks(k_clip_site<false, false, SLOTS_TET_CELL, R>, sms, r + 0) ||
-      resident_blocks(k_clip_site<true, false, SLOTS_FAST, R>, sms, r + 1) ||
+  if constexpr (R)  // (with float predicates the mesh pass does the tet-cell method)
+    if (resident_blocks(k_clip_site<false, false, SLOTS_TET_CELL, true>, sms, r + 0)) return -2;
+  if (resident_blocks(k_clip_site<true, false, SLOTS_FAST, R>, sms, r + 1) ||
       resident_blocks(k_clip_site<true, false, SLOTS_REDO, R>, sms, r + 2) ||
       resident_blocks(k_clip_site<true, true, SLOTS_FAST, R>, sms, r + 3) ||
       resident_blocks(k_clip_site<true, true, SLOTS_REDO, R>, sms, r + 4) ||
@@ -1835,7 +1833,7 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
   }
   const bool ref_mesh = !R && store.rec != nullptr && store.last != nullptr;
   int* const g_clip_resident_blocks = resident();
-  if (g_clip_resident_blocks[0] == 0 && prepare()) return -2;
+  if (g_clip_resident_blocks[1] == 0 && prepare()) return -2;
   if (!cell_tet && probs) {
     set_error("the tet-cell method runs one problem at a time");
     return -1;
@@ -1845,14 +1843,19 @@ int ClipPasses<R>::run(bool cell_tet, const float4* sites, int n, unsigned* knn,
     return -1;
   }
   if (!cell_tet && !ref_mesh) {
-    // a few waves of resident blocks, sites dealt round-robin
-    const long long want = (long long)g_clip_resident_blocks[0] * 4, need = (n + CLIP_WARPS - 1) / CLIP_WARPS;
-    k_clip_site<false, false, SLOTS_TET_CELL, R><<<(int)(want < need ? want : need), CLIP_WARPS * WARP, 0, st>>>(
-        sites, n, knn, probs, site_prob, lone, verts, tets, site_start, site_tets, mom, stats, nullptr, nullptr,
-        nullptr, nullptr, nullptr, nullptr, nullptr, prob_secmiss, nullptr, nullptr, nullptr, nullptr, nullptr,
-        CellStore{}, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
-    VGB_CUDA_TRY(cudaGetLastError());
-    return 0;
+    if constexpr (!R) {
+      set_error("the tet-cell method needs its tet records");
+      return -1;
+    } else {
+      // a few waves of resident blocks, sites dealt round-robin
+      const long long want = (long long)g_clip_resident_blocks[0] * 4, need = (n + CLIP_WARPS - 1) / CLIP_WARPS;
+      k_clip_site<false, false, SLOTS_TET_CELL, R><<<(int)(want < need ? want : need), CLIP_WARPS * WARP, 0, st>>>(
+          sites, n, knn, probs, site_prob, lone, verts, tets, site_start, site_tets, mom, stats, nullptr, nullptr,
+          nullptr, nullptr, nullptr, nullptr, nullptr, prob_secmiss, nullptr, nullptr, nullptr, nullptr, nullptr,
+          CellStore{}, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+      VGB_CUDA_TRY(cudaGetLastError());
+      return 0;
+    }
   }
   // counters: [0] sites the first pass hands on, [1] sites the one-warp and
   // pieces passes hand to the 128-vertex pass, [2..4] the three passes' work
