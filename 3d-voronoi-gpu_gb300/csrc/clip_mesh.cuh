@@ -168,17 +168,26 @@ struct MeshSum {
     comp_add(hz, lz, z);
     v = x = y = z = 0.f;
   }
-};
-// Sum of a compensated pair per lane, a pair again.
-__device__ __forceinline__ void warp_sum_pair(float& h, float& l) {
-#pragma unroll
-  for (int o = WARP / 2; o > 0; o >>= 1) {
-    const float x = __shfl_xor_sync(FULL, h, o), y = __shfl_xor_sync(FULL, l, o);
-    comp_add(h, l, x);
-    l += y;
+  // over the warp (one loop, not unrolled: unrolled a quantity at a time these
+  // sums are 5 KB of code)
+  __device__ __forceinline__ void reduce() {
+#pragma unroll 1
+    for (int o = WARP / 2; o > 0; o >>= 1) {
+      auto pair = [o](float& h, float& l) {
+        const float x = __shfl_xor_sync(FULL, h, o), y = __shfl_xor_sync(FULL, l, o);
+        comp_add(h, l, x);
+        l += y;
+      };
+      pair(hv, lv);
+      pair(hx, lx);
+      pair(hy, ly);
+      pair(hz, lz);
+      mag += __shfl_xor_sync(FULL, mag, o);
+      open += __shfl_xor_sync(FULL, open, o);
+      way += __shfl_xor_sync(FULL, way, o);
+    }
   }
-}
-
+};
 // Around each face of a cell, and around each triangle, the pieces of its lines
 // close: their vectors sum to nothing.  One sum checks them all, each piece by
 // its product with a vector of its face (hashed, components within 1).
@@ -790,11 +799,8 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
         __syncwarp();
         sum.flush();
       }
-      warp_sum_pair(sum.hv, sum.lv);
-      warp_sum_pair(sum.hx, sum.lx);
-      warp_sum_pair(sum.hy, sum.ly);
-      warp_sum_pair(sum.hz, sum.lz);
-      const float v6 = sum.hv + sum.lv, mag = warp_sum(sum.mag);
+      sum.reduce();
+      const float v6 = sum.hv + sum.lv, mag = sum.mag;
       pr2 = warp_max_nonneg(far2);
       // exact where it meets the mesh when that lies within half the K-th
       // neighbour's distance; else completed by the completion pass (and open as
@@ -821,8 +827,8 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
       // large terms for a small sum: a sliver, or a cell that only touches the
       // mesh (or no number at all)
       bad |= !(mag <= MESH_RATIO * v6 || mag == 0.f);
-      const float tol = __fmaf_rn(MESH_CLOSED, pr2 > 0.f ? sqrtf(pr2) : Rc, MESH_WAY * warp_sum(sum.way));
-      open = !(fabsf(warp_sum(sum.open)) <= tol) || __reduce_add_sync(FULL, skew) != 0;
+      const float tol = __fmaf_rn(MESH_CLOSED, pr2 > 0.f ? sqrtf(pr2) : Rc, MESH_WAY * sum.way);
+      open = !(fabsf(sum.open) <= tol) || __reduce_add_sync(FULL, skew) != 0;
       break;
     }
     bad |= open && !beyond;
