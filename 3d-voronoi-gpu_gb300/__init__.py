@@ -219,14 +219,18 @@ class Engine:
     verts (nv,3) float32 and sites (n,3) float32 in [0,1000]^3, tets (nt,4)
     int32 positively oriented.  Site i of the input keeps id i; the engine
     stores sites in grid order.  exact=True (cell-tet): cells inside the mesh
-    are taken whole and the others are clipped by every tet within reach,
-    instead of the reference's per-tet sums over tet_k candidates.
-    robust_predicates=True: vertex-vs-plane tests within 1e-4 of zero (relative
-    to their terms) are decided by exact determinant signs (the reference's
-    arithmetic filter, with an exact fallback); degenerate inputs such as
-    lattice sites come out whole.  tet_pieces=True (cell-tet): the pieces
-    cell ^ tet of the cells the first pass does not finish are built from
-    their tets, clipped by the cell faces crossing them; False (default)
+    are taken whole, and of the others the part inside every tet within reach
+    counts, instead of the reference's per-tet sums over tet_k candidates.
+    With float predicates that part is summed over the cell's edges and the
+    mesh's open triangles; what such sums cannot do (slivers, degenerate cells,
+    more than 64 vertices) and every cell with robust_predicates=True is
+    clipped by each tet.  robust_predicates=True: vertex-vs-plane tests within
+    1e-4 of zero (relative to their terms) are decided by pairs of floats or
+    exact determinant signs (the reference's arithmetic filter, with an exact
+    fallback); degenerate inputs such as lattice sites come out whole.
+    tet_pieces=True (exact form, where cells are clipped by each tet, or on a
+    mesh of fewer than a tet per 256 sites): the pieces cell ^ tet are built
+    from their tets, clipped by the cell faces crossing them; False (default)
     clips a copy of the cell by each tet.
     """
 

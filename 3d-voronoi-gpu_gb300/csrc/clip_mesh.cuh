@@ -109,7 +109,8 @@ struct MeshSmem {
   int rng[2][WARP];     // the rows in hand: first tet, tets of the rows before
   unsigned cnt[WC_N];
   unsigned here[WC_N], spare[WC_N];  // of the site in hand; of its second sum (not counted)
-  unsigned tr2[MESH_TETS];           // tet-cell method: how far each tet's piece reaches (squared, float bits)
+  unsigned tr2[MESH_TETS];           // tet-cell method: how far each tet's piece reaches (squared, float bits),
+  unsigned char tfar[MESH_TETS];     // and the tets that reach far enough to matter
 };
 
 // dot product ending in + c, the same rounding in every kernel
@@ -646,10 +647,12 @@ __global__ void __launch_bounds__(MESH_WARPS * WARP, VGB_MESH_MIN_BLOCKS) k_cell
           // the pieces that reach beyond half the K-th neighbour's distance (of
           // tets that do, alone)
           const unsigned reach = __ballot_sync(FULL, lane < nb && (S.tinf[lane & (MESH_TETS - 1)] & 64u) != 0u);
+          if ((reach >> lane) & 1u) S.tfar[__popc(reach & lt_mask)] = (unsigned char)lane;
+          __syncwarp();
 #pragma unroll 1
-          for (int w = lane; w < 6 * nb; w += WARP) {
-            const int b = w / 6;
-            const float r2 = (reach >> b) & 1u ? tet_edge(b, w - 6 * b) : -1.f;
+          for (int w = lane; w < 6 * __popc(reach); w += WARP) {
+            const int b = S.tfar[w / 6];
+            const float r2 = tet_edge(b, w % 6);
             if (r2 >= 0.f) {
               S.thit[b] = 1;
               atomicMax(S.tr2 + b, __float_as_uint(r2));

@@ -521,7 +521,7 @@ def run_ours(args):
                    "site_k": K, "tet_k": pkg.tet_k(n, len(P.tets)), "grid_dim": grid_dim, "method": args.method,
                    "knn_tiers": ([32, K] if exact and args.method == "cell_tet" and K > 32 else [K]),
                    "robust_predicates": bool(args.robust_predicates), "launch_shape": shape,
-                   "form": "exact (inside cells whole, boundary cells against every tet in reach)" if exact
+                   "form": "exact (inside cells whole, boundary cells as far as the tets in reach hold them)" if exact
                            else "reference (per-tet sums over tet_k candidates)",
                    "moments": "f32 atomics" if args.method == "plain" else "compensated f32 per site, f64 out",
                    "cuda_graph": True, "l2": "inputs larger than L2 (neighbour lists and tet records > 129 MB), "

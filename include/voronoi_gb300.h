@@ -148,8 +148,8 @@ typedef struct vgb_config {
                    batched form tunes them with the grid density (grid_dim 0).      */
   int tet_pieces; /* cell-tet method, where cells are clipped by each tet (with
                    float predicates a cell's edges and the mesh's open triangles are
-                   summed instead, unless this is 1 and the mesh has fewer than a
-                   tet per 256 sites).  0 (default): a copy of the cell is clipped by
+                   summed instead, unless this is 1, the form is exact and the mesh
+                   has fewer than a tet per 256 sites).  0 (default): a copy of the cell is clipped by
                    each candidate tet's four faces, one warp per site.  1: each piece
                    (cell ^ tet) of a cell the first pass does not finish is built
                    from its tet, clipped by the cell faces that cross the tet, four
