@@ -32,7 +32,8 @@
 //     again at 64 vertices, k_cell_mesh over what it finishes, and 8 slots (256
 //     vertices) over the rest, clipped by each tet.
 //   The tet-cell method is k_clip_site with 3 slots (96 vertices, the
-//   reference's triangle capacity).  Within a warp or group:
+//   reference's triangle capacity) with robust predicates, the mesh pass with
+//   float ones.  Within a warp or group:
 //   * the K bisector planes of the site are computed once, in coordinates
 //     relative to the site, and staged in shared memory; every candidate tet
 //     of the site reuses them;

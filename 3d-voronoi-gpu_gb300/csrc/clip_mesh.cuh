@@ -35,15 +35,15 @@
 // the pieces tells (face_mark): the cell is given back and clipped by each tet.
 //
 // One warp per site: lanes take candidate tets, then (tet, edge) pairs, then
-// faces.  Bound by latency (issuing on 63% of cycles, five blocks of four warps
+// faces.  Bound by latency (issuing on 65% of cycles, five blocks of four warps
 // per SM; stalls on fixed latencies and on the tets' records from L2).  Loops
 // are kept rolled: at 70 KB of code half the stalls were instruction fetches
-// and the pass took 2.0 ms where it takes 1.4 at 50 KB.  A boundary cell (at 1M
-// torus sites 36 edges, 20 tets, 6 open triangles) needs no vertices of its
-// pieces, whose inner faces only cancel.  Measured per Lloyd iteration: 1M sites in 1.96M tets 15.0 ->
-// 5.7 ms from random sites and 4.6 -> 1.8 ms once relaxed (the one-warp pass
-// before, now that pass without its tets and this one); 131k sites in 1.57M
-// tets 6.9 -> 2.3 ms and 1.6 -> 0.5 ms (pieces from the tets before).
+// and the pass took 2.0 ms where it took 1.4 at 50 KB (1.5 with the checks and
+// sums above).  A boundary cell (at 1M torus sites 36 edges, 20 tets, 6 open
+// triangles) needs no vertices of its pieces, whose inner faces only cancel.
+// Measured per Lloyd iteration, 1M sites in 1.96M tets: 15.0 -> 5.9 ms from random
+// sites and 4.6 -> 1.9 ms once relaxed (the one-warp pass before, now that pass
+// without its tets and this one).
 #pragma once
 
 #include "clip_warp.cuh"
